@@ -185,3 +185,47 @@ def test_table_to_planar_layout(gb, dtype, m):
     co = src_np.reshape(nrow, m, 3, 2)  # [r, k, p, c]
     exp[:, :, :2 * m] = co.transpose(0, 2, 1, 3).reshape(nrow, 3, 2 * m)
     np.testing.assert_array_equal(got, exp.astype(got.dtype))
+
+
+# edges of the kernels' splits: one warp or four warps an atom (the lines lie
+# at 10 to 32 atoms for each of 152 SMs), 32-slot neighbour groups, full
+# 32-wide output chunks and the tail after them, 128-wide passes, and rows
+# that are not 16-byte aligned
+@pytest.mark.parametrize("dtype", [torch.float64, torch.float32])
+@pytest.mark.parametrize("nloc,nnei,M,shift", [
+    (1519, 5, 20, 0), (1520, 5, 20, 0), (3039, 5, 9, 0), (3040, 5, 9, 0), (3647, 3, 7, 0),
+    (3648, 3, 7, 0), (4863, 5, 20, 0), (4864, 5, 20, 0), (1, 129, 128, 0), (2, 32, 97, 0), (3, 33, 31, 0),
+    (2, 128, 129, 0), (4, 31, 159, 1), (3, 46, 100, 1), (4865, 3, 33, 1), (2, 200, 256, 0)])
+def test_split_edges_vs_oracle(oracle, dtype, nloc, nnei, M, shift):
+    ops = __import__("dpmd_public_gb300.ops", fromlist=["x"])
+    rng = np.random.default_rng(7 * nloc + 3 * nnei + M)
+    npd = np.float64 if dtype == torch.float64 else np.float32
+    table, info, em_x, em = (a.astype(npd) for a in _random_case(rng, dtype, nloc, nnei, M))
+    dy = rng.normal(0, 1, (nloc, 4, M)).astype(npd)
+    dzx = rng.normal(0, 1, (nloc, nnei)).astype(npd)
+    dzm = rng.normal(0, 1, (nloc, nnei, 4)).astype(npd)
+
+    def dev(a):
+        """On the device, ``shift`` elements past an aligned address."""
+        buf = torch.empty(a.size + shift, dtype=dtype, device=DEV)
+        buf[shift:].copy_(torch.from_numpy(a).reshape(-1))
+        return buf[shift:].view(a.shape)
+
+    tab, inf = torch.tensor(table, device=DEV), torch.tensor(info)
+    ex, emt = dev(em_x), dev(em)
+    # sums of at most 256 terms: 2e-5 (FP32) and 1e-10 (FP64) of the largest
+    tol = 1e-10 if dtype == torch.float64 else 2e-5
+
+    def close(got, ref):
+        np.testing.assert_allclose(got.cpu().numpy().reshape(ref.shape), ref, rtol=0,
+                                   atol=tol * max(1.0, float(np.abs(ref).max())))
+
+    x1 = em_x.reshape(-1, 1)
+    close(ops.tabulate_forward(tab, inf, ex, emt, M),
+          oracle.tabulate_fusion_se_a(table, info, x1, em, M))
+    gx, gm = ops.tabulate_grad(tab, inf, ex, emt, dev(dy))
+    rx, rm = oracle.tabulate_fusion_se_a_grad(table, info, x1, em, dy)
+    close(gx, rx.reshape(nloc, nnei))
+    close(gm, rm)
+    close(ops.tabulate_grad_grad(tab, inf, ex, emt, dev(dzx), dev(dzm), M),
+          oracle.tabulate_fusion_se_a_grad_grad(table, info, x1, em, dzx, dzm, M))
