@@ -1060,15 +1060,11 @@ def kernel_times(model, batch, coord, flush, reps: int = 5):
                            check_status=False, out=b.env)
 
     def fwd():
-        if model._tc_nets is not None:
-            lib.gbdp_se_a_descriptor_fwd_split_f32(P(b.X), P(b.D), P(b.D_lo), P(b.D_rs), P(b.env.em),
-                                                   P(b.atype), P(b.drow), model._tab_ptrs,
-                                                   model._tab_infos, cfg.ntypes, model._sel_c,
-                                                   int(cfg.type_one_side), b.nloc, M, A, S())
-        else:
-            lib.gbdp_se_a_descriptor_fwd_f32(P(b.X), P(b.D), P(b.env.em), P(b.atype), P(b.drow),
-                                             model._tab_ptrs, model._tab_infos, cfg.ntypes,
-                                             model._sel_c, int(cfg.type_one_side), b.nloc, M, A, S())
+        tc = model._tc_nets is not None
+        lib.gbdp_se_a_descriptor_fwd_blk_f32(
+            P(b.X), P(b.D), P(b.D_lo) if tc else None, P(b.D_rs) if tc else None, P(b.env.em),
+            P(b.atype), P(b.drow), model._tab_ptrs, model._tab_infos, cfg.ntypes, model._sel_c,
+            int(cfg.type_one_side), b.nloc, M, A, S())
 
     def fit():
         if model._tc_nets is not None:
@@ -1077,7 +1073,7 @@ def kernel_times(model, batch, coord, flush, reps: int = 5):
             model.fitting_rows(b)
 
     def bwd():
-        lib.gbdp_se_a_descriptor_bwd_f32(
+        lib.gbdp_se_a_descriptor_bwd_blk_f32(
             P(b.force), P(b.vir), P(b.X), P(b.dD), P(b.drow), P(b.env.em), P(b.env.nlist_ext), P(b.env.ext_coord),
             P(b.env.ext_map), P(b.atype), P(model.dstd_inv), P(b.atom_frame), P(b.frame_aoff), P(b.frame_eoff),
             model._tab_ptrs, model._tab_infos, cfg.ntypes, model._sel_c, int(cfg.type_one_side),
@@ -1301,7 +1297,7 @@ def _fit_flops(cfg):
 
 
 PART_KERNEL = {"env_nlist": "k_nlist_env (+ cell build and ghost fill)",
-               "desc_fwd": "k_desc_fwd", "desc_bwd": "k_desc_bwd"}
+               "desc_fwd": "k_fwd_blk", "desc_bwd": "k_bwd_blk"}
 
 # dram__bytes_read.sum + dram__bytes_write.sum per local atom, from one ncu
 # capture of the 12,288-atom step (profiles/k_desc_fwd_bwd_12288.md,

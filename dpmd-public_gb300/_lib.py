@@ -80,6 +80,10 @@ _SIGS = {
     "gbdp_table_planar_row_elems": (ctypes.c_size_t, [_I, _I]),
     "gbdp_table_to_planar_f32": (_I, [_P, _P, _I, _I, _P]),
     "gbdp_table_to_planar_f64": (_I, [_P, _P, _I, _I, _P]),
+    "gbdp_table_blocked_row_elems": (ctypes.c_size_t, [_I]),
+    "gbdp_table_to_blocked_f32": (_I, [_P, _P, _I, _I, _P]),
+    "gbdp_se_a_descriptor_fwd_blk_f32": (_I, [_P] * 9 + [_I, _P, _I, _I, _I, _I, _P]),
+    "gbdp_se_a_descriptor_bwd_blk_f32": (_I, [_P] * 16 + [_I, _P, _I, _F, _F, _I, _I, _I, _I, _P, _P]),
     "gbdp_se_a_descriptor_fwd_split_f32": (_I, [_P] * 9 + [_I, _P, _I, _I, _I, _I, _P]),
     "gbdp_fitting_tc_workspace_bytes": (_Z, [_I]),
     "gbdp_fitting_tc_set_persistent_min_tiles": (None, [_I]),

@@ -188,6 +188,77 @@ __device__ __forceinline__ T dpoly5(const T* a, T x) {
   return a[1] + (T(2) * a[2] + (T(3) * a[3] + (T(4) * a[4] + T(5) * a[5] * x) * x) * x) * x;
 }
 
+template <typename T>
+struct TabVec;
+template <>
+struct TabVec<float> {
+  using v2 = float2;
+};
+template <>
+struct TabVec<double> {
+  using v2 = double2;
+};
+
+// The six coefficients of output k as the pairs (a0, a1), (a2, a3), (a4, a5)
+// that they lie in.
+template <typename T>
+struct Coef {
+  typename TabVec<T>::v2 p[3];
+};
+// Powers of the in-row offset that the polynomials of one neighbour share.
+template <typename T>
+struct XPow;
+template <>
+struct XPow<float> {
+  float x, x2;
+  float2 s, ds;  // (x^2, x^2), (2 x^2, 2 x^2)
+  __device__ __forceinline__ explicit XPow(float v)
+      : x(v), x2(v + v), s(make_float2(v * v, v * v)), ds(make_float2(x2 * v, x2 * v)) {}
+};
+template <>
+struct XPow<double> {
+  double x;
+  __device__ __forceinline__ explicit XPow(double v) : x(v) {}
+};
+
+// FP32: the polynomial as t0(x^2) + x t1(x^2), t0 and t1 the even and odd
+// coefficients, which are the halves of the pairs as loaded: two packed FMAs
+// and one FMA for the value (five in Horner's form), and one packed FMA and
+// two more for the slope t1 + 2 x (u0 + x u1), u = p1 + 2 x^2 p2.
+__device__ __forceinline__ float tab_val(const Coef<float>& c, const XPow<float>& w) {
+  const float2 t = __ffma2_rn(w.s, __ffma2_rn(w.s, c.p[2], c.p[1]), c.p[0]);
+  return fmaf(t.y, w.x, t.x);
+}
+__device__ __forceinline__ void tab_val_slope(const Coef<float>& c, const XPow<float>& w, float& v,
+                                              float& d) {
+  const float2 t = __ffma2_rn(w.s, __ffma2_rn(w.s, c.p[2], c.p[1]), c.p[0]);
+  const float2 u = __ffma2_rn(w.ds, c.p[2], c.p[1]);
+  v = fmaf(t.y, w.x, t.x);
+  d = fmaf(w.x2, fmaf(w.x, u.y, u.x), t.y);
+}
+// FP64 (bound by the FP64 pipe, 2 FMA a clock and SM): Horner's form, value
+// and slope in one sweep of 9 FMAs
+__device__ __forceinline__ double tab_val(const Coef<double>& c, const XPow<double>& w) {
+  double v = fma(c.p[2].y, w.x, c.p[2].x);
+  v = fma(v, w.x, c.p[1].y);
+  v = fma(v, w.x, c.p[1].x);
+  v = fma(v, w.x, c.p[0].y);
+  return fma(v, w.x, c.p[0].x);
+}
+__device__ __forceinline__ void tab_val_slope(const Coef<double>& c, const XPow<double>& w,
+                                              double& vo, double& d) {
+  double v = c.p[2].y, dv = c.p[2].y;
+  v = fma(v, w.x, c.p[2].x);
+  dv = fma(dv, w.x, v);
+  v = fma(v, w.x, c.p[1].y);
+  dv = fma(dv, w.x, v);
+  v = fma(v, w.x, c.p[1].x);
+  dv = fma(dv, w.x, v);
+  v = fma(v, w.x, c.p[0].y);
+  d = fma(dv, w.x, v);
+  vo = fma(v, w.x, c.p[0].x);
+}
+
 // --------------------------------------------------- bulk async copy (TMA) --
 // cp.async.bulk global -> shared completing on an mbarrier.  Both addresses
 // must be 16-byte aligned and the size a multiple of 16.

@@ -44,71 +44,13 @@
 #include <map>
 #include <mutex>
 
-#include "common.cuh"
+#include "fused.cuh"
 
 namespace gbdp {
 namespace {
 
-constexpr int kMaxTab = 16;
-constexpr int kMaxTypes = 4;
 constexpr int kFWarps = 4;
 constexpr int kBWarps = 4;
-constexpr int kAxis = 16;
-
-template <typename T>
-struct TabSet {
-  const T* table[kMaxTab];
-  TableInfo<T> info[kMaxTab];
-  int ntypes;
-  int one_side;  // 1: table per neighbour type; 0: per (neighbour, centre)
-  int ps;        // plane pitch of the k-planar tables (elements)
-  int sec[kMaxTab + 1];
-};
-
-template <typename T>
-__device__ __forceinline__ int tab_index(const TabSet<T>& ts, int tj, int ti) {
-  return ts.one_side ? tj : tj * ts.ntypes + ti;
-}
-
-// plane pitch of the k-planar layout: 2 M elements rounded up to 128 bytes
-template <typename T>
-__host__ __device__ constexpr int kp_pitch(int M) {
-  return sizeof(T) == 4 ? (2 * M + 31) & ~31 : (2 * M + 15) & ~15;
-}
-
-template <typename T>
-struct Vec;
-template <>
-struct Vec<float> {
-  using v2 = float2;
-  using v4 = float4;
-};
-struct alignas(32) dbl4 {
-  double x, y, z, w;
-};
-template <>
-struct Vec<double> {
-  using v2 = double2;
-  using v4 = dbl4;
-};
-template <typename T>
-using V4 = typename Vec<T>::v4;
-
-// L1 policy.  The table rows are the only data the kernels re-read across
-// atoms; everything per atom (env rows, X, dE/dD) streams through once or
-// twice.  Table loads carry L1::evict_last, per-atom rows L1::no_allocate
-// (read once) or L1::evict_first (read twice), so that the hot band of
-// table rows stays resident in L1.
-__device__ __forceinline__ float2 ld_tab2(const float2* p) {
-  float2 v;
-  asm("ld.global.nc.L1::evict_last.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "l"(p));
-  return v;
-}
-__device__ __forceinline__ double2 ld_tab2(const double2* p) {
-  double2 v;
-  asm("ld.global.nc.L1::evict_last.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "l"(p));
-  return v;
-}
 
 // the six coefficients of output k from a k-planar row
 template <typename T>
@@ -178,79 +120,6 @@ __device__ __forceinline__ void bwd_tab_grad_pairs(float* p, const float* __rest
       p[4] += dv * (e.x * d[0] + e.y * d[1] + e.z * d[2] + e.w * d[3]);
     }
   }
-}
-
-// a non-binding prefetch of the 128-byte line holding p into L2
-__device__ __forceinline__ void prefetch_l2(const void* p) {
-  asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
-}
-
-// one row of 4 values (16-byte aligned), not allocated in L1
-__device__ __forceinline__ float4 ld_stream4(const float* p) {
-  float4 v;
-  asm("ld.global.nc.L1::no_allocate.v4.f32 {%0, %1, %2, %3}, [%4];"
-      : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
-      : "l"(p));
-  return v;
-}
-__device__ __forceinline__ dbl4 ld_stream4(const double* p) {
-  dbl4 v;
-  asm("ld.global.nc.L1::no_allocate.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "l"(p));
-  asm("ld.global.nc.L1::no_allocate.v2.f64 {%0, %1}, [%2];" : "=d"(v.z), "=d"(v.w) : "l"(p + 2));
-  return v;
-}
-__device__ __forceinline__ float ld_stream(const float* p) {
-  float v;
-  asm("ld.global.nc.L1::no_allocate.f32 %0, [%1];" : "=f"(v) : "l"(p));
-  return v;
-}
-__device__ __forceinline__ double ld_stream(const double* p) {
-  double v;
-  asm("ld.global.nc.L1::no_allocate.f64 %0, [%1];" : "=d"(v) : "l"(p));
-  return v;
-}
-
-// a row of 4 values read twice by the same warp: first out of L1
-__device__ __forceinline__ float4 ld_first4(const float* p) {
-  float4 v;
-  asm("ld.global.nc.L1::evict_first.v4.f32 {%0, %1, %2, %3}, [%4];"
-      : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
-      : "l"(p));
-  return v;
-}
-__device__ __forceinline__ dbl4 ld_first4(const double* p) {
-  dbl4 v;
-  asm("ld.global.nc.L1::evict_first.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "l"(p));
-  asm("ld.global.nc.L1::evict_first.v2.f64 {%0, %1}, [%2];" : "=d"(v.z), "=d"(v.w) : "l"(p + 2));
-  return v;
-}
-__device__ __forceinline__ float ld_first(const float* p) {
-  float v;
-  asm("ld.global.nc.L1::evict_first.f32 %0, [%1];" : "=f"(v) : "l"(p));
-  return v;
-}
-__device__ __forceinline__ double ld_first(const double* p) {
-  double v;
-  asm("ld.global.nc.L1::evict_first.f64 %0, [%1];" : "=d"(v) : "l"(p));
-  return v;
-}
-
-// one row of 4 values through the default path (16-byte aligned)
-__device__ __forceinline__ float4 ld_row4(const float* p) {
-  return __ldg(reinterpret_cast<const float4*>(p));
-}
-__device__ __forceinline__ dbl4 ld_row4(const double* p) {
-  const double2 a = __ldg(reinterpret_cast<const double2*>(p));
-  const double2 b = __ldg(reinterpret_cast<const double2*>(p) + 1);
-  return dbl4{a.x, a.y, b.x, b.y};
-}
-
-__device__ __forceinline__ void st_row4(float* p, const float4& v) {
-  *reinterpret_cast<float4*>(p) = v;
-}
-__device__ __forceinline__ void st_row4(double* p, const dbl4& v) {
-  reinterpret_cast<double2*>(p)[0] = double2{v.x, v.y};
-  reinterpret_cast<double2*>(p)[1] = double2{v.z, v.w};
 }
 
 // Per-warp shared slot arrays: env row (or, after phase 1, dE/d em), in-row
@@ -498,45 +367,6 @@ __global__ void __launch_bounds__(W * 32)
 }
 
 // --------------------------------------------------------------- backward --
-template <typename T>
-__device__ __forceinline__ void spline5_d(T& vv, T& dd, T xx, T rmin, T rmax) {
-  if (xx < rmin) {
-    dd = T(0);
-    vv = T(1);
-  } else if (xx < rmax) {
-    T uu = (xx - rmin) / (rmax - rmin);
-    T du = T(1) / (rmax - rmin);
-    vv = uu * uu * uu * (T(-6) * uu * uu + T(15) * uu - T(10)) + T(1);
-    dd = (T(3) * uu * uu * (T(-6) * uu * uu + T(15) * uu - T(10)) +
-          uu * uu * uu * (T(-12) * uu + T(15))) *
-         du;
-  } else {
-    dd = T(0);
-    vv = T(0);
-  }
-}
-
-__device__ __forceinline__ float rsqrt_t(float x) { return rsqrtf(x); }
-__device__ __forceinline__ double rsqrt_t(double x) { return rsqrt(x); }
-
-struct BwdGeom {
-  const int* atom_frame;   // [nloc_total] frame of each centre
-  const int* frame_aoff;   // [nframes] first local atom of each frame
-  const int* frame_eoff;   // [nframes] first extended slot of each frame
-};
-
-// Number of filled slots of a section: the env kernel fills each type
-// section from its start, so the filled slots are a prefix.
-__device__ __forceinline__ int filled_prefix(const int* __restrict__ nl, int ns) {
-  const int lane = threadIdx.x & 31;
-  int n = 0;
-  for (int b = 0; b < ns; b += 32) {
-    const bool ok = b + lane < ns && nl[b + lane] >= 0;
-    n += __popc(__ballot_sync(kFull, ok));
-  }
-  return n;
-}
-
 template <typename T>
 __host__ __device__ constexpr size_t bwd_warp_bytes(int nnei, int m) {
   // dy4 [M] and X^T [M] while dX is formed, then the slot arrays over them
@@ -1421,6 +1251,95 @@ extern "C" int gbdp_se_a_descriptor_fwd_split_f32(
     return desc_fwd<float>(X, static_cast<float*>(D_hi), D_lo, D_rscale, em, atype, d_row,
                            tables, table_infos, ntypes, sel, type_one_side, nloc,
                            last_layer_size, axis_neuron, st, w);
+  });
+}
+
+// ---- the descriptor on blocked FP32 tables (kernels in desc_blk.cu)
+extern "C" int gbdp_se_a_descriptor_fwd_blk_f32(
+    float* X, void* D, void* D_lo, float* D_rscale, const float* em, const int* atype,
+    const int* d_row, const float* const* tables, const float* table_infos, int ntypes,
+    const int* sel, int type_one_side, int nloc, int last_layer_size, int axis_neuron,
+    gbdp_stream stream) {
+  const cudaStream_t st = (cudaStream_t)stream;
+  const int M = last_layer_size;
+  TabSet<float> ts;
+  int rc = make_tabset(ts, tables, table_infos, ntypes, sel, type_one_side, M);
+  if (rc) return rc;
+  const int nnei = ts.sec[ntypes];
+  rc = check_shapes<float>(M, axis_neuron, nnei);
+  if (rc) return rc;
+  if (nloc == 0) return GBDP_OK;
+  GBDP_REQUIRE(X && D && em && atype && (!D_lo || D_rscale),
+               "se_a descriptor fwd: null argument");
+  GBDP_REQUIRE(((uintptr_t)em & 15) == 0 && ((uintptr_t)D & 15) == 0 && ((uintptr_t)D_lo & 15) == 0,
+               "se_a descriptor fwd: em / D must be 16-byte aligned");
+  const size_t wb = fwd_warp_bytes<float>(nnei, 128);
+  GBDP_REQUIRE((size_t)kFWarps * wb <= 200 * 1024,
+               "se_a descriptor fwd: nnei %d needs %zu bytes of shared memory", nnei,
+               (size_t)kFWarps * wb);
+  const DescFwdArgs a{X, D, D_lo, D_rscale, em, atype, d_row};
+  return tune_run(kTuneFwd, 4, M, nnei, nloc, st, [&](int w) -> int {
+    if (w == 0) w = tuned_code(kTuneFwd, 4, M, nnei, nloc, kFWarps);
+    return desc_fwd_blk(a, ts, nloc, M, code_warps(w), st);
+  });
+}
+
+extern "C" int gbdp_se_a_descriptor_bwd_blk_f32(
+    float* force, double* virial_acc, const float* X, const float* dE_dD, const int* d_row,
+    const float* em, const int* nlist_ext, const float* ext_coord, const int* ext_map,
+    const int* atype, const float* inv_std, const int* atom_frame, const int* frame_atom_off,
+    const int* frame_ext_off, const float* const* tables, const float* table_infos, int ntypes,
+    const int* sel, int type_one_side, float rcut_smth, float rcut, int nloc, int nframes,
+    int last_layer_size, int axis_neuron, long long* force_fx, gbdp_stream stream) {
+  const cudaStream_t st = (cudaStream_t)stream;
+  const int M = last_layer_size;
+  TabSet<float> ts;
+  int rc = make_tabset(ts, tables, table_infos, ntypes, sel, type_one_side, M);
+  if (rc) return rc;
+  GBDP_REQUIRE(force && virial_acc && nframes >= 1,
+               "se_a descriptor bwd: null output / nframes");
+  const int nnei = ts.sec[ntypes];
+  rc = check_shapes<float>(M, axis_neuron, nnei);
+  if (rc) return rc;
+  GBDP_REQUIRE(((uintptr_t)force_fx & 7) == 0, "se_a descriptor bwd: force_fx not 8-byte aligned");
+  const size_t wb = bwd_warp_bytes<float>(nnei, M);
+  if (nloc > 0) {
+    GBDP_REQUIRE(X && dE_dD && em && nlist_ext && ext_coord && ext_map && atype && inv_std &&
+                     atom_frame && frame_atom_off && frame_ext_off,
+                 "se_a descriptor bwd: null argument");
+    GBDP_REQUIRE(((uintptr_t)em & 15) == 0 && ((uintptr_t)dE_dD & 15) == 0 &&
+                     ((uintptr_t)inv_std & 15) == 0,
+                 "se_a descriptor bwd: em / dE_dD / inv_std must be 16-byte aligned");
+    GBDP_REQUIRE((size_t)kBWarps * wb <= 200 * 1024,
+                 "se_a descriptor bwd: nnei %d needs %zu bytes of shared memory", nnei,
+                 (size_t)kBWarps * wb);
+  }
+  const DescBwdArgs a{force,   virial_acc, force_fx, X,
+                      dE_dD,   d_row,      em,       nlist_ext,
+                      ext_coord, ext_map,  atype,    inv_std,
+                      {atom_frame, frame_atom_off, frame_ext_off}, rcut_smth, rcut};
+  return tune_run(kTuneBwd, 4, M, nnei, nloc, st, [&](int w) -> int {
+    cudaMemsetAsync(virial_acc, 0, sizeof(double) * 9 * (size_t)nframes, st);
+    if (!force_fx || nloc == 0)
+      cudaMemsetAsync(force, 0, sizeof(float) * 3 * (size_t)nloc, st);
+    else
+      cudaMemsetAsync(force_fx, 0, sizeof(long long) * 3 * (size_t)nloc, st);
+    if (nloc == 0) return GBDP_OK;
+    // untuned: two neighbours in flight while the SMs hold less than four
+    // atoms each (192 atoms: 27.6 against 31.7 us; 768 atoms: 41.9 / 39.9)
+    if (w == 0)
+      w = tuned_code(kTuneBwd, 4, M, nnei, nloc, nloc < 152 * 4 ? kBWarps | 8 : kBWarps);
+    int rc = desc_bwd_blk(a, ts, nloc, M, code_warps(w), code_nbrs(w), st);
+    if (rc) return rc;
+    if (force_fx) {
+      const size_t nf = 3 * (size_t)nloc;
+      k_fx_finish<float><<<(unsigned)((nf + 255) / 256), 256, 0, st>>>(force, force_fx, nf,
+                                                                       FxScale<float>::force);
+      k_fx_finish_inplace<<<1, 256, 0, st>>>(virial_acc, 9 * (size_t)nframes,
+                                             FxScale<float>::virial);
+    }
+    GBDP_CHECK_LAUNCH("se_a_descriptor_bwd");
+    return GBDP_OK;
   });
 }
 

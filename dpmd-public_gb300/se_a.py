@@ -164,8 +164,10 @@ class SeAModel:
             self.table_infos = np.asarray(table_infos, np.float64)
             self.table_info_t = [torch.tensor(i, dtype=dtype) for i in self.table_infos]  # CPU
             ct = ctypes.c_double if dtype == torch.float64 else ctypes.c_float
-            # the fused kernels read a k-planar copy of each table
-            self.tables_kp = [self._planar(t) for t in self.tables]
+            # the fused kernels read a copy of each table: blocked in FP32,
+            # k-planar in FP64
+            relay = self._blocked if dtype == torch.float32 else self._planar
+            self.tables_kp = [relay(t) for t in self.tables]
             self._tab_ptrs = (_P * len(self.tables_kp))(*[t.data_ptr() for t in self.tables_kp])
             flat = self.table_infos.reshape(-1)
             self._tab_infos = (ct * len(flat))(*flat.tolist())
@@ -226,14 +228,27 @@ class SeAModel:
         lib = L.load()
         nrow, w6 = table.shape
         m = w6 // 6
-        re = lib.gbdp_table_planar_row_elems(m, table.element_size())
-        dst = torch.empty(nrow * re, dtype=table.dtype, device=table.device)
-        if dst.data_ptr() % 128:
-            raise RuntimeError("planar table allocation is not 128-byte aligned")
+        dst = self._table_copy(table, lib.gbdp_table_planar_row_elems(m, table.element_size()))
         stream = torch.cuda.current_stream(table.device).cuda_stream
         fn = lib.gbdp_table_to_planar_f64 if table.dtype == torch.float64 else \
             lib.gbdp_table_to_planar_f32
         L.check(fn(dst.data_ptr(), table.data_ptr(), nrow, m, stream), "table_to_planar")
+        return dst
+
+    def _blocked(self, table: torch.Tensor) -> torch.Tensor:
+        lib = L.load()
+        nrow, w6 = table.shape
+        dst = self._table_copy(table, lib.gbdp_table_blocked_row_elems(w6 // 6))
+        stream = torch.cuda.current_stream(table.device).cuda_stream
+        L.check(lib.gbdp_table_to_blocked_f32(dst.data_ptr(), table.data_ptr(), nrow, w6 // 6,
+                                              stream), "table_to_blocked")
+        return dst
+
+    @staticmethod
+    def _table_copy(table: torch.Tensor, row_elems: int) -> torch.Tensor:
+        dst = torch.empty(table.shape[0] * row_elems, dtype=table.dtype, device=table.device)
+        if dst.data_ptr() % 128:
+            raise RuntimeError("table copy is not 128-byte aligned")
         return dst
 
     # ------------------------------------------------------------- batches --
@@ -332,25 +347,27 @@ class SeAModel:
             env_mat_packed(b.plan, coord, b.atype, self.davg, self.dstd, cfg.rcut_smth,
                            list(cfg.sel), check_status=False, out=b.env)
         lib = self._lib
+        tabs = (self._tab_ptrs, self._tab_infos, cfg.ntypes, self._sel_c, int(cfg.type_one_side))
+        if self.dtype == torch.float32:
+            L.check(lib.gbdp_se_a_descriptor_fwd_blk_f32(
+                _ptr(b.X), _ptr(b.D), _ptr(getattr(b, "D_lo", None)),
+                _ptr(getattr(b, "D_rs", None)), _ptr(b.env.em), _ptr(b.atype), _ptr(b.drow), *tabs,
+                n, M, A, _stream()), "se_a_descriptor_fwd_blk")
+            bwd = lib.gbdp_se_a_descriptor_bwd_blk_f32
+        else:
+            L.check(lib.gbdp_se_a_descriptor_fwd_f64(
+                _ptr(b.X), _ptr(b.D), _ptr(b.env.em), _ptr(b.atype), _ptr(b.drow), *tabs, n, M, A,
+                _stream()), "se_a_descriptor_fwd")
+            bwd = lib.gbdp_se_a_descriptor_bwd_f64
         if self._tc_nets is not None:
-            L.check(lib.gbdp_se_a_descriptor_fwd_split_f32(
-                _ptr(b.X), _ptr(b.D), _ptr(b.D_lo), _ptr(b.D_rs), _ptr(b.env.em), _ptr(b.atype),
-                _ptr(b.drow),
-                self._tab_ptrs, self._tab_infos, cfg.ntypes, self._sel_c, int(cfg.type_one_side), n,
-                M, A, _stream()), "se_a_descriptor_fwd_split")
             self.fitting_tc(b)
         else:
-            L.check(getattr(lib, f"gbdp_se_a_descriptor_fwd_{self._sfx}")(
-                _ptr(b.X), _ptr(b.D), _ptr(b.env.em), _ptr(b.atype), _ptr(b.drow), self._tab_ptrs,
-                self._tab_infos, cfg.ntypes, self._sel_c, int(cfg.type_one_side), n, M, A,
-                _stream()), "se_a_descriptor_fwd")
             self.fitting_rows(b)
-        L.check(getattr(lib, f"gbdp_se_a_descriptor_bwd_{self._sfx}")(
+        L.check(bwd(
             _ptr(b.force), _ptr(b.vir), _ptr(b.X), _ptr(b.dD), _ptr(b.drow), _ptr(b.env.em),
             _ptr(b.env.nlist_ext),
             _ptr(b.env.ext_coord), _ptr(b.env.ext_map), _ptr(b.atype), _ptr(self.dstd_inv),
-            _ptr(b.atom_frame), _ptr(b.frame_aoff), _ptr(b.frame_eoff), self._tab_ptrs,
-            self._tab_infos, cfg.ntypes, self._sel_c, int(cfg.type_one_side),
+            _ptr(b.atom_frame), _ptr(b.frame_aoff), _ptr(b.frame_eoff), *tabs,
             ctypes.c_float(cfg.rcut_smth), ctypes.c_float(cfg.rcut), n, b.nframes, M, A,
             _ptr(b.force_fx() if deterministic else None), _stream()), "se_a_descriptor_bwd")
         L.check(getattr(lib, f"gbdp_frame_energy_{self._sfx}")(

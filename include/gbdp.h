@@ -490,6 +490,33 @@ GBDP_API int gbdp_se_a_descriptor_fwd_split_f32(
     const float* const* tables, const float* table_infos, int ntypes, const int* sel,
     int type_one_side, int nloc, int last_layer_size, int axis_neuron, gbdp_stream stream);
 
+/* The FP32 descriptor on blocked tables (the faster form; same quantities,
+ * arguments and checks as gbdp_se_a_descriptor_fwd_f32 / _fwd_split_f32 /
+ * _bwd_f32, sums grouped differently).  D_lo NULL: D is FP32 [nrows,
+ * M * axis_neuron]; D_lo given: D and D_lo are the FP16 parts and D_rscale
+ * the inverse row scales, as gbdp_se_a_descriptor_fwd_split_f32 writes them.
+ * gbdp_table_to_blocked_f32 writes a table ([nspline, 6 M] as above) in
+ * blocks of 32 outputs of 192 elements: block b of row r holds, for c < 3 and
+ * t < 16 at 64 c + 4 t, {a_2c[k], a_2c[k + 16], a_2c+1[k], a_2c+1[k + 16]},
+ * k = 32 b + t, with zeros past M.  row_elems = 192 ceil(M / 32); dst holds
+ * nrow * row_elems elements, 128-byte aligned; src and dst device.  No
+ * reference counterpart: a layout choice of this library. */
+GBDP_API size_t gbdp_table_blocked_row_elems(int last_layer_size);
+GBDP_API int gbdp_table_to_blocked_f32(float* dst, const float* src, int nrow,
+                                       int last_layer_size, gbdp_stream stream);
+GBDP_API int gbdp_se_a_descriptor_fwd_blk_f32(
+    float* X, void* D, void* D_lo, float* D_rscale, const float* em, const int* atype,
+    const int* d_row, const float* const* tables, const float* table_infos, int ntypes,
+    const int* sel, int type_one_side, int nloc, int last_layer_size, int axis_neuron,
+    gbdp_stream stream);
+GBDP_API int gbdp_se_a_descriptor_bwd_blk_f32(
+    float* force, double* virial_acc, const float* X, const float* dE_dD, const int* d_row,
+    const float* em, const int* nlist_ext, const float* ext_coord, const int* ext_map,
+    const int* atype, const float* inv_std, const int* atom_frame, const int* frame_atom_off,
+    const int* frame_ext_off, const float* const* tables, const float* table_infos, int ntypes,
+    const int* sel, int type_one_side, float rcut_smth, float rcut, int nloc, int nframes,
+    int last_layer_size, int axis_neuron, long long* force_fx, gbdp_stream stream);
+
 /* ------------------------------------------------------------------------
  * Fitting nets on the tensor cores (tcgen05 kind::f16, each FP32 operand as
  * a scaled FP16 hi/lo pair, which keeps FP32-level accuracy), for the
@@ -544,8 +571,9 @@ GBDP_API void gbdp_fitting_tc_set_persistent_min_tiles(int tiles_per_sm);
 
 /* ---- launch-shape autotuning ----------------------------------------------
  * The fused descriptor kernels (the gbdp_se_a_descriptor_ fwd and bwd entry
- * points) run 1, 2 or 4 centre atoms per CTA, and the FP32 backward 1 or 2
- * neighbours in flight per 16-lane group.  With autotuning on, the first
+ * points) run 1, 2 or 4 warps per CTA, one centre atom each (on blocked
+ * tables the 4 warps share an atom in small batches), and the FP32 backward 1
+ * or 2 neighbours in flight per 16-lane group.  With autotuning on, the first
  * call for a shape key
  * (kernel, dtype, last_layer_size, nnei, floor(log2 nloc)) that is not under
  * stream capture times every choice on the caller's stream (it synchronises
