@@ -253,3 +253,34 @@ def test_external_nlist_bad_index_is_reported(gb):
             torch.tensor(g["ext_type"][None], device=DEV), torch.tensor(nl_in[None], device=DEV),
             torch.tensor(avg, device=DEV), torch.tensor(std, device=DEV), float(g["rcut"]), 0.5,
             sel)
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("inside,width,sel", [
+    (0, 5, (3, 4)), (1, 1, (3, 4)), (32, 40, (50, 60)), (33, 33, (16, 17)), (64, 127, (64, 64)),
+    (65, 128, (65, 1)), (128, 129, (100, 28)), (128, 200, (64, 63)), (129, 300, (90, 90)),
+    (250, 257, (46, 92)), (60, 256, (20, 0, 40))])
+def test_external_nlist_candidate_counts(gb, oracle, dtype, inside, width, sel):
+    """The formatted list at the edges of the sort: none to 250 candidates
+    within rcut (32-, 64- and 128-key sorts, ranking above 128 or above
+    sum(sel)), equal distances, list widths off the 128-entry passes."""
+    rng = np.random.default_rng(1000 * inside + width)
+    nloc, rcut, nt = 6, 6.0, len(sel)
+    cen = rng.uniform(0, 0.1, (nloc, 3))
+
+    def shell(n, lo, hi):
+        v = rng.normal(size=(n, 3))
+        return v / np.linalg.norm(v, axis=1)[:, None] * rng.uniform(lo, hi, (n, 1))
+
+    near = shell(inside, 1.0, 5.7)
+    near[1::7] = near[0:max(inside - 1, 0):7]  # equal distances, ordered by list position
+    far = shell(width - inside, 6.5, 8.0)
+    ext = np.concatenate([cen, near, far]).astype(dtype)
+    typ = rng.integers(0, nt, len(ext)).astype(np.int32)
+    nl = np.stack([nloc + rng.permutation(width) for _ in range(nloc)]).astype(np.int32)
+    avg, std = (np.zeros((nt, sum(sel) * 4), dtype), np.ones((nt, sum(sel) * 4), dtype))
+    D = lambda a: torch.tensor(a[None] if a is not avg and a is not std else a, device=DEV)
+    _, _, _, got = torch.ops.deepmd.prod_env_mat_a_nlist(D(ext), D(typ), D(nl), D(avg), D(std),
+                                                         rcut, 0.5, list(sel))
+    exp = oracle.format_nlist_pt(ext, typ, nl, nloc, rcut, list(sel))
+    np.testing.assert_array_equal(got.cpu().numpy().reshape(nloc, -1), exp)
