@@ -45,6 +45,21 @@ __device__ __forceinline__ T warp_sum(T v) {
 
 __device__ __forceinline__ int lane_id() { return threadIdx.x & 31; }
 
+// v[0 .. 2 N - 1] -> this lane's half of the sums over lanes `o` apart
+template <int N>
+__device__ __forceinline__ void halve(float* v, int o, bool up) {
+#pragma unroll
+  for (int k = 0; k < N; ++k) {
+    const float send = up ? v[k] : v[k + N];
+    const float keep = up ? v[k + N] : v[k];
+    v[k] = keep + __shfl_xor_sync(kFull, send, o);
+  }
+}
+
+__device__ __forceinline__ float2 lo2(const float4& v) { return make_float2(v.x, v.y); }
+__device__ __forceinline__ float2 hi2(const float4& v) { return make_float2(v.z, v.w); }
+__device__ __forceinline__ float2 dup2(float v) { return make_float2(v, v); }
+
 // ------------------------------------------------------ vector reductions --
 // red.global.add over 2 or 4 consecutive floats (sm_90 and later) where the
 // address is 8- / 16-byte aligned; scalar atomics for the rest and for double

@@ -65,10 +65,6 @@ __device__ __forceinline__ void atom_range(int n, int w, int& lo, int& hi) {
   }
 }
 
-__device__ __forceinline__ float2 lo2(const float4& v) { return make_float2(v.x, v.y); }
-__device__ __forceinline__ float2 hi2(const float4& v) { return make_float2(v.z, v.w); }
-__device__ __forceinline__ float2 dup2(float v) { return make_float2(v, v); }
-
 __device__ __forceinline__ float dot44(const float4& a, const float4& b) {
   const float2 h = __ffma2_rn(hi2(a), hi2(b), __fmul2_rn(lo2(a), lo2(b)));
   return h.x + h.y;
@@ -335,17 +331,6 @@ template <int S>
 __host__ __device__ constexpr size_t bwd_bytes(int nnei, int M) {
   const size_t sl = slot_bytes(nnei), dx = (size_t)M * 32 + (S > 1 ? S * 256 : 0);
   return sl > dx ? sl : dx;
-}
-
-// v[0 .. 2 N - 1] -> this lane's half of the sums over lanes `o` apart
-template <int N>
-__device__ __forceinline__ void halve(float* v, int o, bool up) {
-#pragma unroll
-  for (int k = 0; k < N; ++k) {
-    const float send = up ? v[k] : v[k + N];
-    const float keep = up ? v[k + N] : v[k];
-    v[k] = keep + __shfl_xor_sync(kFull, send, o);
-  }
 }
 
 // Phase-1 sums of one neighbour over a lane's outputs (16 lanes a
