@@ -1,9 +1,10 @@
-"""Build libgbdp.so (the C-ABI CUDA library) in-tree for sm_103a, and
-libdeepmd_op_gb300.so (the libtorch registration of the deepmd operators
-over it, for C++ TorchScript hosts).
+"""Build libgbdp.so (the C-ABI CUDA library) in-tree for sm_103a, and over it
+libdeepmd_op_gb300.so (the libtorch registration of the deepmd operators for
+C++ TorchScript hosts) and libgbdp_torch_gb300.so (the native part of the
+Python operators).
 
 Each CUDA translation unit under csrc/ is compiled to an object in parallel
-(the libtorch shim alongside), then linked beside this file.  Rebuilds only
+(the libtorch sides alongside), then linked beside this file.  Rebuilds only
 what a newer source or header affects.
 """
 
@@ -32,8 +33,10 @@ NVCC_FLAGS = ARCH + [
 ]
 
 
-TORCH_SRC = os.path.join(CSRC, "torch_ops.cpp")
-TORCH_LIB = os.path.join(HERE, "libdeepmd_op_gb300.so")
+# libtorch sides over libgbdp.so: the TorchScript shim (registers the deepmd
+# namespace itself) and the native part of the Python operators
+TORCH_LIBS = {os.path.join(CSRC, "torch_ops.cpp"): os.path.join(HERE, "libdeepmd_op_gb300.so"),
+              os.path.join(CSRC, "torch_native.cpp"): os.path.join(HERE, "libgbdp_torch_gb300.so")}
 
 
 def nvcc() -> str:
@@ -81,34 +84,33 @@ def _torch_flags():
             [f"-L{lib}", f"-Wl,-rpath,{lib}", "-ltorch", "-ltorch_cpu", "-lc10", "-lc10_cuda"])
 
 
-def _compile_torch_shim() -> str:
-    """The libtorch registration of the deepmd operators (a C++ TorchScript
-    host loads it in place of the reference's libdeepmd_op_pt.so)."""
+def _compile_torch(src: str) -> str:
     cxx = shutil.which("g++") or "g++"
     cflags, _ = _torch_flags()
-    obj = os.path.join(OBJ, "torch_ops.o")
-    r = subprocess.run([cxx] + cflags + ["-c", TORCH_SRC, "-o", obj], capture_output=True,
-                       text=True)
+    obj = os.path.join(OBJ, os.path.basename(src)[:-4] + ".o")
+    r = subprocess.run([cxx] + cflags + ["-c", src, "-o", obj], capture_output=True, text=True)
     if r.returncode != 0:
-        raise RuntimeError(f"g++ failed on torch_ops.cpp:\n{r.stderr[-4000:]}")
+        raise RuntimeError(f"g++ failed on {os.path.basename(src)}:\n{r.stderr[-4000:]}")
     return obj
 
 
-def _torch_needs_build() -> bool:
-    if not os.path.exists(TORCH_LIB):
+def _torch_needs_build(src: str) -> bool:
+    if not os.path.exists(TORCH_LIBS[src]):
         return True
-    t = os.path.getmtime(TORCH_LIB)
-    deps = [TORCH_SRC, __file__] + glob.glob(os.path.join(ROOT, "include", "*.h"))
+    t = os.path.getmtime(TORCH_LIBS[src])
+    deps = [src, __file__, os.path.join(CSRC, "torch_tab.h")] + glob.glob(
+        os.path.join(ROOT, "include", "*.h"))
     return any(os.path.getmtime(p) > t for p in deps)
 
 
 def build(force: bool = False, verbose_ptxas: bool = False) -> str:
-    if not force and not needs_build() and not _torch_needs_build():
+    torch_srcs = [p for p in TORCH_LIBS if force or _torch_needs_build(p)]
+    if not force and not needs_build() and not torch_srcs:
         return LIB
     os.makedirs(OBJ, exist_ok=True)
     extra = ["-Xptxas", "-v"] if verbose_ptxas else []
-    with cf.ThreadPoolExecutor(max_workers=min(8, os.cpu_count() or 1)) as ex:
-        shim = ex.submit(_compile_torch_shim) if (force or _torch_needs_build()) else None
+    with cf.ThreadPoolExecutor(max_workers=min(10, os.cpu_count() or 1)) as ex:
+        torch_objs = [(p, ex.submit(_compile_torch, p)) for p in torch_srcs]
         if force or needs_build():
             objs = list(ex.map(lambda s: _compile(s, extra), _sources()))
             tmp = LIB + ".tmp"
@@ -117,16 +119,16 @@ def build(force: bool = False, verbose_ptxas: bool = False) -> str:
             if r.returncode != 0:
                 raise RuntimeError(f"link failed:\n{r.stderr}")
             os.replace(tmp, LIB)
-        shim_obj = shim.result() if shim else None
-    if shim_obj:
+        torch_objs = [(p, o.result()) for p, o in torch_objs]
+    for src, obj in torch_objs:
         _, ldflags = _torch_flags()
-        tmp = TORCH_LIB + ".tmp"
-        cmd = [shutil.which("g++") or "g++", "-shared", "-o", tmp, shim_obj, "-L" + HERE,
+        out = TORCH_LIBS[src]
+        cmd = [shutil.which("g++") or "g++", "-shared", "-o", out + ".tmp", obj, "-L" + HERE,
                "-Wl,-rpath,$ORIGIN", "-lgbdp"] + ldflags
         r = subprocess.run(cmd, capture_output=True, text=True)
         if r.returncode != 0:
-            raise RuntimeError(f"link of libdeepmd_op_gb300.so failed:\n{r.stderr[-4000:]}")
-        os.replace(tmp, TORCH_LIB)
+            raise RuntimeError(f"link of {os.path.basename(out)} failed:\n{r.stderr[-4000:]}")
+        os.replace(out + ".tmp", out)
     return LIB
 
 

@@ -24,6 +24,8 @@ There is no CPU implementation: CPU tensors raise.
 from __future__ import annotations
 
 import ctypes
+import os
+import types
 
 import numpy as np
 import torch
@@ -128,42 +130,42 @@ def tabulate_grad_grad(table, table_info, em_x, em, dz_dem_x, dz_dem, last_layer
     return dz
 
 
-class _TabulateGradFn(torch.autograd.Function):
-    """dy -> (dy_dem_x, dy_dem); its backward is the grad-grad kernel, which
-    (as in the reference) differentiates wrt dy only."""
-
-    @staticmethod
-    def forward(ctx, table, table_info, em_x, em, dy):
-        ctx.save_for_backward(table, table_info, em_x, em)
-        ctx.M = dy.shape[2]
-        return tabulate_grad(table, table_info, em_x, em, dy)
-
-    @staticmethod
-    def backward(ctx, g_dem_x, g_dem):
-        table, table_info, em_x, em = ctx.saved_tensors
-        if g_dem_x is None:
-            g_dem_x = torch.zeros_like(em_x)
-        if g_dem is None:
-            g_dem = torch.zeros_like(em)
-        dz = tabulate_grad_grad(table, table_info, em_x, em, g_dem_x, g_dem, ctx.M)
-        return None, None, None, None, dz
+# ------------------------------------------------- native operator part --
+# csrc/torch_native.cpp: the operators below and their autograd in C++ (the
+# host work of a small training batch went into Python autograd functions and
+# ctypes calls).  Its errors are raised as GbdpError where they are the
+# library's own (a status code or a device status).
+NATIVE_PATH = os.path.join(os.path.dirname(os.path.abspath(__file__)), "libgbdp_torch_gb300.so")
+_native = None
 
 
-class TabulateFusionSeAFn(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, table, table_info, em_x, em, last_layer_size):
-        ctx.save_for_backward(table, table_info, em_x, em)
-        return tabulate_forward(table, table_info, em_x, em, last_layer_size)
+def native():
+    """The operators of csrc/torch_native.cpp (loaded once; no fallback)."""
+    global _native
+    if _native is None:
+        L.load()
+        if not os.path.exists(NATIVE_PATH):
+            raise RuntimeError(
+                f"{NATIVE_PATH} is missing: build it with __graft_entry__.build()")
+        torch.ops.load_library(NATIVE_PATH)
+        ns = torch.ops.gbdp_native
+        _native = types.SimpleNamespace(**{n: getattr(ns, n).default for n in (
+            "tab", "prod_force", "prod_virial", "env_mat", "env_mat_nlist")})
+    return _native
 
-    @staticmethod
-    def backward(ctx, dy):
-        table, table_info, em_x, em = ctx.saved_tensors
-        gx, gm = _TabulateGradFn.apply(table, table_info, em_x, em, dy.contiguous())
-        return None, None, gx, gm, None
+
+def _call(op, *args):
+    try:
+        return op(*args)
+    except RuntimeError as e:
+        msg = str(e)
+        if type(e) is RuntimeError and (" device status " in msg or " failed (" in msg.split("\n")[0]):
+            raise L.GbdpError(msg.split("\n")[0]) from None
+        raise
 
 
 def tabulate_fusion_se_a(table, table_info, em_x, em, last_layer_size: int):
-    return [TabulateFusionSeAFn.apply(table, table_info, em_x, em, int(last_layer_size))]
+    return [_call(native().tab, table, table_info, em_x, em, last_layer_size)]
 
 
 # ------------------------------------------------------- neighbour plan --
@@ -323,49 +325,12 @@ def env_mat_skin(plan: NeighborPlan, vl: VerletList, coord, atype, avg, std, rcu
 
 
 # ---------------------------------------------------- TF-contract ops --
-_PLAN_CACHE: dict = {}
-
-
-def _plan_for(nloc, boxes_np, rcut, device, dtype):
-    key = (int(nloc), boxes_np.tobytes(), float(rcut), str(device), dtype)
-    p = _PLAN_CACHE.get(key)
-    if p is None:
-        if len(_PLAN_CACHE) > 16:
-            _PLAN_CACHE.clear()
-        p = NeighborPlan([nloc] * boxes_np.shape[0], boxes_np, rcut, device, dtype)
-        _PLAN_CACHE[key] = p
-    return p
-
-
 def prod_env_mat_a_impl(coord, atype, natoms, box, mesh, davg, dstd, rcut_a: float,
                         rcut_r: float, rcut_r_smth: float, sel_a, sel_r):
     """TF ProdEnvMatA in its internal-PBC mode (mesh of 6 ints).  The box is
     read on the host to plan the cell grid, as the reference does."""
-    _need_cuda(coord, atype, davg, dstd)
-    if any(int(s) != 0 for s in sel_r):
-        raise RuntimeError("Rotational free descriptor only support all-angular information: "
-                           "sel_r should be all zero.")
-    nat = [int(v) for v in natoms.reshape(-1).tolist()]
-    nloc, nall = nat[0], nat[1]
-    ntypes = len(nat) - 2
-    if mesh.numel() != 6:
-        raise NotImplementedError(
-            "only the internal periodic mode (mesh of 6) is implemented on GB300")
-    if nloc != nall:
-        raise RuntimeError("internal periodic mode requires nloc == nall")
-    if len(sel_a) != ntypes:
-        raise RuntimeError("number of types should match the length of sel array")
-    nf = coord.shape[0]
-    dt = coord.dtype
-    boxes = box.detach().to("cpu", torch.float64).reshape(nf, 9).numpy()
-    plan = _plan_for(nloc, boxes, rcut_r, coord.device, dt)
-    nnei = int(sum(sel_a))
-    r = env_mat_packed(plan, coord.reshape(nf * nloc, 3).contiguous(),
-                       atype.reshape(nf * nloc).to(torch.int32).contiguous(),
-                       davg.to(dt).contiguous(), dstd.to(dt).contiguous(), rcut_r_smth,
-                       [int(s) for s in sel_a])
-    return [r.em.reshape(nf, nloc * nnei * 4), r.em_deriv.reshape(nf, nloc * nnei * 12),
-            r.rij.reshape(nf, nloc * nnei * 3), r.nlist.reshape(nf, nloc * nnei)]
+    return _call(native().env_mat, coord, atype, natoms, box, mesh, davg, dstd, rcut_r,
+                 rcut_r_smth, sel_a, sel_r)
 
 
 def prod_env_mat_a_nlist_impl(coord, atype, nlist, davg, dstd, rcut: float, rcut_smth: float,
@@ -378,37 +343,7 @@ def prod_env_mat_a_nlist_impl(coord, atype, nlist, davg, dstd, rcut: float, rcut
     sort, then deepmd/pt/utils/nlist.py:304-337, and returns the ProdEnvMatA
     outputs (descrpt, descrpt_deriv, rij, nlist) with nlist in the extended
     index space."""
-    _need_cuda(coord, atype, nlist, davg, dstd)
-    nf, nloc, nnei_in = (int(x) for x in nlist.shape)
-    dt = coord.dtype
-    nall = coord.reshape(nf, -1).shape[1] // 3
-    if atype.reshape(nf, -1).shape[1] != nall:
-        raise RuntimeError("type must have nall entries per frame")
-    sel = [int(x) for x in sel]
-    nnei = sum(sel)
-    dev = coord.device
-    em = torch.empty((nf, nloc * nnei * 4), dtype=dt, device=dev)
-    emd = torch.empty((nf, nloc * nnei * 12), dtype=dt, device=dev)
-    rij = torch.empty((nf, nloc * nnei * 3), dtype=dt, device=dev)
-    nl_out = torch.empty((nf, nloc * nnei), dtype=torch.int32, device=dev)
-    status = torch.zeros(1, dtype=torch.int32, device=dev)
-    sel_c = (ctypes.c_int * len(sel))(*sel)
-    # converted copies stay referenced until the launch is enqueued
-    coord = coord.contiguous()
-    atype = atype.to(torch.int32).contiguous()
-    nlist = nlist.to(torch.int32).contiguous()
-    davg = davg.to(dt).contiguous()
-    dstd = dstd.to(dt).contiguous()
-    fn = getattr(L.load(), f"gbdp_prod_env_mat_a_nlist_{L.sfx(dt)}")
-    L.check(fn(_ptr(em), _ptr(emd), _ptr(rij), _ptr(nl_out), _ptr(status), _ptr(coord),
-               _ptr(atype), _ptr(nlist), _ptr(davg), _ptr(dstd), nf, nloc, nall, nnei_in,
-               ctypes.c_float(rcut), ctypes.c_float(rcut_smth), sel_c, len(sel), _stream()),
-            "prod_env_mat_a_nlist")
-    st = int(status.item())
-    if st:
-        raise L.GbdpError(f"prod_env_mat_a_nlist device status {st}: "
-                          f"{L.GBDP_STATUS.get(st, '?')}")
-    return [em, emd, rij, nl_out]
+    return _call(native().env_mat_nlist, coord, atype, nlist, davg, dstd, rcut, rcut_smth, sel)
 
 
 def prod_force_se_a_impl(net_deriv, in_deriv, nlist, natoms, n_a_sel: int, n_r_sel: int,
@@ -509,41 +444,16 @@ def prod_virial_grad_impl(grad, in_deriv, rij, nlist, nloc, nnei, nf):
     return out
 
 
-class ProdForceFn(torch.autograd.Function):
+def prod_force(net_deriv, in_deriv, nlist, natoms, n_a_sel: int, n_r_sel: int):
     """force = prod_force(net_deriv); backward wrt net_deriv is prod_force_grad
     (the TF ProdForceSeA gradient, source/op/tf/prod_force_grad_multi_device.cc)."""
-
-    @staticmethod
-    def forward(ctx, net_deriv, in_deriv, nlist, natoms, n_a_sel, n_r_sel):
-        ctx.save_for_backward(in_deriv, nlist)
-        nat = [int(v) for v in natoms.reshape(-1).tolist()]
-        ctx.dims = (nat[0], nat[1], int(n_a_sel) + int(n_r_sel), net_deriv.shape[0])
-        return prod_force_se_a_impl(net_deriv, in_deriv, nlist, natoms, n_a_sel, n_r_sel)
-
-    @staticmethod
-    def backward(ctx, g_force):
-        in_deriv, nlist = ctx.saved_tensors
-        nloc, nall, nnei, nf = ctx.dims
-        g = g_force.reshape(nf, nall, 3)[:, :nloc, :].contiguous()
-        return prod_force_grad_impl(g, in_deriv, nlist, nloc, nnei, nf), None, None, None, None, None
+    return _call(native().prod_force, net_deriv, in_deriv, nlist, natoms, n_a_sel, n_r_sel)
 
 
-class ProdVirialFn(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, net_deriv, in_deriv, rij, nlist, natoms, n_a_sel, n_r_sel):
-        ctx.save_for_backward(in_deriv, rij, nlist)
-        nat = [int(v) for v in natoms.reshape(-1).tolist()]
-        ctx.dims = (nat[0], nat[1], int(n_a_sel) + int(n_r_sel), net_deriv.shape[0])
-        return prod_virial_se_a_impl(net_deriv, in_deriv, rij, nlist, natoms, n_a_sel, n_r_sel)
-
-    @staticmethod
-    def backward(ctx, g_vir, g_atom_vir):
-        in_deriv, rij, nlist = ctx.saved_tensors
-        nloc, nall, nnei, nf = ctx.dims
-        if g_vir is None:
-            return None, None, None, None, None, None, None
-        g = prod_virial_grad_impl(g_vir.contiguous(), in_deriv, rij, nlist, nloc, nnei, nf)
-        return g, None, None, None, None, None, None
+def prod_virial(net_deriv, in_deriv, rij, nlist, natoms, n_a_sel: int, n_r_sel: int):
+    """[virial, atom_virial]; backward of the virial wrt net_deriv is
+    prod_virial_grad (source/op/tf/prod_virial_grad_multi_device.cc)."""
+    return _call(native().prod_virial, net_deriv, in_deriv, rij, nlist, natoms, n_a_sel, n_r_sel)
 
 
 # -------------------------------------------------------- registration --
@@ -556,7 +466,7 @@ def register() -> None:
     global _REGISTERED
     if _REGISTERED:
         return
-    L.load()
+    native()
     try:
         lib = torch.library.Library("deepmd", "DEF")
     except RuntimeError:
@@ -584,11 +494,7 @@ def register() -> None:
          "Tensor dstd, float rcut, float rcut_smth, int[] sel) -> Tensor[]",
          prod_env_mat_a_nlist_impl)
     _def("prod_force_se_a(Tensor net_deriv, Tensor in_deriv, Tensor nlist, Tensor natoms, "
-         "int n_a_sel, int n_r_sel) -> Tensor",
-         lambda net_deriv, in_deriv, nlist, natoms, n_a_sel, n_r_sel: ProdForceFn.apply(
-             net_deriv, in_deriv, nlist, natoms, n_a_sel, n_r_sel))
+         "int n_a_sel, int n_r_sel) -> Tensor", prod_force)
     _def("prod_virial_se_a(Tensor net_deriv, Tensor in_deriv, Tensor rij, Tensor nlist, "
-         "Tensor natoms, int n_a_sel, int n_r_sel) -> Tensor[]",
-         lambda net_deriv, in_deriv, rij, nlist, natoms, n_a_sel, n_r_sel: list(
-             ProdVirialFn.apply(net_deriv, in_deriv, rij, nlist, natoms, n_a_sel, n_r_sel)))
+         "Tensor natoms, int n_a_sel, int n_r_sel) -> Tensor[]", prod_virial)
     _REGISTERED = True

@@ -698,7 +698,7 @@ class Trainable:
                 h = out + h if skip == "same" else out
             E_atom = E_atom.index_add(0, idx, (self._mm(h, wf) + bf)[:, 0] + m.bias_atom_e[t])
         net = torch.autograd.grad(E_atom.sum(), em, create_graph=True)[0]
-        from .ops import ProdForceFn, ProdVirialFn
+        from .ops import prod_force, prod_virial
 
         F, V = [], []
         for f in range(b.nframes):
@@ -708,9 +708,9 @@ class Trainable:
             nd = net[a0:a0 + nl].reshape(1, -1)
             ed = env.em_deriv[a0:a0 + nl].reshape(1, -1)
             nls = env.nlist[a0:a0 + nl].reshape(1, -1)
-            F.append(ProdForceFn.apply(nd, ed, nls, natoms, nnei, 0).reshape(nl, 3))
-            V.append(ProdVirialFn.apply(nd, ed, env.rij[a0:a0 + nl].reshape(1, -1), nls, natoms, nnei,
-                                        0)[0].reshape(9))
+            F.append(prod_force(nd, ed, nls, natoms, nnei, 0).reshape(nl, 3))
+            V.append(prod_virial(nd, ed, env.rij[a0:a0 + nl].reshape(1, -1), nls, natoms, nnei,
+                                 0)[0].reshape(9))
         E = torch.zeros(b.nframes, dtype=m.dtype, device=m.device).index_add(0, b.frame_of_atom, E_atom)
         return E, torch.cat(F), torch.stack(V)
 
