@@ -77,17 +77,32 @@ struct TcCfg {
   static constexpr int TBN = TBN_, STAGES = STAGES_, NACC = NACC_;
   static constexpr int B_TILE = TBN * TBK * 2;
   static constexpr int STAGE = 2 * A_TILE + 2 * B_TILE;
-  static constexpr uint32_t ACC_COLS = TBN <= 128 ? 128 : 256;  // TMEM columns per accumulator
+  // TMEM columns per accumulator
+  static constexpr uint32_t ACC_COLS = TBN <= 32 ? 32 : TBN <= 64 ? 64 : TBN <= 128 ? 128 : 256;
   static constexpr int TMEM_COLS = (NACC + 1) * (int)ACC_COLS;   // NACC main + 1 cross-term
   static constexpr int COLP = ((5 * TBN * 4) + 127) & ~127;       // per-column epilogue parameters
   static constexpr int SMEM = STAGES * STAGE + 1024 + 256 + COLP;  // + alignment slack + barriers
   static_assert(TBN % 16 == 0 && TBN <= 256, "tcgen05 M=128 needs N % 16 == 0, N <= 256");
   // CTAs that fit an SM by shared memory must also fit its 512 TMEM columns
   static_assert((228 * 1024 / SMEM) * TMEM_COLS <= 512, "TMEM over-subscribed");
+  static_assert((TMEM_COLS & (TMEM_COLS - 1)) == 0 && TMEM_COLS >= 32, "TMEM allocation size");
   static_assert(SMEM <= 227 * 1024, "shared memory per CTA");
 };
 using CfgLongK = TcCfg<128, 3, 3>;
 using CfgShortK = TcCfg<80, 2, 1>;
+// Few row blocks: a layer is one tile's latency, so the tiles are narrow (a
+// short epilogue, one to three 16-column chunks, and few bytes a stage) and
+// all of a K-240 layer's loads are in flight at once: 16 columns while that
+// many tiles fit the SMs in one wave (up to 10 row blocks), then 48 (up to
+// 30); B1 in 48-column tiles up to 4 row blocks.  The whole fitting of 192 /
+// 768 / 1,800 / 3,750 atoms, same bits: 86 / 89 / 95 / 102 us with the
+// configurations above, 61 / 65 / 80 / 90 us with these (48 columns at 192
+// atoms: 71 us; 16 at 1,800: 117 us; 48 at 4,500: 121 against 109 us).
+using CfgLong16 = TcCfg<16, 5, 3>;
+using CfgShort16 = TcCfg<16, 4, 1>;
+using CfgLong48 = TcCfg<48, 4, 3>;
+using CfgShort48 = TcCfg<48, 4, 1>;
+constexpr int kMaxNarrowRows = 30 * TBM;  // rows that the narrow tiles serve at most
 constexpr int FIT_W = 240;                           // hidden width this kernel serves
 constexpr int FIT_D = 1600;                          // descriptor width this kernel serves
 
@@ -939,9 +954,17 @@ TcWs carve_tc(void* base, long rows) {
   w.gz2l = f16();
   w.gz1h = f16();
   w.gz1l = f16();
-  w.epart = static_cast<float*>(take(sizeof(float) * (size_t)rows * (FIT_W / 80)));
+  w.epart = static_cast<float*>(
+      take(sizeof(float) * (size_t)rows * (FIT_W / (rows <= kMaxNarrowRows ? 16 : 80))));
   w.bytes = off;
   return w;
+}
+
+template <class C>
+cudaError_t launch_tile(cudaLaunchConfig_t& lc, const TcMaps& maps, const TcEpi& ep, int K) {
+  cudaFuncSetAttribute(k_fit_tc<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM);
+  lc.dynamicSmemBytes = C::SMEM;
+  return cudaLaunchKernelEx(&lc, k_fit_tc<C>, maps, ep, K);
 }
 
 }  // namespace
@@ -1000,10 +1023,6 @@ extern "C" int gbdp_fitting_tc_f32(float* e, float* dE_dD, const void* D_hi, con
   int* status = reinterpret_cast<int*>(static_cast<char*>(workspace) + ws.bytes);
   cudaStream_t st = (cudaStream_t)stream;
   cudaMemsetAsync(status, 0, sizeof(int) * 4, st);
-  cudaFuncSetAttribute(k_fit_tc<CfgLongK>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       CfgLongK::SMEM);
-  cudaFuncSetAttribute(k_fit_tc<CfgShortK>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       CfgShortK::SMEM);
   cudaFuncSetAttribute(k_fit_pers, cudaFuncAttributeMaxDynamicSharedMemorySize, PERS_SMEM);
   // SM count of the device (initialised once, thread-safe)
   static const int nsm = [] {
@@ -1027,13 +1046,28 @@ extern "C" int gbdp_fitting_tc_f32(float* e, float* dE_dD, const void* D_hi, con
     GBDP_REQUIRE(((uintptr_t)nets[t].idt[1] & 15) == 0 && ((uintptr_t)nets[t].idt[2] & 15) == 0,
                  "fit_tc: idt not 16-byte aligned");
   }
-  enum { LONGK = 0, SHORTK, PERSIST };
+  enum { LONGK = 0, SHORTK, PERSIST, LONG16, SHORT16, LONG48, SHORT48 };
   // the K-240 layers go to the persistent kernel from this many tiles per SM
   const long short_tiles = (rows / TBM) * (FIT_W / CfgShortK::TBN);
-  const int short_cfg =
-      short_tiles >= (long)g_short_pers_min_tiles.load() * nsm ? PERSIST : SHORTK;
+  const long nblk = rows / TBM;
+  const bool narrow16 = nblk <= kMaxNarrowRows / TBM && nblk * (FIT_W / 16) <= nsm,
+             narrow48 = nblk <= kMaxNarrowRows / TBM && nblk * (FIT_W / 48) <= nsm;
+  const int long_cfg = narrow16 ? LONG16 : narrow48 ? LONG48 : LONGK;
+  const int short_cfg = short_tiles >= (long)g_short_pers_min_tiles.load() * nsm ? PERSIST
+                        : narrow16                                                ? SHORT16
+                        : narrow48                                                ? SHORT48
+                                                                                  : SHORTK;
+  // B1 in 48-column tiles while they fit one wave
+  const int b1_cfg = nblk * ((FIT_D + 47) / 48) <= nsm ? SHORT48 : PERSIST;
+  auto width_of = [](int cfg) {
+    return cfg == LONGK                        ? CfgLongK::TBN
+           : cfg == SHORTK                     ? CfgShortK::TBN
+           : cfg == PERSIST                    ? PERS_TBN
+           : cfg == LONG16 || cfg == SHORT16 ? 16
+                                               : 48;
+  };
   // F3's partial energies: one per N tile of the kernel that runs it
-  base.ntile_n = short_cfg == PERSIST ? (FIT_W + PERS_TBN - 1) / PERS_TBN : FIT_W / CfgShortK::TBN;
+  base.ntile_n = (FIT_W + width_of(short_cfg) - 1) / width_of(short_cfg);
   // act: index into act_scale of the split output (-1: none)
   struct Step {
     int kind;
@@ -1050,7 +1084,7 @@ extern "C" int gbdp_fitting_tc_f32(float* e, float* dE_dD, const void* D_hi, con
                 "tile widths must divide the layer widths (F1's last tile may be partial)");
   const Step steps[6] = {
       {EPI_F1, D_hi, D_lo, FIT_D, FIT_W, 0, true, {nullptr, nullptr}, {ws.t1, ws.h1h, ws.h1l}, 0,
-       LONGK},
+       long_cfg},
       {EPI_F2, ws.h1h, ws.h1l, FIT_W, FIT_W, 1, true, {ws.t1, nullptr}, {ws.t2, ws.h2h, ws.h2l},
        1, short_cfg},
       {EPI_F3, ws.h2h, ws.h2l, FIT_W, FIT_W, 2, true, {ws.t1, ws.t2},
@@ -1060,7 +1094,7 @@ extern "C" int gbdp_fitting_tc_f32(float* e, float* dE_dD, const void* D_hi, con
       {EPI_B2, ws.gz2h, ws.gz2l, FIT_W, FIT_W, 1, false, {ws.t1, ws.g2},
        {nullptr, ws.gz1h, ws.gz1l}, 4, short_cfg},
       {EPI_B1, ws.gz1h, ws.gz1l, FIT_W, FIT_D, 0, false, {nullptr, nullptr},
-       {dE_dD, nullptr, nullptr}, -1, PERSIST}};
+       {dE_dD, nullptr, nullptr}, -1, b1_cfg}};
   for (const Step& sp : steps) {
     TcMaps maps;
     memset(&maps, 0, sizeof(maps));
@@ -1071,7 +1105,7 @@ extern "C" int gbdp_fitting_tc_f32(float* e, float* dE_dD, const void* D_hi, con
       // forward B = W_l^T [out, in]; backward B = W_l [in, out]: both K-major
       const void* bh = sp.fwd ? n.wt_hi[sp.layer] : n.w_hi[sp.layer];
       const void* bl = sp.fwd ? n.wt_lo[sp.layer] : n.w_lo[sp.layer];
-      const int tbn = sp.cfg == LONGK ? CfgLongK::TBN : sp.cfg == SHORTK ? CfgShortK::TBN : PERS_TBN;
+      const int tbn = width_of(sp.cfg);
       rc = make_map(&maps.b_hi[t], bh, sp.N, sp.K, tbn);
       if (!rc) rc = make_map(&maps.b_lo[t], bl, sp.N, sp.K, tbn);
     }
@@ -1113,14 +1147,16 @@ extern "C" int gbdp_fitting_tc_f32(float* e, float* dE_dD, const void* D_hi, con
     lc.blockDim = dim3(128);
     lc.stream = st;
     cudaError_t le;
-    if (sp.cfg == LONGK) {
-      lc.gridDim = dim3((sp.N + CfgLongK::TBN - 1) / CfgLongK::TBN, (unsigned)(rows / TBM));
-      lc.dynamicSmemBytes = CfgLongK::SMEM;
-      le = cudaLaunchKernelEx(&lc, k_fit_tc<CfgLongK>, maps, ep, sp.K);
-    } else if (sp.cfg == SHORTK) {
-      lc.gridDim = dim3(sp.N / CfgShortK::TBN, (unsigned)(rows / TBM));
-      lc.dynamicSmemBytes = CfgShortK::SMEM;
-      le = cudaLaunchKernelEx(&lc, k_fit_tc<CfgShortK>, maps, ep, sp.K);
+    if (sp.cfg != PERSIST) {
+      lc.gridDim = dim3((sp.N + width_of(sp.cfg) - 1) / width_of(sp.cfg), (unsigned)nblk);
+      switch (sp.cfg) {
+        case LONGK: le = launch_tile<CfgLongK>(lc, maps, ep, sp.K); break;
+        case SHORTK: le = launch_tile<CfgShortK>(lc, maps, ep, sp.K); break;
+        case LONG16: le = launch_tile<CfgLong16>(lc, maps, ep, sp.K); break;
+        case SHORT16: le = launch_tile<CfgShort16>(lc, maps, ep, sp.K); break;
+        case LONG48: le = launch_tile<CfgLong48>(lc, maps, ep, sp.K); break;
+        default: le = launch_tile<CfgShort48>(lc, maps, ep, sp.K); break;
+      }
     } else {
       // one CTA per SM walking the layer's tiles
       const int ntn = (sp.N + PERS_TBN - 1) / PERS_TBN, ntiles = ntn * (int)(rows / TBM);

@@ -99,3 +99,37 @@ def test_persistent_short_k_layers_equal_per_tile(setup):
     torch.testing.assert_close(out[0][0], out[1][0], rtol=1e-6, atol=1e-6)
     for x, y in zip(out[0][1:], out[1][1:]):
         assert torch.equal(x, y)
+
+
+@pytest.mark.parametrize("mols", [1, 40, 43, 190, 256, 416, 427, 1193, 1280])
+def test_tile_widths_by_rows_vs_fp64(setup, mols):
+    """Per-row energy and dE/dD of random descriptor rows against FP64, at row
+    counts on both sides of the lines between the 16-, 48- and 80 / 128-wide
+    tiles (10 and 30 row blocks of 128; B1: 4 row blocks).  Operands are split
+    to 2^-22, sums of 1,600 terms in FP32: 1e-5 of the largest magnitude."""
+    m = setup[3]("tc-f16x3")
+    n = 3 * mols
+    b = m.batch([np.tile(np.array([0, 1, 1], np.int32), mols)], np.diag([60.0] * 3).reshape(1, 9))
+    g = torch.Generator(device=DEV).manual_seed(mols)
+    D = torch.randn(n, 1600, generator=g, device=DEV) * 0.2
+    rows = b.drow.long()
+    sc = torch.exp2(14 - torch.floor(torch.log2(D.abs().amax(1))))
+    y = D * sc[:, None]
+    b.D[rows] = y.half()
+    b.D_lo[rows] = (y - y.half().float()).half()
+    b.D_rs[rows] = 1 / sc
+    m.fitting_tc(b)
+    torch.cuda.synchronize()
+    for t, (s0, cnt) in enumerate(b.type_rows):
+        d = ((b.D[s0:s0 + cnt].double() + b.D_lo[s0:s0 + cnt].double())
+             * b.D_rs[s0:s0 + cnt].double()[:, None]).requires_grad_(True)
+        h = d
+        hidden, wf, bf = m.fit[t]
+        for w, bb, idt, skip in hidden:
+            o = torch.tanh(h @ w.double() + bb.double())
+            o = o if idt is None else o * idt.double()
+            h = o + h if skip == "same" else o
+        e = (h @ wf.double() + bf.double())[:, 0]
+        ref = torch.autograd.grad(e.sum(), d)[0]
+        assert float((b.ae[s0:s0 + cnt].double() - e).abs().max()) <= 1e-5 * float(e.abs().max())
+        assert float((b.dD[s0:s0 + cnt].double() - ref).abs().max()) <= 1e-5 * float(ref.abs().max())
