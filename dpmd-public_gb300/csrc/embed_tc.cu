@@ -13,16 +13,19 @@
 // accumulation in tensor memory); layer 1, the activations (tanh.approx),
 // the skips, G^T R and D are FP32.
 //
-// Work unit: two atoms of one centre type.  For each neighbour type the two
-// atoms' section rows are concatenated and cut into 128-row tiles; a tile's
-// rows are one thread's each (thread r <-> TMEM lane r); one warpgroup per
-// CTA, two CTAs per SM.
+// A tile is 128 rows, one thread each (thread r <-> TMEM lane r), 32 a warp;
+// the rows of a warp are its own atom's (see the row mapping below); one
+// warpgroup per CTA, three CTAs per SM forward and two backward.
 //   layer 1 (SIMT)  -> A (bf16, 128 x 64, SW128 K-major, shared)
-//   MMA  D2 = A W2   (N 64, TMEM columns 0-63)
+//   MMA  D2 = A W2   (N 64)
 //   epilogue 2       -> A (bf16), the layer-2 output in FP32 registers
-//   MMA  D3 = A W3   (N 128, TMEM columns 128-255)
-//   epilogue 3       -> G (FP32, shared), every column of the thread's row
-//   G^T R            -> X of the two atoms (FP32, shared)
+//   MMA  D3 = A W3   (N 128)
+//   epilogue 3       -> G, 32 columns at a time through the warp's part of A
+//   G^T R            -> X of the warp's atom (FP32, registers, lane = column)
+// With two atoms' sections concatenated over tiles, both nets restaged for
+// every pair of atoms, padding rows evaluated one by one and G of 128 rows in
+// shared memory (8 warps an SM), 6,141 atoms took 342 us forward and 306 us
+// backward; now 151 and 176 us, same bits.
 #include <cuda_bf16.h>
 
 #include <algorithm>
@@ -47,10 +50,6 @@ constexpr int kNetFwdBytes = kNetPar + 320 * 4;  // what the forward stages
 constexpr int kParW1 = 0, kParB1 = 64, kParB2 = 128, kParB3 = 192;
 
 constexpr int kRows = 128;
-// FP32 rows of G / dG in shared memory: an odd stride, so that a warp's
-// 32 rows writing one column hit 32 banks
-template <int N3>
-__host__ __device__ constexpr int gstride() { return N3 % 2 ? N3 : N3 + 1; }
 constexpr int kSlot = 26624;   // one staged net, forward part (1024-aligned)
 constexpr int kMaxTypes = 8;
 
@@ -187,266 +186,401 @@ struct Skip {
   }
 };
 
-// Epilogue 3 for one half of the D3 columns (G0 compile-time, so
-// that the skip reads h2 with static register indices): G row -> grow.
-template <int N2, int N3, int G0>
-__device__ __forceinline__ void epi3(uint32_t trow, const float* par, const float* h2, bool live,
-                                     float* grow) {
-  constexpr int NC = N3 > G0 * 64 ? ((N3 - G0 * 64 + 15) / 16 < 4 ? (N3 - G0 * 64 + 15) / 16 : 4)
-                                  : 0;  // 16-column chunks of this half
-  if constexpr (NC > 0) {
-  uint32_t v[4][16];
+// ------------------------------------------------------------ row mapping --
+// A tile's 128 rows are four slabs of 32, one per warp, each from that warp's
+// own atom: a CTA takes two units (four atoms) at a time, section by section,
+// and a warp walks its atom's section 32 rows a tile.  Padding slots repeat
+// one env row, and equal rows give equal embeddings: the rows from the first
+// of the equal ones at a section's end to its last slot are evaluated once
+// (water: some 30 and 60 of 46 and 92 rows).
+//
+// rows of section [s0, s0 + ns) of an atom to evaluate: 1 + the last row that
+// differs from the section's last row, plus one for the equal rest (NaN
+// differs from itself: every row)
+__device__ __forceinline__ int distinct_rows(const float4* __restrict__ em, int ns) {
+  const int lane = threadIdx.x & 31;
+  const float4 last = __ldg(em + ns - 1);
+  int top = -1;
+  for (int b = 0; b < ns; b += 128) {
+    bool ne[4];
 #pragma unroll
-  for (int c16 = 0; c16 < NC; ++c16) tmem_ld16_nw(trow + 128 + G0 * 64 + c16 * 16, v[c16]);
-  tmem_wait();
-#pragma unroll
-  for (int c16 = 0; c16 < NC; ++c16) {
-    const int m0 = G0 * 64 + c16 * 16;
-#pragma unroll
-    for (int k = 0; k < 16; ++k) {
-      const int m = m0 + k;
-      if (m < N3) {
-        float gv = 0.f;
-        if (live)
-          gv = tanh_fast(__uint_as_float(v[c16][k]) + par[kParB3 + m]) + Skip<N2, N3>::at(h2, m);
-        grow[m] = gv;
+    for (int u = 0; u < 4; ++u) {
+      const int j = b + 32 * u + lane;
+      ne[u] = false;
+      if (j < ns) {
+        const float4 e = __ldg(em + j);
+        ne[u] = !(e.x == last.x && e.y == last.y && e.z == last.z && e.w == last.w);
       }
     }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const unsigned m = __ballot_sync(kFull, ne[u]);
+      if (m) top = b + 32 * u + 31 - __clz(m);
+    }
   }
+  return min(ns, top + 2);
+}
+
+// the group's units that share nets: both in one pass, or (nets per centre
+// type and types differ) one pass each
+struct Group {
+  int atom;    // this warp's atom (-1: none)
+  int ti[2];   // centre type of each unit
+  bool both;
+};
+__device__ __forceinline__ Group load_group(const int* __restrict__ units,
+                                            const int* __restrict__ atype, int nunits, int g,
+                                            int warp, bool one_side) {
+  Group r;
+  const int u0 = 2 * g, u1 = u0 + 1;
+  const int mine = u0 + (warp >> 1);
+  r.atom = mine < nunits ? units[2 * mine + (warp & 1)] : -1;
+  r.ti[0] = atype[units[2 * u0]];
+  r.ti[1] = u1 < nunits ? atype[units[2 * u1]] : r.ti[0];
+  r.both = one_side || r.ti[0] == r.ti[1];
+  return r;
+}
+
+// 16 columns of a parameter row, read as float4 broadcasts
+__device__ __forceinline__ void par16(const float* par, float* v) {
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const float4 u = reinterpret_cast<const float4*>(par)[q];
+    v[4 * q] = u.x;
+    v[4 * q + 1] = u.y;
+    v[4 * q + 2] = u.z;
+    v[4 * q + 3] = u.w;
+  }
+}
+
+// Columns 32 C .. 32 C + 31 of epilogue 3: G = tanh(D3 + b3) + skip(h2) of
+// this lane's row into the warp's [32 rows][32 columns] buffer, 16-byte piece
+// p of row r at piece p ^ (r & 7) (stores of a row by its lane and loads of a
+// column by its lane both without bank conflicts)
+template <int N2, int N3, int C>
+__device__ __forceinline__ void epi3(uint32_t trow, const float* par, const float* h2,
+                                     float* gbuf) {
+  constexpr int NC = N3 - 32 * C >= 32 ? 2 : (N3 - 32 * C + 15) / 16;
+  const int lane = threadIdx.x & 31;
+  uint32_t v[NC][16];
+#pragma unroll
+  for (int c = 0; c < NC; ++c) tmem_ld16_nw(trow + 32 * C + 16 * c, v[c]);
+  tmem_wait();
+#pragma unroll
+  for (int c = 0; c < NC; ++c) {
+    float b[16], gv[16];
+    par16(par + kParB3 + 32 * C + 16 * c, b);
+#pragma unroll
+    for (int k = 0; k < 16; ++k) {
+      const int m = 32 * C + 16 * c + k;
+      gv[k] = m < N3 ? tanh_fast(__uint_as_float(v[c][k]) + b[k]) +
+                           Skip<N2, N3>::at(h2, m < N3 ? m : 0)
+                     : 0.f;
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      *reinterpret_cast<float4*>(gbuf + lane * 32 + (((4 * c + q) ^ (lane & 7)) << 2)) =
+          make_float4(gv[4 * q], gv[4 * q + 1], gv[4 * q + 2], gv[4 * q + 3]);
   }
 }
 
 // ---------------------------------------------------------------- kernel --
+// G^T R keeps the order of the sums of a 128-row tile of two concatenated
+// atoms: rows in ascending order in one chain of FMAs per column, broken
+// where (member of the unit) sel + row is a multiple of 128 (X feeds BF16
+// operands in the backward: another grouping would move their rounding).
 template <int N1, int N2, int N3>
-__global__ void __launch_bounds__(128, 2) k_emb_fwd(const __grid_constant__ EmbArgs p) {
+__global__ void __launch_bounds__(128, 3) k_emb_fwd(const __grid_constant__ EmbArgs p) {
   static_assert(N1 <= 32 && N2 <= 64 && N3 <= 128 && N3 >= 1, "embedding widths");
-  constexpr int kGStride = gstride<N3>();
+  constexpr int NCH = (N3 + 31) / 32;  // 32-column chunks
   extern __shared__ unsigned char smem_raw[];
   unsigned char* sm = reinterpret_cast<unsigned char*>(
       (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  unsigned char* slot = sm;                   // the staged net (one at a time)
-  unsigned char* atile = sm + kSlot;          // A operand, 16 KiB
-  float* gsm = reinterpret_cast<float*>(atile + 16384);   // [128][kGStride]
-  float* rsm = gsm + kRows * kGStride;                    // [128][4]
-  float* xacc = rsm + kRows * 4;                          // [2][4][128]
-  uint64_t* bar = reinterpret_cast<uint64_t*>(xacc + 2 * 4 * 128);
+  unsigned char* slots = sm;                  // two staged nets: section t in slot t & 1
+  unsigned char* atile = sm + 2 * kSlot;      // A operand, 16 KiB; a warp's quarter is its buffer
+  float4* rsm = reinterpret_cast<float4*>(atile + 16384);  // [128] env rows
+  uint64_t* bar = reinterpret_cast<uint64_t*>(rsm + kRows);
   uint32_t* tslot = reinterpret_cast<uint32_t*>(bar + 1);
-  int* cached = reinterpret_cast<int*>(tslot + 1);        // net index held by each slot
-  __shared__ float dred[8];                               // D-row bound: [warp][k, a] maxima
+  int* cached = reinterpret_cast<int*>(tslot + 1);  // [2] net held by each slot
+  int* nslab = cached + 2;                          // [4 warps] slabs of the section
 
-  const int tid = threadIdx.x, warp = tid >> 5;
-  const int r = tid;                       // this thread's tile row = TMEM lane
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int r = tid;  // this thread's tile row = TMEM lane
 
   if (tid == 0) {
     mbar_init(bar, 1);
     fence_mbar_init();
-    cached[0] = -1;
+    cached[0] = cached[1] = -1;
   }
   if (warp == 0) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 256;" ::"r"(
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 128;" ::"r"(
                      smem_addr(tslot))
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
-  for (int k = tid; k < 2 * 4 * 128; k += 128) xacc[k] = 0.f;
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = *tslot;
+  const uint32_t tmem = *tslot;  // D2 in columns 0 .. 63, then D3 in 0 .. 127
   const uint32_t trow = tmem + ((uint32_t)(warp * 32) << 16);
+  const uint32_t aaddr = smem_addr(atile);
+  float* gbuf = reinterpret_cast<float*>(atile + warp * 4096);
   unsigned phase = 0;
   bool alive = true;
-
-  const int per = (p.nunits + gridDim.x - 1) / gridDim.x;
-  const int u0 = blockIdx.x * per, u1 = min(p.nunits, u0 + per);
   const float inv_nnei = 1.f / (float)p.nnei;
+  const int ngroups = (p.nunits + 1) >> 1;
 
-  for (int u = u0; u < u1 && alive; ++u) {
-    const int at0 = p.units[2 * u], at1 = p.units[2 * u + 1];
-    const int na = at1 >= 0 ? 2 : 1;
-    const int ti = p.atype[at0];
-    for (int tj = 0; tj < p.ntypes && alive; ++tj) {
-      const int sel = p.sec[tj + 1] - p.sec[tj];
-      if (sel == 0) continue;
-      const int net = p.type_one_side ? tj : tj * p.ntypes + ti;
-      if (cached[0] != net) {  // uniform: stage this net's weights and params
+  for (int g = blockIdx.x; g < ngroups && alive; g += gridDim.x) {
+    const Group gr = load_group(p.units, p.atype, p.nunits, g, warp, p.type_one_side);
+    float2 xt[NCH][2];  // this lane's columns of X (sums), components (0, 1), (2, 3)
+#pragma unroll
+    for (int c = 0; c < NCH; ++c) xt[c][0] = xt[c][1] = make_float2(0.f, 0.f);
+    for (int pass = 0; pass < (gr.both ? 1 : 2) && alive; ++pass) {
+      const bool act = gr.atom >= 0 && (gr.both || (warp >> 1) == pass);
+      for (int tj = 0; tj < p.ntypes && alive; ++tj) {
+        const int sel = p.sec[tj + 1] - p.sec[tj];
+        if (sel == 0) continue;
+        const int net = p.type_one_side ? tj : tj * p.ntypes + gr.ti[pass];
+        unsigned char* slot = slots + (tj & 1) * kSlot;
+        const float4* em = reinterpret_cast<const float4*>(p.em) +
+                           (size_t)(act ? gr.atom : 0) * p.nnei + p.sec[tj];
+        const int neff = act ? distinct_rows(em, sel) : 0;
+        if (lane == 0) nslab[warp] = (neff + 31) >> 5;
         __syncthreads();
-        const uint4* src = reinterpret_cast<const uint4*>(p.nets + (size_t)net * kNetBytes);
-        uint4* dst = reinterpret_cast<uint4*>(slot);
-        for (int k = tid; k < kNetFwdBytes / 16; k += 128) dst[k] = __ldg(src + k);
-        fence_proxy_async_smem();
-        __syncthreads();
-        if (tid == 0) cached[0] = net;
-        __syncthreads();
-      }
-      const float* par = reinterpret_cast<const float*>(slot + kNetPar);
-      const uint32_t b2 = smem_addr(slot + kNetB2), b3 = smem_addr(slot + kNetB3);
-      const uint32_t aaddr = smem_addr(atile);
-      const int nr_all = na * sel;
-      for (int t0 = 0; t0 < nr_all && alive; t0 += kRows) {
-        const int nrow = min(kRows, nr_all - t0);
-        const bool live = r < nrow;
-        const int gi = t0 + r;
-        const int a = live ? gi / sel : 0;
+        const int nsl = max(max(nslab[0], nslab[1]), max(nslab[2], nslab[3]));
+        if (cached[tj & 1] != net) {  // uniform: stage this net's weights and params
+          const uint4* src = reinterpret_cast<const uint4*>(p.nets + (size_t)net * kNetBytes);
+          uint4* dst = reinterpret_cast<uint4*>(slot);
+          for (int k = tid; k < kNetFwdBytes / 16; k += 128) dst[k] = __ldg(src + k);
+          fence_proxy_async_smem();
+          __syncthreads();
+          if (tid == 0) cached[tj & 1] = net;
+        }
+        __syncthreads();  // nslab and cached read before they change again
+        const float* par = reinterpret_cast<const float*>(slot + kNetPar);
+        const uint32_t b2 = smem_addr(slot + kNetB2), b3 = smem_addr(slot + kNetB3);
+        float2 acc[NCH][2];
+#pragma unroll
+        for (int c = 0; c < NCH; ++c) acc[c][0] = acc[c][1] = make_float2(0.f, 0.f);
+        auto flush = [&](int c) {
+          xt[c][0] = make_float2(xt[c][0].x + acc[c][0].x, xt[c][0].y + acc[c][0].y);
+          xt[c][1] = make_float2(xt[c][1].x + acc[c][1].x, xt[c][1].y + acc[c][1].y);
+          acc[c][0] = acc[c][1] = make_float2(0.f, 0.f);
+        };
         float4 e = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (live) {
-          const int atom = a ? at1 : at0;
-          const int slot_j = p.sec[tj] + gi - a * sel;
-          e = __ldg(reinterpret_cast<const float4*>(p.em + ((size_t)atom * p.nnei + slot_j) * 4));
-        }
-        reinterpret_cast<float4*>(rsm)[r] = e;
-        // ---- layer 1 (FP32): h1 = tanh(s w1 + b1), all N1 columns per thread
-        float h1[N1];
+        if (lane < neff) e = __ldg(em + lane);
+        for (int sl = 0; sl < nsl && alive; ++sl) {
+          const int nrow = min(32, neff - 32 * sl);  // live rows of this warp (may be <= 0)
+          rsm[r] = e;
+          // ---- layer 1 (FP32): h1 = tanh(s w1 + b1), all N1 columns per thread
+          float h1[N1];
 #pragma unroll
-        for (int j = 0; j < N1; ++j) h1[j] = tanh_fast(fmaf(e.x, par[kParW1 + j], par[kParB1 + j]));
-        // A = h1 (bf16), the row's eight 16-byte pieces
-        st_half<N1, 0>(atile, r, h1);
-        st_half<N1, 1>(atile, r, h1);
-        fence_proxy_async_smem();
-        tc_fence_before();
-        __syncthreads();
-        if (tid == 0) {
-          tc_fence_after();
+          for (int j = 0; j < N1; ++j)
+            h1[j] = tanh_fast(fmaf(e.x, par[kParW1 + j], par[kParB1 + j]));
+          st_half<N1, 0>(atile, r, h1);
+          st_half<N1, 1>(atile, r, h1);
+          // the next slab's row
+          const int jn = 32 * (sl + 1) + lane;
+          e = jn < neff ? __ldg(em + jn) : make_float4(0.f, 0.f, 0.f, 0.f);
+          fence_proxy_async_smem();
+          tc_fence_before();
+          __syncthreads();
+          if (tid == 0) {
+            tc_fence_after();
 #pragma unroll
-          for (int kk = 0; kk < 4; ++kk)
-            umma_bf16(tmem, sdesc_sw128(aaddr + kk * 32), sdesc_sw128(b2 + kk * 32),
-                      idesc_bf16(64), kk > 0);
-          umma_commit(bar);
-        }
-        alive = __syncthreads_and(mbar_wait_bounded(bar, phase, p.status));
-        phase ^= 1u;
-        if (!alive) break;
-        tc_fence_after();
-        // ---- epilogue 2: h2 = tanh(D2 + b2) + skip(h1), all N2 columns
-        float h2[N2];
-        {
-          constexpr int NC = (N2 + 15) / 16;
-          uint32_t v[NC][16];
-#pragma unroll
-          for (int c16 = 0; c16 < NC; ++c16) tmem_ld16_nw(trow + c16 * 16, v[c16]);
-          tmem_wait();
-#pragma unroll
-          for (int c16 = 0; c16 < NC; ++c16)
-#pragma unroll
-            for (int k = 0; k < 16; ++k) {
-              const int j = c16 * 16 + k;
-              if (j < N2)
-                h2[j] = tanh_fast(__uint_as_float(v[c16][k]) + par[kParB2 + j]) +
-                        Skip<N1, N2>::at(h1, j);
-            }
-        }
-        tc_fence_before();
-        __syncthreads();  // every lane has read D2 and MMA 2 is done with A
-        st_half<N2, 0>(atile, r, h2);
-        st_half<N2, 1>(atile, r, h2);
-        fence_proxy_async_smem();
-        __syncthreads();
-        if (tid == 0) {
-          tc_fence_after();
-#pragma unroll
-          for (int kk = 0; kk < 4; ++kk)
-            umma_bf16(tmem + 128, sdesc_sw128(aaddr + kk * 32), sdesc_sw128(b3 + kk * 32),
-                      idesc_bf16(128), kk > 0);
-          umma_commit(bar);
-        }
-        alive = __syncthreads_and(mbar_wait_bounded(bar, phase, p.status));
-        phase ^= 1u;
-        if (!alive) break;
-        tc_fence_after();
-        // ---- epilogue 3: G = tanh(D3 + b3) + skip(h2), both column halves
-        epi3<N2, N3, 0>(trow, par, h2, live, gsm + r * kGStride);
-        epi3<N2, N3, 1>(trow, par, h2, live, gsm + r * kGStride);
-        tc_fence_before();
-        __syncthreads();
-        // ---- G^T R: thread m, for each atom over that atom's tile rows
-        for (int ah = 0; ah < na; ++ah) {
-          const int m = tid;
-          if (m < N3) {
-            const int lo = max(0, ah * sel - t0), hi = min(nrow, (ah + 1) * sel - t0);
-            float acc[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll 4
-            for (int rr = lo; rr < hi; ++rr) {
-              const float4 R = reinterpret_cast<const float4*>(rsm)[rr];
-              const float gv = gsm[rr * kGStride + m];
-              acc[0] = fmaf(R.x, gv, acc[0]);
-              acc[1] = fmaf(R.y, gv, acc[1]);
-              acc[2] = fmaf(R.z, gv, acc[2]);
-              acc[3] = fmaf(R.w, gv, acc[3]);
-            }
-#pragma unroll
-            for (int c = 0; c < 4; ++c) xacc[(ah * 4 + c) * 128 + m] += acc[c];
+            for (int kk = 0; kk < 4; ++kk)
+              umma_bf16(tmem, sdesc_sw128(aaddr + kk * 32), sdesc_sw128(b2 + kk * 32),
+                        idesc_bf16(64), kk > 0);
+            umma_commit(bar);
           }
+          alive = __syncthreads_and(mbar_wait_bounded(bar, phase, p.status));
+          phase ^= 1u;
+          if (!alive) break;
+          tc_fence_after();
+          // ---- epilogue 2: h2 = tanh(D2 + b2) + skip(h1), all N2 columns
+          float h2[N2];
+          {
+            constexpr int NC = (N2 + 15) / 16;
+            uint32_t v[NC][16];
+#pragma unroll
+            for (int c = 0; c < NC; ++c) tmem_ld16_nw(trow + c * 16, v[c]);
+            tmem_wait();
+#pragma unroll
+            for (int c = 0; c < NC; ++c) {
+              float b[16];
+              par16(par + kParB2 + 16 * c, b);
+#pragma unroll
+              for (int k = 0; k < 16; ++k) {
+                const int j = c * 16 + k;
+                if (j < N2)
+                  h2[j] = tanh_fast(__uint_as_float(v[c][k]) + b[k]) + Skip<N1, N2>::at(h1, j);
+              }
+            }
+          }
+          // MMA 2 is done with A and a warp rewrites only its own rows; the
+          // barrier orders every warp's D2 loads and A stores before MMA 3
+          st_half<N2, 0>(atile, r, h2);
+          st_half<N2, 1>(atile, r, h2);
+          fence_proxy_async_smem();
+          tc_fence_before();
+          __syncthreads();
+          if (tid == 0) {
+            tc_fence_after();
+#pragma unroll
+            for (int kk = 0; kk < 4; ++kk)
+              umma_bf16(tmem, sdesc_sw128(aaddr + kk * 32), sdesc_sw128(b3 + kk * 32),
+                        idesc_bf16(128), kk > 0);
+            umma_commit(bar);
+          }
+          alive = __syncthreads_and(mbar_wait_bounded(bar, phase, p.status));
+          phase ^= 1u;
+          if (!alive) break;
+          tc_fence_after();
+          // ---- epilogue 3 and G^T R, 32 columns at a time: a lane per column
+          //      over the warp's rows, through the warp's quarter of A (MMA 3
+          //      is done with it)
+          if (nrow > 0) {  // uniform over the warp
+            const float4* R = rsm + warp * 32;
+            const int pos = (warp & 1) * sel + 32 * sl;
+            const int brk = (128 - (pos & 127)) & 127;  // row before which the chain breaks
+            const bool tail = 32 * sl + nrow == neff;   // the last row stands for the equal rest
+            const int plain = tail ? nrow - 1 : nrow;
+            float gt[NCH];
+            auto chunk = [&](int c) {
+              auto rows = [&](int lo, int hi) {
+#pragma unroll 4
+                for (int rr = lo; rr < hi; ++rr) {
+                  const float gv = gbuf[rr * 32 + ((((lane >> 2) ^ (rr & 7)) << 2) | (lane & 3))];
+                  const float4 q = R[rr];
+                  acc[c][0] = __ffma2_rn(lo2(q), dup2(gv), acc[c][0]);
+                  acc[c][1] = __ffma2_rn(hi2(q), dup2(gv), acc[c][1]);
+                }
+              };
+              if (brk < plain) {
+                rows(0, brk);
+                flush(c);
+                rows(brk, plain);
+              } else {
+                rows(0, plain);
+              }
+              const int rr = nrow - 1;
+              gt[c] = gbuf[rr * 32 + ((((lane >> 2) ^ (rr & 7)) << 2) | (lane & 3))];
+            };
+            __syncwarp();
+            epi3<N2, N3, 0>(trow, par, h2, gbuf);
+            __syncwarp();
+            chunk(0);
+            if constexpr (NCH > 1) {
+              __syncwarp();
+              epi3<N2, N3, 1>(trow, par, h2, gbuf);
+              __syncwarp();
+              chunk(1);
+            }
+            if constexpr (NCH > 2) {
+              __syncwarp();
+              epi3<N2, N3, 2>(trow, par, h2, gbuf);
+              __syncwarp();
+              chunk(2);
+            }
+            if constexpr (NCH > 3) {
+              __syncwarp();
+              epi3<N2, N3, 3>(trow, par, h2, gbuf);
+              __syncwarp();
+              chunk(3);
+            }
+            if (tail) {
+              const float4 q = R[nrow - 1];
+              const bool one = q.y == 0.f && q.z == 0.f && q.w == 0.f;  // a padding row
+              int at = (warp & 1) * sel + neff - 1;
+              for (int left = sel - neff + 1; left > 0;) {
+                if ((at & 127) == 0)
+#pragma unroll
+                  for (int c = 0; c < NCH; ++c) flush(c);
+                const int n = min(left, 128 - (at & 127));
+                if (one) {
+                  for (int k = 0; k < n; ++k)
+#pragma unroll
+                    for (int c = 0; c < NCH; ++c) acc[c][0].x = fmaf(q.x, gt[c], acc[c][0].x);
+                } else {
+                  for (int k = 0; k < n; ++k)
+#pragma unroll
+                    for (int c = 0; c < NCH; ++c) {
+                      acc[c][0] = __ffma2_rn(lo2(q), dup2(gt[c]), acc[c][0]);
+                      acc[c][1] = __ffma2_rn(hi2(q), dup2(gt[c]), acc[c][1]);
+                    }
+                }
+                at += n;
+                left -= n;
+              }
+            }
+            __syncwarp();
+          }
+          tc_fence_before();
         }
-        __syncthreads();
+#pragma unroll
+        for (int c = 0; c < NCH; ++c) flush(c);
       }
     }
     if (!alive) break;
-    // ---- X and D of the unit's atoms
-    for (int ah = 0; ah < na; ++ah) {
-      const int m = tid;
-      const int atom = ah ? at1 : at0;
-      const size_t row = p.drow ? (size_t)p.drow[atom] : (size_t)atom;
-      float xm[4] = {0.f, 0.f, 0.f, 0.f};
-      if (m < N3) {
+    // ---- X and D of this warp's atom
+    if (gr.atom >= 0) {
+      const size_t row = p.drow ? (size_t)p.drow[gr.atom] : (size_t)gr.atom;
+      float4* xT = reinterpret_cast<float4*>(gbuf);
+      float nk = 0.f, na = 0.f;
+      __syncwarp();
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          xm[c] = xacc[(ah * 4 + c) * 128 + m] * inv_nnei;
-          p.X[((size_t)atom * 4 + c) * N3 + m] = xm[c];
+      for (int c = 0; c < NCH; ++c) {
+        const int m = 32 * c + lane;
+        if (m < N3) {
+          const float4 x = make_float4(xt[c][0].x * inv_nnei, xt[c][0].y * inv_nnei,
+                                       xt[c][1].x * inv_nnei, xt[c][1].y * inv_nnei);
+          xT[m] = x;
+          float* Xa = p.X + (size_t)gr.atom * 4 * N3 + m;
+          Xa[0] = x.x;
+          Xa[N3] = x.y;
+          Xa[2 * N3] = x.z;
+          Xa[3 * N3] = x.w;
+          const float q = x.x * x.x + x.y * x.y + x.z * x.z + x.w * x.w;
+          nk = fmaxf(nk, q);
+          if (m < p.A) na = fmaxf(na, q);
         }
       }
+      __syncwarp();
+      auto dval = [&](int m, int a) {
+        const float4 u = xT[m], w = xT[a];
+        return fmaf(u.w, w.w, fmaf(u.z, w.z, fmaf(u.y, w.y, fmaf(u.x, w.x, 0.f))));
+      };
       if (p.D_lo) {
         // split for the tensor-core fitting: FP16 hi / lo of c D, c = 2^s
         // from |D_ka| <= |X_k| |X_a| (Cauchy-Schwarz over the 4 rows of X)
-        const float q = xm[0] * xm[0] + xm[1] * xm[1] + xm[2] * xm[2] + xm[3] * xm[3];
-        float qk = q, qa = m < p.A ? q : 0.f;
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) {
-          qk = fmaxf(qk, __shfl_xor_sync(kFull, qk, o));
-          qa = fmaxf(qa, __shfl_xor_sync(kFull, qa, o));
+          nk = fmaxf(nk, __shfl_xor_sync(kFull, nk, o));
+          na = fmaxf(na, __shfl_xor_sync(kFull, na, o));
         }
-        if ((tid & 31) == 0) {
-          dred[warp * 2] = qk;
-          dred[warp * 2 + 1] = qa;
+        const float sc = f16_scale_for(sqrtf(nk * na) * 1.0001f);
+        __half* dh = static_cast<__half*>(p.D) + row * (size_t)N3 * p.A;
+        __half* dl = static_cast<__half*>(p.D_lo) + row * (size_t)N3 * p.A;
+        for (int at = 4 * lane; at < N3 * p.A; at += 128) {
+          const int m = at / p.A, a = at - m * p.A;
+          const float v[4] = {dval(m, a), dval(m, a + 1), dval(m, a + 2), dval(m, a + 3)};
+          st_split4_f16(dh + at, dl + at, v, sc);
         }
-        __syncthreads();
-        qk = fmaxf(fmaxf(dred[0], dred[2]), fmaxf(dred[4], dred[6]));
-        qa = fmaxf(fmaxf(dred[1], dred[3]), fmaxf(dred[5], dred[7]));
-        __syncthreads();  // dred is reused by the next atom
-        const float sc = f16_scale_for(sqrtf(qk * qa) * 1.0001f);
-        if (m < N3) {
-          __half* dh = static_cast<__half*>(p.D) + row * (size_t)N3 * p.A + (size_t)m * p.A;
-          __half* dl = static_cast<__half*>(p.D_lo) + row * (size_t)N3 * p.A + (size_t)m * p.A;
-          for (int a2 = 0; a2 < p.A; a2 += 4) {
-            float v[4];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              v[j] = 0.f;
-#pragma unroll
-              for (int c = 0; c < 4; ++c)
-                v[j] = fmaf(xm[c], xacc[(ah * 4 + c) * 128 + a2 + j] * inv_nnei, v[j]);
-            }
-            st_split4_f16(dh + a2, dl + a2, v, sc);
-          }
-        }
-        if (tid == 0) p.D_rs[row] = 1.f / sc;
-      } else if (m < N3) {
-        float* d = static_cast<float*>(p.D) + row * (size_t)N3 * p.A + (size_t)m * p.A;
-        for (int a2 = 0; a2 < p.A; ++a2) {
-          float v = 0.f;
-#pragma unroll
-          for (int c = 0; c < 4; ++c) v = fmaf(xm[c], xacc[(ah * 4 + c) * 128 + a2] * inv_nnei, v);
-          d[a2] = v;
+        if (lane == 0) p.D_rs[row] = 1.f / sc;
+      } else {
+        float* d = static_cast<float*>(p.D) + row * (size_t)N3 * p.A;
+        for (int at = lane; at < N3 * p.A; at += 32) {
+          const int m = at / p.A;
+          d[at] = dval(m, at - m * p.A);
         }
       }
+      __syncwarp();
     }
-    __syncthreads();
-    for (int k = tid; k < 2 * 4 * 128; k += 128) xacc[k] = 0.f;
-    __syncthreads();
   }
   tc_fence_before();
   __syncthreads();
   if (warp == 0)
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 256;" ::"r"(tmem) : "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 128;" ::"r"(tmem) : "memory");
 }
 
 // ------------------------------------------------------------- backward --
@@ -598,7 +732,7 @@ constexpr int kBwdSlot = kNetBytes;  // the whole net block (forward and transpo
 // operand (bf16, chunk G0).
 template <int N1, int N2, int N3, int G0>
 __device__ __forceinline__ void bepi3(uint32_t trow, const float* par, const float* t2,
-                                      const float* h1, bool live, float4 R, const float* dx,
+                                      const float* h1, bool live, float4 R, const float4* dx,
                                       float* sk, unsigned char* atile, int r, float* dr) {
   unsigned char* chunk = atile + G0 * 16384;
 #pragma unroll
@@ -622,7 +756,8 @@ __device__ __forceinline__ void bepi3(uint32_t trow, const float* par, const flo
             const int j = m < N2 ? m : m - N2;
             gv += t2[j] + Skip<N1, N2>::at(h1, j);
           }
-          const float d0 = dx[m], d1 = dx[128 + m], d2 = dx[256 + m], d3 = dx[384 + m];
+          const float4 q = dx[m];
+          const float d0 = q.x, d1 = q.y, d2 = q.z, d3 = q.w;
           const float dg = R.x * d0 + R.y * d1 + R.z * d2 + R.w * d3;
           dr[0] = fmaf(gv, d0, dr[0]);
           dr[1] = fmaf(gv, d1, dr[1]);
@@ -647,12 +782,13 @@ __global__ void __launch_bounds__(128, 2) k_emb_bwd(const __grid_constant__ EmbB
       (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   unsigned char* slot = sm;                      // one staged net (all images)
   unsigned char* atile = sm + kBwdSlot;          // A operand, 2 chunks of 16 KiB
-  float* dxsm = reinterpret_cast<float*>(atile + 32768);  // [2 atoms][4][128]
-  uint64_t* bar = reinterpret_cast<uint64_t*>(dxsm + 2 * 4 * 128);
+  float4* dxsm = reinterpret_cast<float4*>(atile + 32768);  // [4 warps][128]: dX^T of its atom
+  uint64_t* bar = reinterpret_cast<uint64_t*>(dxsm + 4 * 128);
   uint32_t* tslot = reinterpret_cast<uint32_t*>(bar + 1);
   int* cached = reinterpret_cast<int*>(tslot + 1);
+  int* nslab = cached + 1;  // [4 warps] slabs of the section
 
-  const int tid = threadIdx.x, warp = tid >> 5;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int r = tid;  // this thread's tile row = TMEM lane
 
   if (tid == 0) {
@@ -674,191 +810,201 @@ __global__ void __launch_bounds__(128, 2) k_emb_bwd(const __grid_constant__ EmbB
   unsigned phase = 0;
   bool alive = true;
 
-  const int per = (p.nunits + gridDim.x - 1) / gridDim.x;
-  const int u0 = blockIdx.x * per, u1 = min(p.nunits, u0 + per);
   const uint32_t aaddr = smem_addr(atile);
+  float4* dx = dxsm + warp * 128;
+  const int ngroups = (p.nunits + 1) >> 1;
 
   for (int tj = 0; tj < p.ntypes && alive; ++tj) {
     const int sel = p.sec[tj + 1] - p.sec[tj];
     if (sel == 0) continue;
-    for (int u = u0; u < u1 && alive; ++u) {
-      const int at0 = p.units[2 * u], at1 = p.units[2 * u + 1];
-      const int na = at1 >= 0 ? 2 : 1;
-      const int ti = p.atype[at0];
-      const int net = p.type_one_side ? tj : tj * p.ntypes + ti;
-      __syncthreads();  // the previous unit is done with the shared buffers
-      if (cached[0] != net) {
-        const uint4* src = reinterpret_cast<const uint4*>(p.nets + (size_t)net * kNetBytes);
-        uint4* dst = reinterpret_cast<uint4*>(slot);
-        for (int k = tid; k < kNetBytes / 16; k += 128) dst[k] = __ldg(src + k);
-        fence_proxy_async_smem();
-        __syncthreads();
-        if (tid == 0) cached[0] = net;
-      }
-      for (int k = tid; k < 2 * 4 * 128; k += 128) {
-        const int ah = k >> 9, c = (k >> 7) & 3, m = k & 127;
-        float v = 0.f;
-        if (ah < na && m < N3) v = p.dxs[((size_t)(ah ? at1 : at0) * 4 + c) * N3 + m];
-        dxsm[k] = v;
-      }
-      __syncthreads();
-      const float* par = reinterpret_cast<const float*>(slot + kNetPar);
-      const uint32_t b2 = smem_addr(slot + kNetB2), b3 = smem_addr(slot + kNetB3);
-      const uint32_t b3t = smem_addr(slot + kNetB3T), b2t = smem_addr(slot + kNetB2T);
-      const int nr_all = na * sel;
-      for (int t0 = 0; t0 < nr_all && alive; t0 += kRows) {
-        const int nrow = min(kRows, nr_all - t0);
-        const bool live = r < nrow;
-        const int gi = t0 + r;
-        const int a = live ? gi / sel : 0;
-        const int atom = a ? at1 : at0;
-        const int slot_j = p.sec[tj] + gi - a * sel;
-        float4 e = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (live)
-          e = __ldg(reinterpret_cast<const float4*>(p.em + ((size_t)atom * p.nnei + slot_j) * 4));
-        // ---- forward recompute: layer 1, MMA 2, epilogue 2, MMA 3
-        float h1[N1];
-#pragma unroll
-        for (int j = 0; j < N1; ++j) h1[j] = tanh_fast(fmaf(e.x, par[kParW1 + j], par[kParB1 + j]));
-        st_half<N1, 0>(atile, r, h1);
-        st_half<N1, 1>(atile, r, h1);
-        fence_proxy_async_smem();
-        tc_fence_before();
-        __syncthreads();
-        if (tid == 0) {
-          tc_fence_after();
-#pragma unroll
-          for (int kk = 0; kk < 4; ++kk)
-            umma_bf16(tmem, sdesc_sw128(aaddr + kk * 32), sdesc_sw128(b2 + kk * 32),
-                      idesc_bf16(64), kk > 0);
-          umma_commit(bar);
-        }
-        alive = __syncthreads_and(mbar_wait_bounded(bar, phase, p.status));
-        phase ^= 1u;
-        if (!alive) break;
-        tc_fence_after();
-        float t2[N2];
-#pragma unroll
-        for (int c16 = 0; c16 < (N2 + 15) / 16; ++c16) {
-          float v[16];
-          tmem_ld16(trow + c16 * 16, v);
-#pragma unroll
-          for (int k = 0; k < 16; ++k) {
-            const int j = c16 * 16 + k;
-            if (j < N2) t2[j] = tanh_fast(v[k] + par[kParB2 + j]);
+    for (int g = blockIdx.x; g < ngroups && alive; g += gridDim.x) {
+      const Group gr = load_group(p.units, p.atype, p.nunits, g, warp, p.type_one_side);
+      for (int pass = 0; pass < (gr.both ? 1 : 2) && alive; ++pass) {
+        const bool act = gr.atom >= 0 && (gr.both || (warp >> 1) == pass);
+        const int net = p.type_one_side ? tj : tj * p.ntypes + gr.ti[pass];
+        const size_t row0 = (size_t)(act ? gr.atom : 0) * p.nnei + p.sec[tj];
+        const float4* em = reinterpret_cast<const float4*>(p.em) + row0;
+        float4* out = reinterpret_cast<float4*>(p.net) + row0;
+        const int neff = act ? distinct_rows(em, sel) : 0;
+        if (lane == 0) nslab[warp] = (neff + 31) >> 5;
+        if (act)
+          for (int m = lane; m < N3; m += 32) {
+            const float* d = p.dxs + (size_t)gr.atom * 4 * N3 + m;
+            dx[m] = make_float4(d[0], d[N3], d[2 * N3], d[3 * N3]);
           }
+        __syncthreads();  // (and the previous group is done with the shared buffers)
+        const int nsl = max(max(nslab[0], nslab[1]), max(nslab[2], nslab[3]));
+        if (cached[0] != net) {
+          const uint4* src = reinterpret_cast<const uint4*>(p.nets + (size_t)net * kNetBytes);
+          uint4* dst = reinterpret_cast<uint4*>(slot);
+          for (int k = tid; k < kNetBytes / 16; k += 128) dst[k] = __ldg(src + k);
+          fence_proxy_async_smem();
+          __syncthreads();
+          if (tid == 0) cached[0] = net;
         }
-        tc_fence_before();
-        __syncthreads();
-        {
-          float h2[N2];
-#pragma unroll
-          for (int j = 0; j < N2; ++j) h2[j] = t2[j] + Skip<N1, N2>::at(h1, j);
-          st_half<N2, 0>(atile, r, h2);
-          st_half<N2, 1>(atile, r, h2);
-        }
-        fence_proxy_async_smem();
-        __syncthreads();
-        if (tid == 0) {
-          tc_fence_after();
-#pragma unroll
-          for (int kk = 0; kk < 4; ++kk)
-            umma_bf16(tmem + 128, sdesc_sw128(aaddr + kk * 32), sdesc_sw128(b3 + kk * 32),
-                      idesc_bf16(128), kk > 0);
-          umma_commit(bar);
-        }
-        alive = __syncthreads_and(mbar_wait_bounded(bar, phase, p.status));
-        phase ^= 1u;
-        if (!alive) break;
-        tc_fence_after();
-        // ---- backward epilogue 3: dG, dR, the skip gradient, dZ3 -> A (K = 128)
-        float dr[4] = {0.f, 0.f, 0.f, 0.f};
-        float sk[N2];
-#pragma unroll
-        for (int j = 0; j < N2; ++j) sk[j] = 0.f;
-        const float* dx = dxsm + a * 512;
-        bepi3<N1, N2, N3, 0>(trow, par, t2, h1, live, e, dx, sk, atile, r, dr);
-        bepi3<N1, N2, N3, 1>(trow, par, t2, h1, live, e, dx, sk, atile, r, dr);
-        fence_proxy_async_smem();
-        tc_fence_before();
-        __syncthreads();
-        if (tid == 0) {  // dH2 (partial) = dZ3 W3: K = 128 in two 64-column chunks
-          tc_fence_after();
-#pragma unroll
-          for (int kk = 0; kk < 8; ++kk) {
-            const uint32_t ca = aaddr + (kk >> 2) * 16384 + (kk & 3) * 32;
-            const uint32_t cb = b3t + (kk >> 2) * 8192 + (kk & 3) * 32;
-            umma_bf16(tmem, sdesc_sw128(ca), sdesc_sw128(cb), idesc_bf16(64), kk > 0);
+        __syncthreads();  // nslab and cached read before they change again
+        const float* par = reinterpret_cast<const float*>(slot + kNetPar);
+        const uint32_t b2 = smem_addr(slot + kNetB2), b3 = smem_addr(slot + kNetB3);
+        const uint32_t b3t = smem_addr(slot + kNetB3T), b2t = smem_addr(slot + kNetB2T);
+        float4 en = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (lane < neff) en = __ldg(em + lane);
+        for (int sl = 0; sl < nsl && alive; ++sl) {
+          const int j = 32 * sl + lane;
+          const bool live = j < neff;
+          const float4 e = en;
+          en = j + 32 < neff ? __ldg(em + j + 32) : make_float4(0.f, 0.f, 0.f, 0.f);
+          // ---- forward recompute: layer 1, MMA 2, epilogue 2, MMA 3
+          float h1[N1];
+  #pragma unroll
+          for (int j = 0; j < N1; ++j) h1[j] = tanh_fast(fmaf(e.x, par[kParW1 + j], par[kParB1 + j]));
+          st_half<N1, 0>(atile, r, h1);
+          st_half<N1, 1>(atile, r, h1);
+          fence_proxy_async_smem();
+          tc_fence_before();
+          __syncthreads();
+          if (tid == 0) {
+            tc_fence_after();
+  #pragma unroll
+            for (int kk = 0; kk < 4; ++kk)
+              umma_bf16(tmem, sdesc_sw128(aaddr + kk * 32), sdesc_sw128(b2 + kk * 32),
+                        idesc_bf16(64), kk > 0);
+            umma_commit(bar);
           }
-          umma_commit(bar);
-        }
-        alive = __syncthreads_and(mbar_wait_bounded(bar, phase, p.status));
-        phase ^= 1u;
-        if (!alive) break;
-        tc_fence_after();
-        // ---- epilogue 4: dH2 = dZ3 W3 + skip(dG), dZ2 = dH2 (1 - t2^2)
-        float sb1[N1];  // t2 becomes dZ2 in place
-        {
-          float dh2[N2];
-#pragma unroll
+          alive = __syncthreads_and(mbar_wait_bounded(bar, phase, p.status));
+          phase ^= 1u;
+          if (!alive) break;
+          tc_fence_after();
+          float t2[N2];
+  #pragma unroll
           for (int c16 = 0; c16 < (N2 + 15) / 16; ++c16) {
             float v[16];
             tmem_ld16(trow + c16 * 16, v);
-#pragma unroll
+  #pragma unroll
             for (int k = 0; k < 16; ++k) {
               const int j = c16 * 16 + k;
-              if (j < N2) {
-                dh2[j] = v[k] + sk[j];
-                t2[j] = dh2[j] * (1.f - t2[j] * t2[j]);
+              if (j < N2) t2[j] = tanh_fast(v[k] + par[kParB2 + j]);
+            }
+          }
+          tc_fence_before();
+          __syncthreads();
+          {
+            float h2[N2];
+  #pragma unroll
+            for (int j = 0; j < N2; ++j) h2[j] = t2[j] + Skip<N1, N2>::at(h1, j);
+            st_half<N2, 0>(atile, r, h2);
+            st_half<N2, 1>(atile, r, h2);
+          }
+          fence_proxy_async_smem();
+          __syncthreads();
+          if (tid == 0) {
+            tc_fence_after();
+  #pragma unroll
+            for (int kk = 0; kk < 4; ++kk)
+              umma_bf16(tmem + 128, sdesc_sw128(aaddr + kk * 32), sdesc_sw128(b3 + kk * 32),
+                        idesc_bf16(128), kk > 0);
+            umma_commit(bar);
+          }
+          alive = __syncthreads_and(mbar_wait_bounded(bar, phase, p.status));
+          phase ^= 1u;
+          if (!alive) break;
+          tc_fence_after();
+          // ---- backward epilogue 3: dG, dR, the skip gradient, dZ3 -> A (K = 128)
+          float dr[4] = {0.f, 0.f, 0.f, 0.f};
+          float sk[N2];
+  #pragma unroll
+          for (int j = 0; j < N2; ++j) sk[j] = 0.f;
+          bepi3<N1, N2, N3, 0>(trow, par, t2, h1, live, e, dx, sk, atile, r, dr);
+          bepi3<N1, N2, N3, 1>(trow, par, t2, h1, live, e, dx, sk, atile, r, dr);
+          fence_proxy_async_smem();
+          tc_fence_before();
+          __syncthreads();
+          if (tid == 0) {  // dH2 (partial) = dZ3 W3: K = 128 in two 64-column chunks
+            tc_fence_after();
+  #pragma unroll
+            for (int kk = 0; kk < 8; ++kk) {
+              const uint32_t ca = aaddr + (kk >> 2) * 16384 + (kk & 3) * 32;
+              const uint32_t cb = b3t + (kk >> 2) * 8192 + (kk & 3) * 32;
+              umma_bf16(tmem, sdesc_sw128(ca), sdesc_sw128(cb), idesc_bf16(64), kk > 0);
+            }
+            umma_commit(bar);
+          }
+          alive = __syncthreads_and(mbar_wait_bounded(bar, phase, p.status));
+          phase ^= 1u;
+          if (!alive) break;
+          tc_fence_after();
+          // ---- epilogue 4: dH2 = dZ3 W3 + skip(dG), dZ2 = dH2 (1 - t2^2)
+          float sb1[N1];  // t2 becomes dZ2 in place
+          {
+            float dh2[N2];
+  #pragma unroll
+            for (int c16 = 0; c16 < (N2 + 15) / 16; ++c16) {
+              float v[16];
+              tmem_ld16(trow + c16 * 16, v);
+  #pragma unroll
+              for (int k = 0; k < 16; ++k) {
+                const int j = c16 * 16 + k;
+                if (j < N2) {
+                  dh2[j] = v[k] + sk[j];
+                  t2[j] = dh2[j] * (1.f - t2[j] * t2[j]);
+                }
+              }
+            }
+  #pragma unroll
+            for (int j = 0; j < N1; ++j) {
+              float sk = 0.f;
+              if (Skip<N1, N2>::kind == 1) sk = dh2[j];
+              if (Skip<N1, N2>::kind == 2) sk = dh2[j] + dh2[j + N1];
+              sb1[j] = sk;
+            }
+          }
+          tc_fence_before();
+          __syncthreads();  // MMA 4 done with A; every lane has read D4
+          st_half<N2, 0>(atile, r, t2);
+          st_half<N2, 1>(atile, r, t2);
+          fence_proxy_async_smem();
+          __syncthreads();
+          if (tid == 0) {  // dH1 (partial) = dZ2 W2
+            tc_fence_after();
+  #pragma unroll
+            for (int kk = 0; kk < 4; ++kk)
+              umma_bf16(tmem + 64, sdesc_sw128(aaddr + kk * 32), sdesc_sw128(b2t + kk * 32),
+                        idesc_bf16(64), kk > 0);
+            umma_commit(bar);
+          }
+          alive = __syncthreads_and(mbar_wait_bounded(bar, phase, p.status));
+          phase ^= 1u;
+          if (!alive) break;
+          tc_fence_after();
+          // ---- epilogue 5: dZ1, ds, and the env-matrix gradient of the row
+          float ds = 0.f;
+  #pragma unroll
+          for (int c16 = 0; c16 < (N1 + 15) / 16; ++c16) {
+            float v[16];
+            tmem_ld16(trow + 64 + c16 * 16, v);
+  #pragma unroll
+            for (int k = 0; k < 16; ++k) {
+              const int j = c16 * 16 + k;
+              if (j < N1) {
+                const float dz1 = (v[k] + sb1[j]) * (1.f - h1[j] * h1[j]);
+                ds = fmaf(dz1, par[kParW1 + j], ds);
               }
             }
           }
-#pragma unroll
-          for (int j = 0; j < N1; ++j) {
-            float sk = 0.f;
-            if (Skip<N1, N2>::kind == 1) sk = dh2[j];
-            if (Skip<N1, N2>::kind == 2) sk = dh2[j] + dh2[j + N1];
-            sb1[j] = sk;
-          }
-        }
-        tc_fence_before();
-        __syncthreads();  // MMA 4 done with A; every lane has read D4
-        st_half<N2, 0>(atile, r, t2);
-        st_half<N2, 1>(atile, r, t2);
-        fence_proxy_async_smem();
-        __syncthreads();
-        if (tid == 0) {  // dH1 (partial) = dZ2 W2
-          tc_fence_after();
-#pragma unroll
-          for (int kk = 0; kk < 4; ++kk)
-            umma_bf16(tmem + 64, sdesc_sw128(aaddr + kk * 32), sdesc_sw128(b2t + kk * 32),
-                      idesc_bf16(64), kk > 0);
-          umma_commit(bar);
-        }
-        alive = __syncthreads_and(mbar_wait_bounded(bar, phase, p.status));
-        phase ^= 1u;
-        if (!alive) break;
-        tc_fence_after();
-        // ---- epilogue 5: dZ1, ds, and the env-matrix gradient of the row
-        float ds = 0.f;
-#pragma unroll
-        for (int c16 = 0; c16 < (N1 + 15) / 16; ++c16) {
-          float v[16];
-          tmem_ld16(trow + 64 + c16 * 16, v);
-#pragma unroll
-          for (int k = 0; k < 16; ++k) {
-            const int j = c16 * 16 + k;
-            if (j < N1) {
-              const float dz1 = (v[k] + sb1[j]) * (1.f - h1[j] * h1[j]);
-              ds = fmaf(dz1, par[kParW1 + j], ds);
+          {
+            const float4 o = make_float4(ds + dr[0], dr[1], dr[2], dr[3]);
+            if (live) out[j] = o;
+            // the last row's gradient is that of the equal rows after it too
+            const int tl = neff - 1 - 32 * sl;
+            if (tl >= 0 && tl < 32) {  // uniform over the warp
+              const float4 q = make_float4(
+                  __shfl_sync(kFull, o.x, tl), __shfl_sync(kFull, o.y, tl),
+                  __shfl_sync(kFull, o.z, tl), __shfl_sync(kFull, o.w, tl));
+              for (int k = neff + lane; k < sel; k += 32) out[k] = q;
             }
           }
+          tc_fence_before();
+          __syncthreads();  // every lane has read D5 before the next tile
         }
-        if (live)
-          *reinterpret_cast<float4*>(p.net + ((size_t)atom * p.nnei + slot_j) * 4) =
-              make_float4(ds + dr[0], dr[1], dr[2], dr[3]);
-        tc_fence_before();
-        __syncthreads();  // every lane has read D5 before the next tile
       }
     }
   }
@@ -868,10 +1014,10 @@ __global__ void __launch_bounds__(128, 2) k_emb_bwd(const __grid_constant__ EmbB
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 256;" ::"r"(tmem) : "memory");
 }
 
-// about 88 KiB: two CTAs per SM (2 x 256 TMEM columns)
+// 92 KiB: two CTAs per SM (2 x 256 TMEM columns)
 template <int N3>
 constexpr size_t bwd_smem() {
-  return 1024 + kBwdSlot + 32768 + 2 * 4 * 128 * 4 + 64;
+  return 1024 + kBwdSlot + 32768 + 4 * 128 * 16 + 64;
 }
 
 template <int N1, int N2, int N3>
@@ -892,24 +1038,20 @@ int emb_bwd_launch(const EmbBwdArgs& a, cudaStream_t st) {
   int dev = 0, sms = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const int grid = std::max(1, std::min(2 * sms, a.nunits));
+  const int grid = std::max(1, std::min(2 * sms, (a.nunits + 1) / 2));
   kern<<<grid, 128, smem, st>>>(a);
   GBDP_CHECK_LAUNCH("embed_bwd_tc");
   return GBDP_OK;
 }
 
-// about 100 KiB for N3 = 100: two CTAs per SM (2 x 256 TMEM columns)
-template <int N3>
-constexpr size_t fwd_smem() {
-  return 1024 + kSlot + 16384 + (size_t)kRows * gstride<N3>() * 4 + kRows * 4 * 4 +
-         2 * 4 * 128 * 4 + 64;
-}
+// 72 KiB: three CTAs per SM (3 x 128 TMEM columns)
+constexpr size_t fwd_smem() { return 1024 + 2 * kSlot + 16384 + kRows * 16 + 64; }
 
 template <int N1, int N2, int N3>
 int emb_fwd_launch(const EmbArgs& a, cudaStream_t st) {
   auto kern = k_emb_fwd<N1, N2, N3>;
-  constexpr size_t smem = fwd_smem<N3>();
-  // the largest shared-memory carveout, so that two CTAs fit an SM
+  constexpr size_t smem = fwd_smem();
+  // the largest shared-memory carveout, so that three CTAs fit an SM
   static const cudaError_t attr = [&] {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e == cudaSuccess)
@@ -918,13 +1060,13 @@ int emb_fwd_launch(const EmbArgs& a, cudaStream_t st) {
     return e;
   }();
   if (attr != cudaSuccess) return cuda_status(attr, "embed_fwd_tc attribute");
-  // two CTAs per SM: registers by __launch_bounds__(128, 2), shared memory
-  // below half an SM's
-  static_assert(2 * (smem + 1024) <= 228 * 1024, "two CTAs per SM");
+  // three CTAs per SM: registers by __launch_bounds__(128, 3), shared memory
+  // below a third of an SM's
+  static_assert(3 * (smem + 1024) <= 228 * 1024, "three CTAs per SM");
   int dev = 0, sms = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const int grid = std::max(1, std::min(2 * sms, a.nunits));
+  const int grid = std::max(1, std::min(3 * sms, (a.nunits + 1) / 2));
   kern<<<grid, 128, smem, st>>>(a);
   GBDP_CHECK_LAUNCH("embed_fwd_tc");
   return GBDP_OK;

@@ -119,3 +119,41 @@ def test_plain_tc_step_vs_fp64(setup, mdl_idx):
     print(f"plain-tc vs FP64: |dF| {ef:.3e} eV/A (max |F| {np.abs(Fr).max():.3f}), "
           f"|dE|/N {ee:.3e} eV, |dV| {ev:.3e} eV")
     assert ef <= 2e-2 and ee <= 1e-3
+
+
+@pytest.mark.parametrize("one_side,mols", [(True, 1), (True, 5), (False, 5), (False, 12)])
+def test_equal_rows_and_slabs(setup, one_side, mols):
+    """Sections whose equal rows at the end start at every edge of the 32-row
+    slabs (none, all, one row off either side), odd numbers of atoms of a
+    type (units without a second atom), nets per type and per type pair:
+    X and dE/d(env matrix) against the FP32 torch embedding, with the
+    tolerances stated above (BF16 operands)."""
+    se_a, water, cfg0, m64, _, _ = setup
+    import dataclasses
+
+    cfg = dataclasses.replace(cfg0, type_one_side=one_side)
+    mdl = importlib.import_module("dpmd_public_gb300.model")
+    m = se_a.SeAModel(cfg, mdl.init_params(cfg, 3), m64.davg.cpu().numpy(),
+                      m64.dstd.cpu().numpy(), DEV, torch.float32)
+    atype = np.tile(np.array([0, 1, 1], np.int32), mols)
+    b = m.batch([atype], np.diag([30.0] * 3).reshape(1, 9))
+    b.ensure_plain_tc(m)
+    g = torch.Generator(device=DEV).manual_seed(mols)
+    em = torch.randn(b.nloc, cfg.nnei, 4, generator=g, device=DEV)
+    edges = {46: [1, 2, 31, 32, 33, 34, 45, 46], 92: [1, 32, 33, 64, 65, 66, 91, 92]}
+    for i in range(b.nloc):
+        for t in range(2):
+            k = edges[cfg.sel[t]][(i + 3 * t) % 8]  # rows k - 1 .. are equal
+            em[i, cfg.sec[t] + k:cfg.sec[t + 1]] = torch.tensor([-0.4, 0.0, 0.0, 0.0], device=DEV)
+            em[i, cfg.sec[t] + k - 1] = em[i, cfg.sec[t + 1] - 1] if k < cfg.sel[t] else em[i, 0]
+    b.dD.copy_(torch.randn(b.dD.shape, generator=g, device=DEV) * 0.05)
+    m.embed_tc_forward(b, em)
+    net = m.embed_tc_backward(b, em)
+    torch.cuda.synchronize()
+    assert int(b.emb_status.item()) == 0
+    x = em.clone().requires_grad_(True)
+    Xr = _ref_x(m, x, b.atype)
+    assert float((b.X - Xr).abs().max()) <= 1e-2 * float(Xr.abs().max())
+    Dr = torch.einsum("ncm,nca->nma", Xr, Xr[:, :, :cfg.axis_neuron]).reshape(b.nloc, -1)
+    ref = torch.autograd.grad(Dr, x, b.dD[b.drow.long()])[0]
+    assert float((net - ref).abs().max()) <= 2e-2 * float(ref.abs().max())
