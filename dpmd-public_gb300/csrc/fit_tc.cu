@@ -123,10 +123,11 @@ constexpr int EPI_IN_BYTES = 2 * 2 * EPI_CHUNK * 4;  // 8 KiB
 constexpr int EPI_OUT_BUF = EPI_CHUNK * 4 + 2 * EPI_CHUNK * 2;  // o0 + hi + lo: 4 KiB
 constexpr int EPI_WARP_BYTES = EPI_IN_BYTES + 2 * EPI_OUT_BUF;  // 16 KiB
 
-enum { EPI_F1 = 0, EPI_F2, EPI_F3, EPI_B3, EPI_B2, EPI_B1 };
+enum { EPI_F1 = 0, EPI_F2, EPI_F3, EPI_B3, EPI_B2, EPI_B1, EPI_F1P };
 
 // Per-row inputs and outputs of each epilogue kind (maps.in / maps.out):
 //   F1  out T1, H1 hi/lo        F2  in T1; out T2, H2 hi/lo
+//   F1P out T1 as pieces (t1p), for k_fit_mid
 //   F3  in T1, T2; out GZ3 hi/lo (+ energy partials)
 //   B3  in T2; out G2, GZ2 hi/lo      B2  in T1, G2; out GZ1 hi/lo
 //   B1  out dE/dD
@@ -145,6 +146,7 @@ struct TcEpi {
   const float* rscale;    // F1: [rows] inverse scale of each D row
   float oscale[2];        // 2^s of the split output (hi / lo)
   float* epart;           // [rows, ntile_n] partial energies (F3)
+  float4* t1p;            // F1P: T1 as [row block][4-column piece][128 rows]
   int ncols;              // the layer's output columns (N): a tile's columns past it are skipped
   int* status;
 };
@@ -358,7 +360,8 @@ __device__ __forceinline__ bool epi_tile(const TcMaps& maps, const TcEpi& ep, in
   // barrier phases stay in step across the tiles of a persistent CTA
   const int nch = min(NCH, (ep.ncols - n0 + 15) / 16);
   // F1: the inverse scale of this thread's D row; the split output's scale
-  const float rsc = ep.kind == EPI_F1 ? __ldg(ep.rscale + yrow + lane) : 1.f;
+  const bool f1 = ep.kind == EPI_F1 || ep.kind == EPI_F1P;
+  const float rsc = f1 ? __ldg(ep.rscale + yrow + lane) : 1.f;
   const float osc = ep.oscale[t];
   if (nin > 0) {
     // the first chunk's inputs; their buffer was last read two chunks ago
@@ -419,10 +422,10 @@ __device__ __forceinline__ bool epi_tile(const TcMaps& maps, const TcEpi& ep, in
     if (ep.kind == EPI_B1) {
 #pragma unroll
       for (int k = 0; k < 16; ++k) o0[k] = v[k];
-    } else if (ep.kind == EPI_F1 || ep.kind == EPI_F2 || ep.kind == EPI_F3) {
+    } else if (f1 || ep.kind == EPI_F2 || ep.kind == EPI_F3) {
       float bb[16], id[16], wo[16], i2[16];
       colp_ld16(cp.bias + c0, bb);
-      if (ep.kind != EPI_F1) colp_ld16(cp.idt + c0, id);
+      if (!f1) colp_ld16(cp.idt + c0, id);
       if (ep.kind == EPI_F3) {
         colp_ld16(cp.wout + c0, wo);
         colp_ld16(cp.idt2 + c0, i2);
@@ -454,6 +457,14 @@ __device__ __forceinline__ bool epi_tile(const TcMaps& maps, const TcEpi& ep, in
         const float tt = x0[k];
         sv[k] = (ep.kind == EPI_B3 ? g * id[k] : g) * (1.f - tt * tt) * osc;
       }
+    }
+    if (ep.kind == EPI_F1P) {
+      // coalesced 16-byte stores: the warp's 32 rows of a piece are adjacent
+      float4* t1 = ep.t1p + ((size_t)(yrow >> 7) * (FIT_W / 4) + (c >> 2)) * TBM + (yrow & 127) + lane;
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        t1[q * TBM] = make_float4(o0[4 * q], o0[4 * q + 1], o0[4 * q + 2], o0[4 * q + 3]);
+      continue;
     }
     uint32_t hw[8], lw[8];
     if (ep.out_mask & 6) pack_split16(sv, hw, lw);
@@ -847,6 +858,508 @@ __global__ void __launch_bounds__(192, 1)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem) : "memory");
 }
 
+// B1 (dE/dD = GZ1 W1^T, K 240, N 1600): the persistent loop of k_fit_pers with
+// an epilogue of its own.  That layer only scales its columns and stores, and
+// with 16-column chunks on four warps the chain of TMEM load, staging, proxy
+// fence and bulk store per chunk bounded it (0.57 us a chunk and row block);
+// the whole fitting 164 -> 150 us at 12,288 atoms, 1,076 -> 1,030 us at 126,000.
+// Eight epilogue warps (two per TMEM lane quarter, 64 columns each) take 32
+// columns a chunk: rows of 128 bytes in shared memory (128-byte swizzle), one
+// bulk store of 32 x 32 floats.
+constexpr int B1_EPI_WARPS = 8;
+constexpr int B1_CHUNK = 32 * 32 * 4;  // 4 KiB
+constexpr int B1_SMEM =
+    PERS_STAGES * PERS_STAGE + B1_EPI_WARPS * 2 * B1_CHUNK + 1024 + 256;
+static_assert(B1_SMEM <= 227 * 1024, "B1 shared memory");
+
+__global__ void __launch_bounds__(64 + B1_EPI_WARPS * 32, 1)
+    k_fit_b1(const __grid_constant__ TcMaps maps, const __grid_constant__ TcEpi ep, int K,
+             int ntn, int ntiles) {
+  constexpr int S = PERS_STAGES, STAGE = PERS_STAGE, B_TILE = PERS_TBN * TBK * 2;
+  extern __shared__ unsigned char smem_raw[];
+  unsigned char* smem =
+      reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  unsigned char* epi = smem + S * STAGE;  // [8 warps][2][B1_CHUNK]
+  uint64_t* full = reinterpret_cast<uint64_t*>(epi + B1_EPI_WARPS * 2 * B1_CHUNK);
+  uint64_t* empty = full + S;
+  uint64_t* tfull = empty + S;   // [2] accumulator buffer ready
+  uint64_t* tempty = tfull + 2;  // [2] accumulator buffer read (8 epilogue warps)
+  uint64_t* mdone = tempty + 2;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(mdone + 1);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int nkb = (K + TBK - 1) / TBK;
+  auto tile_at = [&](int tile, int& row0, int& n0, int& t) {
+    const int rb = tile / ntn;
+    row0 = rb * TBM;
+    n0 = (tile - rb * ntn) * PERS_TBN;
+    t = 0;
+    while (t + 1 < ep.ntypes && row0 >= ep.row_off[t + 1]) ++t;
+  };
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < S; ++i) {
+      mbar_init(&full[i], 1);
+      mbar_init(&empty[i], 1);
+    }
+    for (int j = 0; j < 2; ++j) {
+      mbar_init(&tfull[j], 1);
+      mbar_init(&tempty[j], B1_EPI_WARPS);
+    }
+    mbar_init(mdone, 1);
+    fence_mbar_init();
+  }
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(
+                     smem_addr(tmem_slot))
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = *tmem_slot;
+
+  if (warp == 0) {
+    if (lane == 0) {
+      // ---- TMA producer; the first stages' B tiles (weights) are requested
+      //      before waiting for the previous layer
+      int issued = 0;
+      bool ok = true, first = true;
+      for (int tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x) {
+        int row0, n0, t;
+        tile_at(tile, row0, n0, t);
+        for (int kb = 0; kb < nkb; ++kb) {
+          const int st_i = issued % S;
+          if (issued >= S &&
+              !mbar_wait_bounded(&empty[st_i], ((issued / S) & 1u) ^ 1u, ep.status)) {
+            ok = false;
+            break;
+          }
+          unsigned char* st = smem + st_i * STAGE;
+          mbar_expect_tx(&full[st_i], STAGE);
+          tma_2d(st + 2 * A_TILE, &maps.b_hi[t], kb * TBK, n0, &full[st_i]);
+          tma_2d(st + 2 * A_TILE + B_TILE, &maps.b_lo[t], kb * TBK, n0, &full[st_i]);
+          ++issued;
+          if (first) {  // the A tiles of the first stages follow the wait
+            if (issued < S && kb + 1 < nkb) continue;
+            griddep_wait();
+            first = false;
+            for (int k = 0; k < issued; ++k) {
+              unsigned char* a = smem + k * STAGE;
+              tma_2d(a, &maps.a_hi, k * TBK, row0, &full[k]);
+              tma_2d(a + A_TILE, &maps.a_lo, k * TBK, row0, &full[k]);
+            }
+          } else {
+            tma_2d(st, &maps.a_hi, kb * TBK, row0, &full[st_i]);
+            tma_2d(st + A_TILE, &maps.a_lo, kb * TBK, row0, &full[st_i]);
+          }
+        }
+      }
+      // no bulk copy of this CTA may land after it exits
+      for (int k = (issued > S ? issued - S : 0); k < issued; ++k)
+        mbar_wait_bounded(&full[k % S], (k / S) & 1u, ep.status);
+    }
+  } else if (warp == 1) {
+    if (lane == 0) {
+      // ---- MMA issuer: D(f32) += A(f16, K-major) B(f16, K-major), M 128, N 128
+      const uint32_t idesc =
+          (1u << 4) | ((uint32_t)(PERS_TBN >> 3) << 17) | ((uint32_t)(TBM >> 4) << 24);
+      int cons = 0;
+      bool ok = true;
+      int it = 0;
+      for (int tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x, ++it) {
+        const int j = it & 1, use = it >> 1;  // this buffer's earlier uses
+        if (use > 0 && !mbar_wait_bounded(&tempty[j], (unsigned)(use - 1) & 1u, ep.status)) break;
+        tc_fence_after();
+        const uint32_t dm = tmem + (uint32_t)(j * 256), dc = dm + 128u;
+        for (int kb = 0; kb < nkb; ++kb) {
+          const int st_i = cons % S;
+          if (!mbar_wait_bounded(&full[st_i], (cons / S) & 1u, ep.status)) {
+            ok = false;
+            break;
+          }
+          tc_fence_after();
+          const uint32_t ah = smem_addr(smem + st_i * STAGE), al = ah + A_TILE,
+                         bh = ah + 2 * A_TILE, bl = bh + B_TILE;
+#pragma unroll
+          for (int kk = 0; kk < TBK / 16; ++kk) {
+            const uint32_t off = kk * 32;
+            const uint64_t dah = sdesc_sw128(ah + off), dal = sdesc_sw128(al + off),
+                           dbh = sdesc_sw128(bh + off), dbl = sdesc_sw128(bl + off);
+            const uint32_t acc = (kb > 0 || kk > 0) ? 1u : 0u;
+            umma_f16(dm, dah, dbh, idesc, acc);
+            umma_f16(dc, dal, dbh, idesc, acc);
+            umma_f16(dc, dah, dbl, idesc, 1u);
+          }
+          umma_commit(&empty[st_i]);
+          ++cons;
+        }
+        if (ok) umma_commit(&tfull[j]);
+      }
+      // every MMA issued complete before TMEM is released
+      umma_commit(mdone);
+      mbar_wait_bounded(mdone, 0, ep.status);
+    }
+  } else {
+    // ---- epilogue warps (B1 reads nothing of the previous layers, but its
+    //      output rows may still be read by launches before this one)
+    griddep_wait();
+    const int ew = warp - 2, q = warp & 3, half = ew >> 2;
+    unsigned char* wsm = epi + ew * 2 * B1_CHUNK;
+    int it = 0, nst = 0;
+    for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x, ++it) {
+      const int j = it & 1;
+      if (!__all_sync(kFull, mbar_wait_bounded(&tfull[j], (unsigned)(it >> 1) & 1u, ep.status)))
+        break;
+      tc_fence_after();
+      // the next launch may start filling SMs once this CTA's last tile drains
+      if (tile + (int)gridDim.x >= ntiles) griddep_launch_dependents();
+      int row0, n0, t;
+      tile_at(tile, row0, n0, t);
+      const uint32_t tacc = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(j * 256 + half * 64);
+      const int c0 = n0 + half * 64;
+#pragma unroll
+      for (int ch = 0; ch < 2; ++ch) {
+        const int c = c0 + 32 * ch;
+        if (c >= ep.ncols) break;  // uniform: past the last, partial tile
+        float v[32], w[32];
+        tmem_ld16x2(tacc + 32u * ch, tacc + 128u + 32u * ch, v, w);
+        tmem_ld16x2(tacc + 32u * ch + 16u, tacc + 128u + 32u * ch + 16u, v + 16, w + 16);
+        const float4* cs = reinterpret_cast<const float4*>(ep.cscale[t] + c);
+        unsigned char* buf = wsm + (nst & 1) * B1_CHUNK;
+        // the buffer was last used by the store before the previous one
+        if (lane == 0 && nst >= 2) bulk_wait_read1();
+        __syncwarp();
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+          const float4 k = __ldg(cs + u);
+          *reinterpret_cast<float4*>(buf + lane * 128 + ((u ^ (lane & 7)) << 4)) =
+              make_float4((v[4 * u] + w[4 * u]) * k.x, (v[4 * u + 1] + w[4 * u + 1]) * k.y,
+                          (v[4 * u + 2] + w[4 * u + 2]) * k.z, (v[4 * u + 3] + w[4 * u + 3]) * k.w);
+        }
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) {
+          tma_store_2d(&maps.out[0], c, row0 + q * 32, buf);
+          bulk_commit();
+        }
+        ++nst;
+      }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&tempty[j]);
+    }
+    if (lane == 0) bulk_wait_all();
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 0)
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem) : "memory");
+}
+
+// ------------------------------------------- the four K-240 layers fused --
+// F2, F3, B3 and B2 of one 128-row block in one CTA (persistent over blocks).
+// The activations never leave the SM as GEMM operands: the epilogue of a
+// layer writes the next one's A (hi / lo, 128-byte swizzle) straight into
+// shared memory, 4 k-blocks of 16 KiB each, and the weights stream through a
+// ring of three 30 KiB pieces (240 rows of one 64-deep k-block, hi or lo).
+//   warp 0      TMA producer of the weight pieces
+//   warp 1      MMA issuer: main accumulator (columns 0 ..), cross terms (256 ..)
+//   warps 2-17  epilogue: warp w takes TMEM lanes 32 (w % 4) .. (its 32 rows)
+//               and the 64 columns of one k-block, so that it alone writes its
+//               rows of that k-block
+// T1 comes from F1 and T2, G2 go to a scratch of the CTA, all as [4-column
+// piece][128 rows] of float4: a warp's loads and stores are 512 contiguous
+// bytes, and the scratch (2 x 120 KiB a CTA) stays in L2.  GZ1 leaves by TMA
+// from the A buffer for B1.
+// Bounded by the serial chain of a block (four times MMAs, then an epilogue
+// over 240 columns), not by the activations' traffic: reading no inputs takes
+// 10 us off the 164 us of 12,288 atoms, no tanh 3 us; eight epilogue warps
+// instead of sixteen cost 6 us.
+constexpr int MID_PIECE = FIT_W * TBK * 2;                      // 30 KiB
+constexpr int MID_RING = 3;
+constexpr int MID_KB = 4;                                      // k-blocks of 64 (the last: 48)
+constexpr int MID_A = MID_KB * A_TILE;                         // one part (hi or lo) of A
+constexpr int MID_SMEM = 2 * MID_A + MID_RING * MID_PIECE + 1024 + 256;
+constexpr int MID_PARTS = 4;              // epilogue warps per TMEM lane quarter
+constexpr int MID_WARPS = 4 * MID_PARTS;
+constexpr int MID_COLS = 256 / MID_PARTS;  // columns a warp takes (the last part fewer)
+static_assert(MID_SMEM <= 227 * 1024 && MID_PIECE % 1024 == 0, "fused fitting layers: shared memory");
+
+struct MidMaps {
+  CUtensorMap w[2][4][2];  // [type][layer][hi, lo]: boxes of 64 columns x 240 rows
+  CUtensorMap gz[2];       // GZ1 hi, lo: boxes of 64 columns x 32 rows
+};
+struct MidArgs {
+  int ntypes, row_off[3], nblk;
+  const float4* t1p;
+  float4 *t2p, *g2p;  // per-CTA scratch
+  float* epart;       // [rows][MID_PARTS]
+  const float *bias2[2], *bias3[2], *idt2[2], *idt3[2], *wout[2];
+  const float* cs[2][4];
+  float osc[2][5];  // scales of H1, H2, GZ3, GZ2, GZ1
+  int* status;
+};
+
+__device__ __forceinline__ void ld_piece16(const float4* p, float* v) {
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const float4 u = p[q * TBM];
+    v[4 * q] = u.x;
+    v[4 * q + 1] = u.y;
+    v[4 * q + 2] = u.z;
+    v[4 * q + 3] = u.w;
+  }
+}
+__device__ __forceinline__ void st_piece16(float4* p, const float* v) {
+#pragma unroll
+  for (int q = 0; q < 4; ++q)
+    p[q * TBM] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+}
+
+// columns c .. c + 15 of row r of A (scaled values), split
+__device__ __forceinline__ void st_a16(unsigned char* a, int r, int c, const float* sv) {
+  uint32_t hw[8], lw[8];
+  pack_split16(sv, hw, lw);
+  unsigned char* row = a + (c >> 6) * A_TILE + r * 128;
+  const int u = (c & 63) >> 3;
+#pragma unroll
+  for (int q = 0; q < 2; ++q) {
+    const int at = ((u + q) ^ (r & 7)) << 4;
+    *reinterpret_cast<uint4*>(row + at) = make_uint4(hw[4 * q], hw[4 * q + 1], hw[4 * q + 2], hw[4 * q + 3]);
+    *reinterpret_cast<uint4*>(row + MID_A + at) =
+        make_uint4(lw[4 * q], lw[4 * q + 1], lw[4 * q + 2], lw[4 * q + 3]);
+  }
+}
+
+__global__ void __launch_bounds__(64 + MID_WARPS * 32, 1)
+    k_fit_mid(const __grid_constant__ MidMaps maps, const __grid_constant__ MidArgs p) {
+  extern __shared__ unsigned char smem_raw[];
+  unsigned char* smem =
+      reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  unsigned char* ring = smem + 2 * MID_A;
+  uint64_t* full = reinterpret_cast<uint64_t*>(ring + MID_RING * MID_PIECE);
+  uint64_t* empty = full + MID_RING;
+  uint64_t* aready = empty + MID_RING;  // A written (8 epilogue warps)
+  uint64_t* accfull = aready + 1;       // a layer's MMAs complete
+  uint64_t* mdone = accfull + 1;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(mdone + 1);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  auto type_of = [&](int rb) {
+    int t = 0;
+    while (t + 1 < p.ntypes && rb * TBM >= p.row_off[t + 1]) ++t;
+    return t;
+  };
+
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < MID_RING; ++i) {
+      mbar_init(&full[i], 1);
+      mbar_init(&empty[i], 1);
+    }
+    mbar_init(aready, MID_WARPS);
+    mbar_init(accfull, 1);
+    mbar_init(mdone, 1);
+    fence_mbar_init();
+  }
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(
+                     smem_addr(tmem_slot))
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = *tmem_slot;
+
+  if (warp == 0) {
+    if (lane == 0) {
+      // ---- TMA producer: hi, lo of each k-block of each layer's weights
+      //      (no dependence on the previous launch)
+      int issued = 0;
+      bool ok = true;
+      for (int rb = blockIdx.x; rb < p.nblk && ok; rb += gridDim.x) {
+        const int t = type_of(rb);
+        for (int i = 0; i < 4 * MID_KB * 2; ++i) {
+          const int st = issued % MID_RING;
+          if (issued >= MID_RING &&
+              !mbar_wait_bounded(&empty[st], ((issued / MID_RING) & 1u) ^ 1u, p.status)) {
+            ok = false;
+            break;
+          }
+          mbar_expect_tx(&full[st], MID_PIECE);
+          tma_2d(ring + st * MID_PIECE, &maps.w[t][i >> 3][i & 1], ((i >> 1) & 3) * TBK, 0, &full[st]);
+          ++issued;
+        }
+      }
+      // no bulk copy of this CTA may land after it exits
+      for (int k = issued > MID_RING ? issued - MID_RING : 0; k < issued; ++k)
+        mbar_wait_bounded(&full[k % MID_RING], (k / MID_RING) & 1u, p.status);
+    }
+  } else if (warp == 1) {
+    if (lane == 0) {
+      // ---- MMA issuer: D(f32) += A(f16, K-major) B(f16, K-major), M 128, N 240
+      const uint32_t idesc =
+          (1u << 4) | ((uint32_t)(FIT_W >> 3) << 17) | ((uint32_t)(TBM >> 4) << 24);
+      const uint32_t dm = tmem, dc = tmem + 256u;
+      int piece = 0;
+      unsigned aph = 0;
+      bool ok = true;
+      for (int rb = blockIdx.x; rb < p.nblk && ok; rb += gridDim.x)
+        for (int l = 0; l < 4 && ok; ++l) {
+          if (!mbar_wait_bounded(aready, aph, p.status)) {
+            ok = false;
+            break;
+          }
+          aph ^= 1u;
+          tc_fence_after();
+          for (int i = 0; i < 2 * MID_KB; ++i, ++piece) {
+            const int st = piece % MID_RING, kb = i >> 1;
+            if (!mbar_wait_bounded(&full[st], (piece / MID_RING) & 1u, p.status)) {
+              ok = false;
+              break;
+            }
+            tc_fence_after();
+            const uint32_t ah = smem_addr(smem + kb * A_TILE), al = ah + MID_A,
+                           b = smem_addr(ring + st * MID_PIECE);
+            const int nkk = kb == MID_KB - 1 ? (FIT_W - 3 * TBK) / 16 : TBK / 16;
+            for (int kk = 0; kk < nkk; ++kk) {
+              const uint32_t off = kk * 32, acc = (kb > 0 || kk > 0) ? 1u : 0u;
+              if (i & 1) {
+                umma_f16(dc, sdesc_sw128(ah + off), sdesc_sw128(b + off), idesc, 1u);
+              } else {
+                umma_f16(dm, sdesc_sw128(ah + off), sdesc_sw128(b + off), idesc, acc);
+                umma_f16(dc, sdesc_sw128(al + off), sdesc_sw128(b + off), idesc, acc);
+              }
+            }
+            umma_commit(&empty[st]);
+          }
+          if (ok) umma_commit(accfull);
+        }
+      // every MMA issued complete before TMEM is released
+      umma_commit(mdone);
+      mbar_wait_bounded(mdone, 0, p.status);
+    }
+  } else {
+    // ---- epilogue warps
+    const int ew = warp - 2, q = warp & 3, part = ew >> 2;
+    const int r = q * 32 + lane;  // row in the block = TMEM lane
+    const int c0 = part * MID_COLS, nch = min(MID_COLS, FIT_W - c0) / 16;
+    const uint32_t tacc = tmem + ((uint32_t)(q * 32) << 16);
+    float4* t2 = p.t2p + (size_t)blockIdx.x * (FIT_W / 4) * TBM + r;
+    float4* g2 = p.g2p + (size_t)blockIdx.x * (FIT_W / 4) * TBM + r;
+    unsigned accph = 0;
+    bool ok = true;
+    griddep_wait();  // F1's T1 visible to this thread
+    for (int rb = blockIdx.x; rb < p.nblk && ok; rb += gridDim.x) {
+      const int t = type_of(rb);
+      const float4* t1 = p.t1p + (size_t)rb * (FIT_W / 4) * TBM + r;
+      // A of F2: H1 = T1
+      for (int ch = 0; ch < nch; ++ch) {
+        const int c = c0 + ch * 16;
+        float v[16];
+        ld_piece16(t1 + (c >> 2) * TBM, v);
+        const float osc = p.osc[t][0];
+#pragma unroll
+        for (int k = 0; k < 16; ++k) v[k] *= osc;
+        st_a16(smem, r, c, v);
+      }
+      float esum = 0.f;
+#pragma unroll 1
+      for (int l = 0; l < 4; ++l) {
+        // A of layer l is written, and the accumulators' last values read
+        fence_proxy_async_smem();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(aready);
+        if (!__all_sync(kFull, mbar_wait_bounded(accfull, accph, p.status))) {
+          ok = false;
+          break;
+        }
+        accph ^= 1u;
+        tc_fence_after();
+        if (l == 3 && rb + (int)gridDim.x >= p.nblk) griddep_launch_dependents();
+        const float* cs = p.cs[t][l];
+        const float osc = p.osc[t][l + 1];
+#pragma unroll 1
+        for (int ch = 0; ch < nch; ++ch) {
+          const int c = c0 + ch * 16, at = (c >> 2) * TBM;
+          float v[16], w[16], x0[16], x1[16], sv[16];
+          // this chunk's inputs (F2: T1; F3: T1, T2; B3: T2; B2: T1, G2)
+          if (l != 2) ld_piece16(t1 + at, x0);
+          if (l == 1 || l == 2) ld_piece16(t2 + at, x1);
+          if (l == 3) ld_piece16(g2 + at, x1);
+          tmem_ld16x2(tacc + (uint32_t)c, tacc + 256u + (uint32_t)c, v, w);
+#pragma unroll
+          for (int k = 0; k < 16; ++k) v[k] += w[k];
+          // undo the operand scales (powers of two: exact)
+          colp_ld16(cs + c, w);
+#pragma unroll
+          for (int k = 0; k < 16; ++k) v[k] *= w[k];
+          if (l <= 1) {
+            float bb[16], id[16];
+            colp_ld16((l ? p.bias3[t] : p.bias2[t]) + c, bb);
+            colp_ld16(p.idt2[t] + c, id);
+#pragma unroll
+            for (int k = 0; k < 16; ++k) v[k] = tanhf(v[k] + bb[k]);
+            if (l == 0) {  // T2, H2 = T2 idt2 + T1
+              st_piece16(t2 + at, v);
+#pragma unroll
+              for (int k = 0; k < 16; ++k) sv[k] = (v[k] * id[k] + x0[k]) * osc;
+            } else {  // H3 = T3 idt3 + H2, e += H3 w_out, GZ3
+              float i3[16];
+              colp_ld16(p.wout[t] + c, w);
+              colp_ld16(p.idt3[t] + c, i3);
+#pragma unroll
+              for (int k = 0; k < 16; ++k) {
+                const float h = v[k] * i3[k] + (x1[k] * id[k] + x0[k]);
+                esum += h * w[k];
+                sv[k] = w[k] * i3[k] * (1.f - v[k] * v[k]) * osc;
+              }
+            }
+          } else if (l == 2) {  // G2 = . + w_out, GZ2 = G2 idt2 (1 - T2^2)
+            float id[16];
+            colp_ld16(p.wout[t] + c, w);
+            colp_ld16(p.idt2[t] + c, id);
+#pragma unroll
+            for (int k = 0; k < 16; ++k) {
+              v[k] += w[k];
+              sv[k] = v[k] * id[k] * (1.f - x1[k] * x1[k]) * osc;
+            }
+            st_piece16(g2 + at, v);
+          } else {  // G1 = . + G2, GZ1 = G1 (1 - T1^2)
+#pragma unroll
+            for (int k = 0; k < 16; ++k)
+              sv[k] = (v[k] + x1[k]) * (1.f - x0[k] * x0[k]) * osc;
+          }
+          st_a16(smem, r, c, sv);
+        }
+      }
+      if (!ok) break;
+      p.epart[(size_t)(rb * TBM + r) * MID_PARTS + part] = esum;
+      // GZ1: this warp's rows of its two k-blocks, from the A buffer
+      fence_proxy_async_smem();
+      __syncwarp();
+      if (lane == 0) {
+#pragma unroll
+        for (int k = 0; k < MID_KB / MID_PARTS; ++k) {
+          const int kb = MID_KB / MID_PARTS * part + k;
+          const unsigned char* src = smem + kb * A_TILE + q * 32 * 128;
+          tma_store_2d(&maps.gz[0], kb * TBK, rb * TBM + q * 32, src);
+          tma_store_2d(&maps.gz[1], kb * TBK, rb * TBM + q * 32, src + MID_A);
+        }
+        bulk_commit();
+        bulk_wait_all();  // A is rewritten next (and nothing is in flight at exit)
+      }
+      tc_fence_before();
+      __syncwarp();
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 0)
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem) : "memory");
+}
+
 // per-row energy: e = sum of the F3 partials + b_out; padding rows get 0
 struct TcRows {
   int row_off[3];
@@ -955,7 +1468,7 @@ TcWs carve_tc(void* base, long rows) {
   w.gz1h = f16();
   w.gz1l = f16();
   w.epart = static_cast<float*>(
-      take(sizeof(float) * (size_t)rows * (FIT_W / (rows <= kMaxNarrowRows ? 16 : 80))));
+      take(sizeof(float) * (size_t)rows * (rows <= kMaxNarrowRows ? FIT_W / 16 : MID_PARTS)));
   w.bytes = off;
   return w;
 }
@@ -967,17 +1480,73 @@ cudaError_t launch_tile(cudaLaunchConfig_t& lc, const TcMaps& maps, const TcEpi&
   return cudaLaunchKernelEx(&lc, k_fit_tc<C>, maps, ep, K);
 }
 
+// Above this many row blocks the four K-240 layers run fused: one launch and
+// 16 MB of T1 in and GZ1 out (12,288 rows) instead of four launches that move
+// 230 MB.  The whole fitting, per layer / fused, us: 4,500 rows 111 / 107,
+// 9,000: 139 / 130, 12,288: 180 / 164, 126,000: 1,372 / 1,066; below, the narrow
+// tiles are ahead (3,750 rows: 91 / 99).
+constexpr int kMidMinBlocks = 30;
+
+int launch_mid(const TcWs& ws, int ntypes, const int* row_off, const gbdp_fit_tc_net* nets,
+               long rows, int nsm, int* status, cudaStream_t st) {
+  MidMaps maps;
+  MidArgs a;
+  memset(&maps, 0, sizeof(maps));
+  memset(&a, 0, sizeof(a));
+  int rc = make_map(&maps.gz[0], ws.gz1h, rows, FIT_W, 32);
+  if (!rc) rc = make_map(&maps.gz[1], ws.gz1l, rows, FIT_W, 32);
+  a.ntypes = ntypes;
+  for (int t = 0; t <= ntypes; ++t) a.row_off[t] = row_off[t];
+  a.nblk = (int)(rows / TBM);
+  a.t1p = reinterpret_cast<const float4*>(ws.t1);
+  a.t2p = reinterpret_cast<float4*>(ws.t2);
+  a.g2p = reinterpret_cast<float4*>(ws.g2);
+  a.epart = ws.epart;
+  a.status = status;
+  for (int t = 0; t < 2 && !rc; ++t) {
+    const gbdp_fit_tc_net& n = nets[t < ntypes ? t : 0];
+    // F2, F3: W^T [out, in]; B3, B2: W [in, out]
+    const void* w[4][2] = {{n.wt_hi[1], n.wt_lo[1]}, {n.wt_hi[2], n.wt_lo[2]},
+                           {n.w_hi[2], n.w_lo[2]}, {n.w_hi[1], n.w_lo[1]}};
+    const float* cs[4] = {n.cs_fwd[1], n.cs_fwd[2], n.cs_bwd[2], n.cs_bwd[1]};
+    for (int l = 0; l < 4 && !rc; ++l) {
+      for (int h = 0; h < 2 && !rc; ++h) rc = make_map(&maps.w[t][l][h], w[l][h], FIT_W, FIT_W, FIT_W);
+      a.cs[t][l] = cs[l];
+    }
+    a.bias2[t] = n.b[1];
+    a.bias3[t] = n.b[2];
+    a.idt2[t] = n.idt[1];
+    a.idt3[t] = n.idt[2];
+    a.wout[t] = n.w_out;
+    for (int k = 0; k < 5; ++k) a.osc[t][k] = n.act_scale[k];
+  }
+  if (rc) return rc;
+  cudaFuncSetAttribute(k_fit_mid, cudaFuncAttributeMaxDynamicSharedMemorySize, MID_SMEM);
+  cudaLaunchConfig_t lc = {};
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  lc.attrs = attr;
+  lc.numAttrs = 1;
+  lc.gridDim = dim3((unsigned)(a.nblk < nsm ? a.nblk : nsm));
+  lc.blockDim = dim3(64 + MID_WARPS * 32);
+  lc.dynamicSmemBytes = MID_SMEM;
+  lc.stream = st;
+  const cudaError_t e = cudaLaunchKernelEx(&lc, k_fit_mid, maps, a);
+  if (e != cudaSuccess) return cuda_status(e, "fit_tc mid launch");
+  return GBDP_OK;
+}
+
 }  // namespace
 }  // namespace gbdp
 
 using namespace gbdp;
 
 namespace {
-// tiles per SM from which the K-240 layers run on the persistent kernel
-// (measured on the ragged water batches: per-tile and persistent within 1 %
-// from 4 to 60 tiles per SM; the layers are bound by their activation
-// traffic, not by launches)
-std::atomic<int> g_short_pers_min_tiles{32};
+// tiles per SM from which the K-240 layers run on the persistent kernel; at
+// the default the library chooses (k_fit_mid or narrow tiles)
+constexpr int kDefaultTilesPerSm = 32;
+std::atomic<int> g_short_pers_min_tiles{kDefaultTilesPerSm};
 }  // namespace
 
 extern "C" void gbdp_fitting_tc_set_persistent_min_tiles(int tiles_per_sm) {
@@ -1024,6 +1593,7 @@ extern "C" int gbdp_fitting_tc_f32(float* e, float* dE_dD, const void* D_hi, con
   cudaStream_t st = (cudaStream_t)stream;
   cudaMemsetAsync(status, 0, sizeof(int) * 4, st);
   cudaFuncSetAttribute(k_fit_pers, cudaFuncAttributeMaxDynamicSharedMemorySize, PERS_SMEM);
+  cudaFuncSetAttribute(k_fit_b1, cudaFuncAttributeMaxDynamicSharedMemorySize, B1_SMEM);
   // SM count of the device (initialised once, thread-safe)
   static const int nsm = [] {
     int dev = 0, n = 0;
@@ -1046,28 +1616,30 @@ extern "C" int gbdp_fitting_tc_f32(float* e, float* dE_dD, const void* D_hi, con
     GBDP_REQUIRE(((uintptr_t)nets[t].idt[1] & 15) == 0 && ((uintptr_t)nets[t].idt[2] & 15) == 0,
                  "fit_tc: idt not 16-byte aligned");
   }
-  enum { LONGK = 0, SHORTK, PERSIST, LONG16, SHORT16, LONG48, SHORT48 };
+  enum { LONGK = 0, SHORTK, PERSIST, LONG16, SHORT16, LONG48, SHORT48, B1PERS };
   // the K-240 layers go to the persistent kernel from this many tiles per SM
   const long short_tiles = (rows / TBM) * (FIT_W / CfgShortK::TBN);
   const long nblk = rows / TBM;
   const bool narrow16 = nblk <= kMaxNarrowRows / TBM && nblk * (FIT_W / 16) <= nsm,
              narrow48 = nblk <= kMaxNarrowRows / TBM && nblk * (FIT_W / 48) <= nsm;
   const int long_cfg = narrow16 ? LONG16 : narrow48 ? LONG48 : LONGK;
-  const int short_cfg = short_tiles >= (long)g_short_pers_min_tiles.load() * nsm ? PERSIST
-                        : narrow16                                                ? SHORT16
-                        : narrow48                                                ? SHORT48
-                                                                                  : SHORTK;
+  const int tiles_per_sm = g_short_pers_min_tiles.load();
+  const bool fused = tiles_per_sm == kDefaultTilesPerSm && nblk > kMidMinBlocks;
+  const int short_cfg = short_tiles >= (long)tiles_per_sm * nsm ? PERSIST
+                        : narrow16                              ? SHORT16
+                        : narrow48                              ? SHORT48
+                                                                : SHORTK;
   // B1 in 48-column tiles while they fit one wave
-  const int b1_cfg = nblk * ((FIT_D + 47) / 48) <= nsm ? SHORT48 : PERSIST;
+  const int b1_cfg = nblk * ((FIT_D + 47) / 48) <= nsm ? SHORT48 : B1PERS;
   auto width_of = [](int cfg) {
     return cfg == LONGK                        ? CfgLongK::TBN
            : cfg == SHORTK                     ? CfgShortK::TBN
-           : cfg == PERSIST                    ? PERS_TBN
+           : cfg == PERSIST || cfg == B1PERS  ? PERS_TBN
            : cfg == LONG16 || cfg == SHORT16 ? 16
                                                : 48;
   };
   // F3's partial energies: one per N tile of the kernel that runs it
-  base.ntile_n = (FIT_W + width_of(short_cfg) - 1) / width_of(short_cfg);
+  base.ntile_n = fused ? MID_PARTS : (FIT_W + width_of(short_cfg) - 1) / width_of(short_cfg);
   // act: index into act_scale of the split output (-1: none)
   struct Step {
     int kind;
@@ -1096,6 +1668,13 @@ extern "C" int gbdp_fitting_tc_f32(float* e, float* dE_dD, const void* D_hi, con
       {EPI_B1, ws.gz1h, ws.gz1l, FIT_W, FIT_D, 0, false, {nullptr, nullptr},
        {dE_dD, nullptr, nullptr}, -1, b1_cfg}};
   for (const Step& sp : steps) {
+    if (fused && sp.kind != EPI_F1 && sp.kind != EPI_B1) {
+      if (sp.kind != EPI_F2) continue;
+      rc = launch_mid(ws, ntypes, row_off, nets, rows, nsm, status, st);
+      if (rc) return rc;
+      continue;
+    }
+    const bool f1p = fused && sp.kind == EPI_F1;
     TcMaps maps;
     memset(&maps, 0, sizeof(maps));
     rc = make_map(&maps.a_hi, sp.a_hi, rows, sp.K, TBM);
@@ -1110,7 +1689,8 @@ extern "C" int gbdp_fitting_tc_f32(float* e, float* dE_dD, const void* D_hi, con
       if (!rc) rc = make_map(&maps.b_lo[t], bl, sp.N, sp.K, tbn);
     }
     TcEpi ep = base;
-    ep.kind = sp.kind;
+    ep.kind = f1p ? EPI_F1P : sp.kind;
+    ep.t1p = reinterpret_cast<float4*>(ws.t1);
     ep.ncols = sp.N;
     ep.nin = 0;
     ep.out_mask = 0;
@@ -1120,9 +1700,11 @@ extern "C" int gbdp_fitting_tc_f32(float* e, float* dE_dD, const void* D_hi, con
         rc = make_epi_map(&maps.in[a], sp.in[a], 4, rows, sp.N);
         ep.nin = a + 1;
       }
-    for (int a = 0; a < 3 && !rc; ++a)
+    for (int a = 0; a < 3 && !rc && !f1p; ++a)
       if (sp.out[a]) {
-        rc = make_epi_map(&maps.out[a], sp.out[a], a == 0 ? 4 : 2, rows, sp.N);
+        rc = sp.cfg == B1PERS ? make_map_box(&maps.out[a], sp.out[a], 4, rows, sp.N, 32, 32,
+                                             CU_TENSOR_MAP_SWIZZLE_128B)
+                              : make_epi_map(&maps.out[a], sp.out[a], a == 0 ? 4 : 2, rows, sp.N);
         ep.out_mask |= 1 << a;
       }
     if (rc) return rc;
@@ -1147,7 +1729,7 @@ extern "C" int gbdp_fitting_tc_f32(float* e, float* dE_dD, const void* D_hi, con
     lc.blockDim = dim3(128);
     lc.stream = st;
     cudaError_t le;
-    if (sp.cfg != PERSIST) {
+    if (sp.cfg != PERSIST && sp.cfg != B1PERS) {
       lc.gridDim = dim3((sp.N + width_of(sp.cfg) - 1) / width_of(sp.cfg), (unsigned)nblk);
       switch (sp.cfg) {
         case LONGK: le = launch_tile<CfgLongK>(lc, maps, ep, sp.K); break;
@@ -1161,9 +1743,11 @@ extern "C" int gbdp_fitting_tc_f32(float* e, float* dE_dD, const void* D_hi, con
       // one CTA per SM walking the layer's tiles
       const int ntn = (sp.N + PERS_TBN - 1) / PERS_TBN, ntiles = ntn * (int)(rows / TBM);
       lc.gridDim = dim3((unsigned)(ntiles < nsm ? ntiles : nsm));
-      lc.blockDim = dim3(192);
-      lc.dynamicSmemBytes = PERS_SMEM;
-      le = cudaLaunchKernelEx(&lc, k_fit_pers, maps, ep, sp.K, ntn, ntiles);
+      const bool b1 = sp.cfg == B1PERS;
+      lc.blockDim = dim3(b1 ? 64 + B1_EPI_WARPS * 32 : 192);
+      lc.dynamicSmemBytes = b1 ? B1_SMEM : PERS_SMEM;
+      le = b1 ? cudaLaunchKernelEx(&lc, k_fit_b1, maps, ep, sp.K, ntn, ntiles)
+              : cudaLaunchKernelEx(&lc, k_fit_pers, maps, ep, sp.K, ntn, ntiles);
     }
     if (le != cudaSuccess) return cuda_status(le, "fit_tc gemm launch");
     GBDP_CHECK_LAUNCH("fit_tc gemm");

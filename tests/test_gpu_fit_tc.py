@@ -101,11 +101,13 @@ def test_persistent_short_k_layers_equal_per_tile(setup):
         assert torch.equal(x, y)
 
 
-@pytest.mark.parametrize("mols", [1, 40, 43, 190, 256, 416, 427, 1193, 1280])
+@pytest.mark.parametrize("mols", [1, 40, 43, 190, 256, 416, 427, 1193, 1280, 1281, 3000,
+                                  6470, 13000])
 def test_tile_widths_by_rows_vs_fp64(setup, mols):
     """Per-row energy and dE/dD of random descriptor rows against FP64, at row
-    counts on both sides of the lines between the 16-, 48- and 80 / 128-wide
-    tiles (10 and 30 row blocks of 128; B1: 4 row blocks).  Operands are split
+    counts on both sides of the lines between the 16-wide tiles, the 48-wide
+    ones and the fused K-240 layers (10 and 30 row blocks of 128; B1: 4 row
+    blocks), and with one, a few more and twice as many row blocks as SMs.  Operands are split
     to 2^-22, sums of 1,600 terms in FP32: 1e-5 of the largest magnitude."""
     m = setup[3]("tc-f16x3")
     n = 3 * mols
