@@ -123,11 +123,10 @@ constexpr int EPI_IN_BYTES = 2 * 2 * EPI_CHUNK * 4;  // 8 KiB
 constexpr int EPI_OUT_BUF = EPI_CHUNK * 4 + 2 * EPI_CHUNK * 2;  // o0 + hi + lo: 4 KiB
 constexpr int EPI_WARP_BYTES = EPI_IN_BYTES + 2 * EPI_OUT_BUF;  // 16 KiB
 
-enum { EPI_F1 = 0, EPI_F2, EPI_F3, EPI_B3, EPI_B2, EPI_B1, EPI_F1P };
+enum { EPI_F1 = 0, EPI_F2, EPI_F3, EPI_B3, EPI_B2, EPI_B1 };
 
 // Per-row inputs and outputs of each epilogue kind (maps.in / maps.out):
 //   F1  out T1, H1 hi/lo        F2  in T1; out T2, H2 hi/lo
-//   F1P out T1 as pieces (t1p), for k_fit_mid
 //   F3  in T1, T2; out GZ3 hi/lo (+ energy partials)
 //   B3  in T2; out G2, GZ2 hi/lo      B2  in T1, G2; out GZ1 hi/lo
 //   B1  out dE/dD
@@ -146,7 +145,7 @@ struct TcEpi {
   const float* rscale;    // F1: [rows] inverse scale of each D row
   float oscale[2];        // 2^s of the split output (hi / lo)
   float* epart;           // [rows, ntile_n] partial energies (F3)
-  float4* t1p;            // F1P: T1 as [row block][4-column piece][128 rows]
+  float4* t1p;            // k_fit_f1: T1 as [row block][4-column piece][128 rows]
   int ncols;              // the layer's output columns (N): a tile's columns past it are skipped
   int* status;
 };
@@ -360,8 +359,7 @@ __device__ __forceinline__ bool epi_tile(const TcMaps& maps, const TcEpi& ep, in
   // barrier phases stay in step across the tiles of a persistent CTA
   const int nch = min(NCH, (ep.ncols - n0 + 15) / 16);
   // F1: the inverse scale of this thread's D row; the split output's scale
-  const bool f1 = ep.kind == EPI_F1 || ep.kind == EPI_F1P;
-  const float rsc = f1 ? __ldg(ep.rscale + yrow + lane) : 1.f;
+  const float rsc = ep.kind == EPI_F1 ? __ldg(ep.rscale + yrow + lane) : 1.f;
   const float osc = ep.oscale[t];
   if (nin > 0) {
     // the first chunk's inputs; their buffer was last read two chunks ago
@@ -422,10 +420,10 @@ __device__ __forceinline__ bool epi_tile(const TcMaps& maps, const TcEpi& ep, in
     if (ep.kind == EPI_B1) {
 #pragma unroll
       for (int k = 0; k < 16; ++k) o0[k] = v[k];
-    } else if (f1 || ep.kind == EPI_F2 || ep.kind == EPI_F3) {
+    } else if (ep.kind == EPI_F1 || ep.kind == EPI_F2 || ep.kind == EPI_F3) {
       float bb[16], id[16], wo[16], i2[16];
       colp_ld16(cp.bias + c0, bb);
-      if (!f1) colp_ld16(cp.idt + c0, id);
+      if (ep.kind != EPI_F1) colp_ld16(cp.idt + c0, id);
       if (ep.kind == EPI_F3) {
         colp_ld16(cp.wout + c0, wo);
         colp_ld16(cp.idt2 + c0, i2);
@@ -457,14 +455,6 @@ __device__ __forceinline__ bool epi_tile(const TcMaps& maps, const TcEpi& ep, in
         const float tt = x0[k];
         sv[k] = (ep.kind == EPI_B3 ? g * id[k] : g) * (1.f - tt * tt) * osc;
       }
-    }
-    if (ep.kind == EPI_F1P) {
-      // coalesced 16-byte stores: the warp's 32 rows of a piece are adjacent
-      float4* t1 = ep.t1p + ((size_t)(yrow >> 7) * (FIT_W / 4) + (c >> 2)) * TBM + (yrow & 127) + lane;
-#pragma unroll
-      for (int q = 0; q < 4; ++q)
-        t1[q * TBM] = make_float4(o0[4 * q], o0[4 * q + 1], o0[4 * q + 2], o0[4 * q + 3]);
-      continue;
     }
     uint32_t hw[8], lw[8];
     if (ep.out_mask & 6) pack_split16(sv, hw, lw);
@@ -851,6 +841,193 @@ __global__ void __launch_bounds__(192, 1)
       if (!ok) break;
     }
     if (lane == 0) epi_drain(ib, es, ep.status);
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 0)
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem) : "memory");
+}
+
+// F1 (T1 = tanh(D W1 + b1), K 1600) as a persistent kernel for the fused form.
+// The 512 TMEM columns hold one tile's three main accumulators and the cross
+// terms, so a tile's MMAs cannot start before the last tile's are read: eight
+// epilogue warps (two per TMEM lane quarter) first add the four accumulators
+// into registers and release TMEM, then do the tanh and store T1 while the next
+// tile's loads and MMAs run.  Bounded by the operands' loads (64 KiB a k-block
+// from L2).  One CTA per tile waited for the whole epilogue before its SM's next
+// loads: the whole fitting of 12,288 atoms 150 -> 129 us, of 126,000 1,030 ->
+// 915 us, same bits.
+template <int TBN_, int STAGES_>
+struct F1Cfg {
+  static constexpr int TBN = TBN_, STAGES = STAGES_;
+  static constexpr int B_TILE = TBN * TBK * 2, STAGE = 2 * A_TILE + 2 * B_TILE;
+  static constexpr int SMEM = STAGES * STAGE + 1024 + 256;
+  static constexpr int HALF = (TBN / 2 + 15) / 16 * 16;  // columns of the first warp of a pair
+  static_assert(SMEM <= 227 * 1024 && STAGE % 1024 == 0, "F1 shared memory");
+};
+using F1Wide = F1Cfg<128, 3>;
+using F1Narrow = F1Cfg<80, 4>;
+
+template <class C>
+__global__ void __launch_bounds__(320, 1)
+    k_fit_f1(const __grid_constant__ TcMaps maps, const __grid_constant__ TcEpi ep, int ntn,
+             int ntiles) {
+  constexpr int S = C::STAGES, STAGE = C::STAGE, TBN = C::TBN, B_TILE = C::B_TILE, NACC = 3;
+  constexpr int nkb = FIT_D / TBK;
+  extern __shared__ unsigned char smem_raw[];
+  unsigned char* smem =
+      reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint64_t* full = reinterpret_cast<uint64_t*>(smem + S * STAGE);
+  uint64_t* empty = full + S;
+  uint64_t* tfull = empty + S;   // the tile's accumulators ready
+  uint64_t* tempty = tfull + 1;  // and read (8 epilogue warps)
+  uint64_t* mdone = tempty + 1;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(mdone + 1);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  auto tile_at = [&](int tile, int& row0, int& n0, int& t) {
+    const int rb = tile / ntn;
+    row0 = rb * TBM;
+    n0 = (tile - rb * ntn) * TBN;
+    t = 0;
+    while (t + 1 < ep.ntypes && row0 >= ep.row_off[t + 1]) ++t;
+  };
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < S; ++i) {
+      mbar_init(&full[i], 1);
+      mbar_init(&empty[i], 1);
+    }
+    mbar_init(tfull, 1);
+    mbar_init(tempty, 8);
+    mbar_init(mdone, 1);
+    fence_mbar_init();
+  }
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(
+                     smem_addr(tmem_slot))
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = *tmem_slot;
+
+  if (warp == 0) {
+    if (lane == 0) {
+      // ---- TMA producer: runs into the next tile's k-blocks as stages free up
+      int issued = 0;
+      bool ok = true;
+      griddep_wait();
+      for (int tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x) {
+        int row0, n0, t;
+        tile_at(tile, row0, n0, t);
+        for (int kb = 0; kb < nkb; ++kb) {
+          const int st_i = issued % S;
+          if (issued >= S &&
+              !mbar_wait_bounded(&empty[st_i], ((issued / S) & 1u) ^ 1u, ep.status)) {
+            ok = false;
+            break;
+          }
+          unsigned char* st = smem + st_i * STAGE;
+          mbar_expect_tx(&full[st_i], STAGE);
+          tma_2d(st, &maps.a_hi, kb * TBK, row0, &full[st_i]);
+          tma_2d(st + A_TILE, &maps.a_lo, kb * TBK, row0, &full[st_i]);
+          tma_2d(st + 2 * A_TILE, &maps.b_hi[t], kb * TBK, n0, &full[st_i]);
+          tma_2d(st + 2 * A_TILE + B_TILE, &maps.b_lo[t], kb * TBK, n0, &full[st_i]);
+          ++issued;
+        }
+      }
+      // no bulk copy of this CTA may land after it exits
+      for (int k = (issued > S ? issued - S : 0); k < issued; ++k)
+        mbar_wait_bounded(&full[k % S], (k / S) & 1u, ep.status);
+    }
+  } else if (warp == 1) {
+    if (lane == 0) {
+      // ---- MMA issuer: D(f32) += A(f16, K-major) B(f16, K-major), M 128
+      const uint32_t idesc = (1u << 4) | ((uint32_t)(TBN >> 3) << 17) | ((uint32_t)(TBM >> 4) << 24);
+      const uint32_t dsmall = tmem + 128u * NACC;
+      int cons = 0, it = 0;
+      bool ok = true;
+      for (int tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x, ++it) {
+        if (it > 0 && !mbar_wait_bounded(tempty, (unsigned)(it - 1) & 1u, ep.status)) break;
+        tc_fence_after();
+        for (int kb = 0; kb < nkb; ++kb) {
+          const int st_i = cons % S;
+          if (!mbar_wait_bounded(&full[st_i], (cons / S) & 1u, ep.status)) {
+            ok = false;
+            break;
+          }
+          tc_fence_after();
+          const uint32_t ah = smem_addr(smem + st_i * STAGE), al = ah + A_TILE,
+                         bh = ah + 2 * A_TILE, bl = bh + B_TILE;
+          const uint32_t dmain = tmem + (uint32_t)(kb % NACC) * 128u;
+#pragma unroll
+          for (int kk = 0; kk < TBK / 16; ++kk) {
+            const uint32_t off = kk * 32;
+            const uint64_t dah = sdesc_sw128(ah + off), dal = sdesc_sw128(al + off),
+                           dbh = sdesc_sw128(bh + off), dbl = sdesc_sw128(bl + off);
+            umma_f16(dmain, dah, dbh, idesc, (kb >= NACC || kk > 0) ? 1u : 0u);
+            umma_f16(dsmall, dal, dbh, idesc, (kb > 0 || kk > 0) ? 1u : 0u);
+            umma_f16(dsmall, dah, dbl, idesc, 1u);
+          }
+          umma_commit(&empty[st_i]);
+          ++cons;
+        }
+        if (ok) umma_commit(tfull);
+      }
+      // every MMA issued complete before TMEM is released
+      umma_commit(mdone);
+      mbar_wait_bounded(mdone, 0, ep.status);
+    }
+  } else {
+    // ---- epilogue warps
+    griddep_wait();  // the row scales visible; earlier readers of T1 done
+    const int q = warp & 3, half = (warp - 2) >> 2;
+    constexpr int NCMAX = C::HALF / 16;
+    int it = 0;
+    for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x, ++it) {
+      if (!__all_sync(kFull, mbar_wait_bounded(tfull, (unsigned)it & 1u, ep.status))) break;
+      tc_fence_after();
+      // the next launch may start filling SMs once this CTA's last tile drains
+      if (tile + (int)gridDim.x >= ntiles) griddep_launch_dependents();
+      int row0, n0, t;
+      tile_at(tile, row0, n0, t);
+      const int r = q * 32 + lane, cl = half * C::HALF;
+      const int nc = min(half ? TBN - C::HALF : C::HALF, FIT_W - n0 - cl) / 16;
+      const uint32_t tacc = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)cl;
+      float acc[NCMAX][16];
+#pragma unroll
+      for (int ch = 0; ch < NCMAX; ++ch) {
+        if (ch >= nc) break;  // uniform
+        float w[16];
+        tmem_ld16x2(tacc + 16u * ch, tacc + 128u + 16u * ch, acc[ch], w);
+#pragma unroll
+        for (int k = 0; k < 16; ++k) acc[ch][k] += w[k];
+        float x[16];
+        tmem_ld16x2(tacc + 256u + 16u * ch, tacc + 384u + 16u * ch, w, x);
+#pragma unroll
+        for (int k = 0; k < 16; ++k) acc[ch][k] = (acc[ch][k] + w[k]) + x[k];
+      }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(tempty);
+      const float rsc = __ldg(ep.rscale + row0 + r);
+      float4* t1 = ep.t1p + (size_t)(row0 >> 7) * (FIT_W / 4) * TBM + r;
+#pragma unroll
+      for (int ch = 0; ch < NCMAX; ++ch) {
+        if (ch >= nc) break;  // uniform
+        const int c = n0 + cl + 16 * ch;
+        float cs[16], bb[16];
+        colp_ld16(ep.cscale[t] + c, cs);
+        colp_ld16(ep.bias[t] + c, bb);
+#pragma unroll
+        for (int k = 0; k < 16; ++k) acc[ch][k] = tanhf(acc[ch][k] * cs[k] * rsc + bb[k]);
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+          t1[((c >> 2) + u) * TBM] = make_float4(acc[ch][4 * u], acc[ch][4 * u + 1],
+                                                 acc[ch][4 * u + 2], acc[ch][4 * u + 3]);
+      }
+    }
   }
   tc_fence_before();
   __syncthreads();
@@ -1616,7 +1793,7 @@ extern "C" int gbdp_fitting_tc_f32(float* e, float* dE_dD, const void* D_hi, con
     GBDP_REQUIRE(((uintptr_t)nets[t].idt[1] & 15) == 0 && ((uintptr_t)nets[t].idt[2] & 15) == 0,
                  "fit_tc: idt not 16-byte aligned");
   }
-  enum { LONGK = 0, SHORTK, PERSIST, LONG16, SHORT16, LONG48, SHORT48, B1PERS };
+  enum { LONGK = 0, SHORTK, PERSIST, LONG16, SHORT16, LONG48, SHORT48, B1PERS, F1WIDE, F1NARROW };
   // the K-240 layers go to the persistent kernel from this many tiles per SM
   const long short_tiles = (rows / TBM) * (FIT_W / CfgShortK::TBN);
   const long nblk = rows / TBM;
@@ -1631,8 +1808,17 @@ extern "C" int gbdp_fitting_tc_f32(float* e, float* dE_dD, const void* D_hi, con
                                                                 : SHORTK;
   // B1 in 48-column tiles while they fit one wave
   const int b1_cfg = nblk * ((FIT_D + 47) / 48) <= nsm ? SHORT48 : B1PERS;
+  // F1 of the fused form: the tile width whose rounds over the SMs move fewer
+  // bytes (the loads bound it): 128 columns read D twice, 80 three times, but
+  // 80 leave a smaller last round (whole fitting, 128 / 80, us: 9,000 rows 113 /
+  // 121, 12,288: 136 / 129, 126,000: 914 / 974)
+  const long wide = (nblk * 2 + nsm - 1) / nsm * F1Wide::STAGE,
+             slim = (nblk * 3 + nsm - 1) / nsm * F1Narrow::STAGE;
+  const int f1_cfg = !fused ? long_cfg : slim < wide ? F1NARROW : F1WIDE;
   auto width_of = [](int cfg) {
-    return cfg == LONGK                        ? CfgLongK::TBN
+    return cfg == F1WIDE                       ? F1Wide::TBN
+           : cfg == F1NARROW                   ? F1Narrow::TBN
+           : cfg == LONGK                        ? CfgLongK::TBN
            : cfg == SHORTK                     ? CfgShortK::TBN
            : cfg == PERSIST || cfg == B1PERS  ? PERS_TBN
            : cfg == LONG16 || cfg == SHORT16 ? 16
@@ -1656,7 +1842,7 @@ extern "C" int gbdp_fitting_tc_f32(float* e, float* dE_dD, const void* D_hi, con
                 "tile widths must divide the layer widths (F1's last tile may be partial)");
   const Step steps[6] = {
       {EPI_F1, D_hi, D_lo, FIT_D, FIT_W, 0, true, {nullptr, nullptr}, {ws.t1, ws.h1h, ws.h1l}, 0,
-       long_cfg},
+       f1_cfg},
       {EPI_F2, ws.h1h, ws.h1l, FIT_W, FIT_W, 1, true, {ws.t1, nullptr}, {ws.t2, ws.h2h, ws.h2l},
        1, short_cfg},
       {EPI_F3, ws.h2h, ws.h2l, FIT_W, FIT_W, 2, true, {ws.t1, ws.t2},
@@ -1689,7 +1875,7 @@ extern "C" int gbdp_fitting_tc_f32(float* e, float* dE_dD, const void* D_hi, con
       if (!rc) rc = make_map(&maps.b_lo[t], bl, sp.N, sp.K, tbn);
     }
     TcEpi ep = base;
-    ep.kind = f1p ? EPI_F1P : sp.kind;
+    ep.kind = sp.kind;
     ep.t1p = reinterpret_cast<float4*>(ws.t1);
     ep.ncols = sp.N;
     ep.nin = 0;
@@ -1729,7 +1915,19 @@ extern "C" int gbdp_fitting_tc_f32(float* e, float* dE_dD, const void* D_hi, con
     lc.blockDim = dim3(128);
     lc.stream = st;
     cudaError_t le;
-    if (sp.cfg != PERSIST && sp.cfg != B1PERS) {
+    if (f1p) {
+      const bool w = sp.cfg == F1WIDE;
+      const int ntn = (FIT_W + width_of(sp.cfg) - 1) / width_of(sp.cfg), ntiles = ntn * (int)nblk;
+      lc.gridDim = dim3((unsigned)(ntiles < nsm ? ntiles : nsm));
+      lc.blockDim = dim3(320);
+      lc.dynamicSmemBytes = w ? F1Wide::SMEM : F1Narrow::SMEM;
+      cudaFuncSetAttribute(k_fit_f1<F1Wide>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           F1Wide::SMEM);
+      cudaFuncSetAttribute(k_fit_f1<F1Narrow>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           F1Narrow::SMEM);
+      le = w ? cudaLaunchKernelEx(&lc, k_fit_f1<F1Wide>, maps, ep, ntn, ntiles)
+             : cudaLaunchKernelEx(&lc, k_fit_f1<F1Narrow>, maps, ep, ntn, ntiles);
+    } else if (sp.cfg != PERSIST && sp.cfg != B1PERS) {
       lc.gridDim = dim3((sp.N + width_of(sp.cfg) - 1) / width_of(sp.cfg), (unsigned)nblk);
       switch (sp.cfg) {
         case LONGK: le = launch_tile<CfgLongK>(lc, maps, ep, sp.K); break;
