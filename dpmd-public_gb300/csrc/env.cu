@@ -12,6 +12,7 @@
 //                cells, per-type rank by (float r^2, index), env matrix row
 //                and its derivative, normalised by davg/dstd.
 #include <algorithm>
+#include <cfloat>
 #include <cstring>
 #include <cmath>
 #include <mutex>
@@ -459,21 +460,42 @@ __device__ __forceinline__ void store4<double>(double* p, double a, double b, do
   *reinterpret_cast<double2*>(p + 2) = make_double2(c, d);
 }
 
+// The four statistics of a slot; one 16-byte load in FP32 when the arrays
+// allow it (vec: both start on a 16-byte boundary; rows are 4 nnei wide).
+template <typename T>
+__device__ __forceinline__ void load4(T* v, const T* p, bool vec) {
+#pragma unroll
+  for (int q = 0; q < 4; ++q) v[q] = p[q];
+}
+template <>
+__device__ __forceinline__ void load4<float>(float* v, const float* p, bool vec) {
+  if (vec) {
+    const float4 r = *reinterpret_cast<const float4*>(p);
+    v[0] = r.x;
+    v[1] = r.y;
+    v[2] = r.z;
+    v[3] = r.w;
+  } else {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) v[q] = p[q];
+  }
+}
+
 // a / b: the fast reciprocal-multiply division in FP32 (2 ulp), IEEE in FP64
 __device__ __forceinline__ float div_t(float a, float b) { return __fdividef(a, b); }
 __device__ __forceinline__ double div_t(double a, double b) { return a / b; }
 
 // Env row of one slot (env_mat.cc:122-226: s(r) [1/r, x/r^2, y/r^2, z/r^2]
 // and its derivative wrt r_ij), normalised by the centre type's davg/dstd
-// (prod_env_mat.cc:84-100), stored at row o; xj == nullptr: the padding row
+// (prod_env_mat.cc:84-100; avg, stdv: the slot's four), stored at row o; xj == nullptr: the padding row
 // (0 - avg) / std; centre type < 0: zeros.  1/r and x/r^2 are formed from
 // 1/sqrt(r^2) and the normalisation divides with div_t (within two ulp of
 // the reference's divisions in FP32); the derivative row is formed only when
 // em_deriv is requested.
 template <typename T>
 __device__ __forceinline__ void env_row_store(const T* xj, T xi, T yi, T zi, int ti,
-                                              const T* av, const T* sd, int s, T rmin, T rmax,
-                                              size_t o, T* em, T* em_deriv, T* rij) {
+                                              const T* avg, const T* stdv, bool vec, T rmin,
+                                              T rmax, size_t o, T* em, T* em_deriv, T* rij) {
   T e[4] = {T(0), T(0), T(0), T(0)};
   T rr[3] = {T(0), T(0), T(0)};
   T inr = T(0), inr2 = T(0), sw = T(0), dsw = T(0);
@@ -491,10 +513,12 @@ __device__ __forceinline__ void env_row_store(const T* xj, T xi, T yi, T zi, int
     e[2] = rr[1] * inr2;
     e[3] = rr[2] * inr2;
   }
-  T out[4];
+  T out[4], av[4], sd[4];
   if (ti >= 0) {
+    load4<T>(av, avg, vec);
+    load4<T>(sd, stdv, vec);
 #pragma unroll
-    for (int q = 0; q < 4; ++q) out[q] = div_t(e[q] * sw - av[s * 4 + q], sd[s * 4 + q]);
+    for (int q = 0; q < 4; ++q) out[q] = div_t(e[q] * sw - av[q], sd[q]);
   } else {
 #pragma unroll
     for (int q = 0; q < 4; ++q) out[q] = T(0);
@@ -522,9 +546,8 @@ __device__ __forceinline__ void env_row_store(const T* xj, T xi, T yi, T zi, int
 #pragma unroll
     for (int q = 0; q < 12; q += 4) {
       if (ti >= 0)
-        store4<T>(dp + q, div_t(dv[q], sd[s * 4 + q / 3]), div_t(dv[q + 1], sd[s * 4 + (q + 1) / 3]),
-                  div_t(dv[q + 2], sd[s * 4 + (q + 2) / 3]),
-                  div_t(dv[q + 3], sd[s * 4 + (q + 3) / 3]));
+        store4<T>(dp + q, div_t(dv[q], sd[q / 3]), div_t(dv[q + 1], sd[(q + 1) / 3]),
+                  div_t(dv[q + 2], sd[(q + 2) / 3]), div_t(dv[q + 3], sd[(q + 3) / 3]));
       else
         store4<T>(dp + q, T(0), T(0), T(0), T(0));
     }
@@ -579,22 +602,83 @@ __device__ __forceinline__ void warp_bitonic(uint64_t* v, int lane) {
   }
 }
 
-// One type's candidates (n <= 32 E keys (r^2, index) at stage[0, n)) sorted
-// by a warp and the first sel of them placed at their ranks in row[].
+// One type's candidates (n <= 32 E, r^2 at r2s[0, n), index at ids[0, n))
+// sorted by (r^2, index) in a warp and the first sel of them placed at their
+// ranks in row[].
 template <int E>
-__device__ __forceinline__ void sort_type_rows(const uint64_t* stage, int n, int sel, int* row,
-                                               int lane) {
+__device__ __forceinline__ void sort_type_rows(const float* r2s, const int* ids, int n, int sel,
+                                               int* row, int lane) {
   uint64_t v[E];
 #pragma unroll
   for (int e = 0; e < E; ++e) {
     const int c = e * 32 + lane;
-    v[e] = c < n ? stage[c] : ~0ull;
+    v[e] = c < n ? ((uint64_t)__float_as_uint(r2s[c]) << 32) | (uint32_t)ids[c] : ~0ull;
   }
   warp_bitonic<E>(v, lane);
 #pragma unroll
   for (int e = 0; e < E; ++e) {
     const int pos = e * 32 + lane;
     if (pos < n && pos < sel) row[pos] = (int)(uint32_t)(v[e] & 0xffffffffu);
+  }
+}
+
+// The same placement by counting: a candidate's rank is the number of
+// smaller r^2, each comparison a saturated multiply-add (1 when smaller, else
+// 0) and an add: two instructions of the FMA pipe a key and candidate, where
+// the network spends some eight of the ALU pipe on every one of its
+// log2(n)^2 / 2 steps.  The r^2 are read four at a time (padded to a multiple
+// of four with FLT_MAX).  Equal r^2, or a difference that 2^100 does not
+// carry past 1, leave a pair uncounted on both sides and the ranks' sum short
+// of n (n - 1) / 2: false then, nothing placed, and the caller sorts.
+template <int E>
+__device__ __forceinline__ bool rank_type_rows(const float* r2s, const int* ids, int n, int sel,
+                                               int* row, int lane) {
+  constexpr float kBig = 0x1p100f;
+  float mine[E], rank[E];
+#pragma unroll
+  for (int e = 0; e < E; ++e) {
+    const int c = e * 32 + lane;
+    mine[e] = c < n ? r2s[c] * kBig : 0.f;
+    rank[e] = 0.f;
+  }
+  for (int d = 0; d < n; d += 4) {
+    const float4 k = *reinterpret_cast<const float4*>(r2s + d);
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+      rank[e] += __saturatef(fmaf(k.x, -kBig, mine[e]));
+      rank[e] += __saturatef(fmaf(k.y, -kBig, mine[e]));
+      rank[e] += __saturatef(fmaf(k.z, -kBig, mine[e]));
+      rank[e] += __saturatef(fmaf(k.w, -kBig, mine[e]));
+    }
+  }
+  int sum = 0;
+#pragma unroll
+  for (int e = 0; e < E; ++e)
+    if (e * 32 + lane < n) sum += (int)rank[e];
+  if (__reduce_add_sync(kFull, sum) != n * (n - 1) / 2) return false;
+#pragma unroll
+  for (int e = 0; e < E; ++e) {
+    const int c = e * 32 + lane, pos = (int)rank[e];
+    if (c < n && pos < sel) row[pos] = ids[c];
+  }
+  return true;
+}
+
+// The first sel of one type's n <= 128 candidates at their places in row[];
+// room for the padding is part of the 128.
+__device__ __forceinline__ void place_type(float* r2s, const int* ids, int n, int sel, int* row,
+                                           int lane) {
+  if (n == 0 || sel == 0) return;
+  if (n + lane < ((n + 3) & ~3)) r2s[n + lane] = FLT_MAX;
+  __syncwarp();
+  if (n <= 32) {
+    if (!rank_type_rows<1>(r2s, ids, n, sel, row, lane))
+      sort_type_rows<1>(r2s, ids, n, sel, row, lane);
+  } else if (n <= 64) {
+    if (!rank_type_rows<2>(r2s, ids, n, sel, row, lane))
+      sort_type_rows<2>(r2s, ids, n, sel, row, lane);
+  } else if (n > 96 || !rank_type_rows<3>(r2s, ids, n, sel, row, lane)) {
+    sort_type_rows<4>(r2s, ids, n, sel, row, lane);
   }
 }
 
@@ -614,6 +698,14 @@ struct VList {
 //   kEnvBuild  candidates from the cell stencil (rc2f = (rcut + skin)^2)
 //              written to the Verlet list; nothing else
 enum { kEnvCells = 0, kEnvList = 1, kEnvBuild = 2 };
+
+// A warp per centre, bound by instruction issue (72 % of the slots, 0.22 ms
+// for 51,304 atoms; some 3,800 warp instructions a centre: 40 % the cell
+// search, a quarter each the ordering and the rows).  On 125,000 atoms of
+// ragged water the neighbour part of a step took 640 us with every half cell
+// of the stencil searched, the types sorted by networks and the statistics
+// loaded one value at a time, and 548 us now; of the three alone, searching
+// every cell again gives 628, sorting 661, single loads 557.
 
 template <typename T, int MODE>
 __global__ void __launch_bounds__(kEnvWarps * 32)
@@ -700,6 +792,25 @@ __global__ void __launch_bounds__(kEnvWarps * 32)
       F[d] = fs[d] * (cc[d] + g.ngcell[d]) + (split ? (hs >> d) & 1 : 0);
     }
   }
+  // A box along the axes: a stencil cell whose nearest point is beyond rc is
+  // skipped without a look at its counts (of 125 half cells half a cutoff
+  // wide some 85 remain).  uf: the centre's position in its own fine cell, in
+  // cell widths wf; the distance to a cell o away is max(o - u, u - o - 1)
+  // widths, less a margin for FP32 rounding: of u (some 3e-7 of the grid's
+  // extent) and of stored image coordinates (far below 1e-3 of a cell).
+  bool diag = MODE != kEnvList;
+  float uf[3], wf[3], mf[3];
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    const float nf = (float)(fs[d] * g.ncell[d]);
+    wf[d] = __fdividef(g.boxf[4 * d], nf);
+    uf[d] = (float)(d == 0 ? xi : d == 1 ? yi : zi) * (g.recf[4 * d] * nf) -
+            (float)(F[d] - fs[d] * g.ngcell[d]);
+    mf[d] = 1e-3f + 1e-6f * nf;
+    diag = diag && g.boxf[4 * d] > 0.f && g.box[3 * d + (d + 1) % 3] == 0. &&
+           g.box[3 * d + (d + 2) % 3] == 0.;
+  }
+  const float far2 = diag ? rc2f * 1.0001f : FLT_MAX;
   const int sy = 2 * hw[1] + 1, sz = 2 * hw[2] + 1;
   const int nst = MODE == kEnvList ? 0 : (2 * hw[0] + 1) * sy * sz;
   // stencil offsets from the flat index by reciprocal multiplies instead of
@@ -716,15 +827,21 @@ __global__ void __launch_bounds__(kEnvWarps * 32)
       const int q1 = (int)(((float)rq + 0.5f) * inv_z), q2 = rq - q1 * sz;
       const int o[3] = {q0 - hw[0], q1 - hw[1], q2 - hw[2]};
       int E[3], h = 0;
+      float d2 = 0.f;
 #pragma unroll
       for (int d = 0; d < 3; ++d) {
         const int fp = F[d] + o[d];  // >= 0: the ghost layers cover the stencil
         E[d] = fs[d] == 2 ? fp >> 1 : fp;
         if (fs[d] == 2) h |= (fp & 1) << d;
+        const float x = (float)o[d] - uf[d];
+        const float gap = fmaxf(fmaxf(x, -1.f - x) - mf[d], 0.f) * wf[d];
+        d2 = fmaf(gap, gap, d2);
       }
-      const int* es = ext_sub + 9 * (size_t)(g.ext_cell_off + (E[0] * n1 + E[1]) * n2 + E[2]);
-      st = es[h];
-      cnt = es[h + 1] - st;
+      if (!(d2 > far2)) {
+        const int* es = ext_sub + 9 * (size_t)(g.ext_cell_off + (E[0] * n1 + E[1]) * n2 + E[2]);
+        st = es[h];
+        cnt = es[h + 1] - st;
+      }
     }
     int incl = cnt;
 #pragma unroll
@@ -780,33 +897,30 @@ __global__ void __launch_bounds__(kEnvWarps * 32)
   }
   for (int s = lane; s < nnei; s += 32) row[s] = -1;
   __syncwarp();
-  if (ncand <= 128 && max_cand >= 256) {
-    // ---- up to 128 candidates: each type's (r^2, index) keys compacted
-    //      into a staging area past them (keys[128, 256)) and sorted on
-    //      their own by the smallest bitonic network that holds them (32,
-    //      64 or 128 keys): about half the compare-exchange steps of one
-    //      128-key sort over all types on water (~30 O and ~60 H)
-    uint64_t* stage = keys + 128;
+  if (ncand <= 128 && max_cand >= 256 && (max_cand & 1) == 0) {
+    // ---- up to 128 candidates: each type's compacted into a staging area
+    //      past the keys (keys[128, 256): 128 r^2, then 128 indices, 16-byte
+    //      aligned when max_cand is even) and ranked by counting up to 96;
+    //      more of one type, or equal r^2, by the smallest bitonic network
+    //      that holds them (32, 64 or 128)
+    float* r2s = reinterpret_cast<float*>(keys + 128);
+    int* ids = reinterpret_cast<int*>(keys + 192);
     for (int t = 0; t < si.ntypes; ++t) {
       int n = 0;
       for (int c0 = 0; c0 < ncand; c0 += 32) {
         const int cc = c0 + lane;
         const bool is_t = cc < ncand && (int)ctype[cc] == t;
         const unsigned m = __ballot_sync(kFull, is_t);
-        if (is_t) stage[n + __popc(m & ((1u << lane) - 1u))] = keys[cc];
+        if (is_t) {
+          const int p = n + __popc(m & ((1u << lane) - 1u));
+          const uint64_t k = keys[cc];
+          r2s[p] = __uint_as_float((uint32_t)(k >> 32));
+          ids[p] = (int)(uint32_t)(k & 0xffffffffu);
+        }
         n += __popc(m);
       }
       __syncwarp();
-      const int sel_t = si.sec[t + 1] - si.sec[t];
-      int* rt = row + si.sec[t];
-      if (n > 0 && sel_t > 0) {
-        if (n <= 32)
-          sort_type_rows<1>(stage, n, sel_t, rt, lane);
-        else if (n <= 64)
-          sort_type_rows<2>(stage, n, sel_t, rt, lane);
-        else
-          sort_type_rows<4>(stage, n, sel_t, rt, lane);
-      }
+      place_type(r2s, ids, n, si.sec[t + 1] - si.sec[t], row + si.sec[t], lane);
       __syncwarp();  // the staging area is read before the next type refills it
     }
   } else if (ncand <= 128) {
@@ -869,11 +983,12 @@ __global__ void __launch_bounds__(kEnvWarps * 32)
   const int nem = nnei * 4;
   const T* av = avg + (size_t)max(ti, 0) * nem;
   const T* sd = stdv + (size_t)max(ti, 0) * nem;
+  const bool vec = (((uintptr_t)avg | (uintptr_t)stdv) & 15) == 0;
   for (int s = lane; s < nnei; s += 32) {
     const int j = row[s];
     const size_t o = ((size_t)i * nnei + s);
-    env_row_store<T>(j >= 0 ? ext_coord + 3 * (eoff + j) : nullptr, xi, yi, zi, ti, av, sd, s,
-                     rmin, rmax, o, em, em_deriv, rij);
+    env_row_store<T>(j >= 0 ? ext_coord + 3 * (eoff + j) : nullptr, xi, yi, zi, ti, av + 4 * s,
+                     sd + 4 * s, vec, rmin, rmax, o, em, em_deriv, rij);
     nlist[o] = j >= 0 ? ext_map[eoff + j] : -1;
     if (nlist_ext) nlist_ext[o] = j;
   }
@@ -925,8 +1040,10 @@ __global__ void __launch_bounds__(kEnvWarps * 32)
   const int cap = (nnei_in + 7) & ~7;
   unsigned char* base = smem + (size_t)warp * nlist_ext_warp_bytes<T>(nnei_in, nnei);
   // candidates within rcut, in list order: distance, list position, type;
-  // row: the candidate of each slot; FP32: 128 sort keys
-  uint64_t* stage = reinterpret_cast<uint64_t*>(base);
+  // row: the candidate of each slot; FP32: 128 distances and
+  // candidate numbers of the type being placed
+  float* rrs = reinterpret_cast<float*>(base);
+  int* ids = reinterpret_cast<int*>(base + 512);
   T* cd = reinterpret_cast<T*>(base + (sizeof(T) == 4 ? 1024 : 0));
   int* row = reinterpret_cast<int*>(cd + cap);
   uint16_t* cpos = reinterpret_cast<uint16_t*>(row + ((nnei + 3) & ~3));
@@ -981,7 +1098,7 @@ __global__ void __launch_bounds__(kEnvWarps * 32)
   for (int s = lane; s < nnei; s += 32) row[s] = -1;
   __syncwarp();
   if (sizeof(T) == 4 && ncand <= 128 && ncand <= nnei) {
-    // ---- every candidate is among the nearest nnei: each type sorted on its
+    // ---- every candidate is among the nearest nnei: each type placed on its
     //      own by (rr, list order), as k_nlist_env does (rr >= 0: its bit
     //      pattern orders as the value)
     for (int t = 0; t < si.ntypes; ++t) {
@@ -990,22 +1107,15 @@ __global__ void __launch_bounds__(kEnvWarps * 32)
         const int c = c0 + lane;
         const bool is_t = c < ncand && (int)ctype[c] == t;
         const unsigned m = __ballot_sync(kFull, is_t);
-        if (is_t)
-          stage[n + __popc(m & ((1u << lane) - 1u))] =
-              ((uint64_t)__float_as_uint((float)cd[c]) << 32) | (uint32_t)c;
+        if (is_t) {
+          const int p = n + __popc(m & ((1u << lane) - 1u));
+          rrs[p] = (float)cd[c];
+          ids[p] = c;
+        }
         n += __popc(m);
       }
       __syncwarp();
-      const int sel_t = si.sec[t + 1] - si.sec[t];
-      int* rt = row + si.sec[t];
-      if (n > 0 && sel_t > 0) {
-        if (n <= 32)
-          sort_type_rows<1>(stage, n, sel_t, rt, lane);
-        else if (n <= 64)
-          sort_type_rows<2>(stage, n, sel_t, rt, lane);
-        else
-          sort_type_rows<4>(stage, n, sel_t, rt, lane);
-      }
+      place_type(rrs, ids, n, si.sec[t + 1] - si.sec[t], row + si.sec[t], lane);
       __syncwarp();  // the staging area is read before the next type refills it
     }
   } else {
@@ -1046,11 +1156,12 @@ __global__ void __launch_bounds__(kEnvWarps * 32)
   const int nem = nnei * 4;
   const T* av = avg + (size_t)max(ti, 0) * nem;
   const T* sd = stdv + (size_t)max(ti, 0) * nem;
+  const bool vec = (((uintptr_t)avg | (uintptr_t)stdv) & 15) == 0;
   for (int s = lane; s < nnei; s += 32) {
     const int c = row[s], j = c >= 0 ? nl[cpos[c]] : -1;
     const size_t o = ((size_t)i * nnei + s);
-    env_row_store<T>(j >= 0 ? xf + 3 * j : nullptr, xi, yi, zi, ti, av, sd, s, rmin, rmax, o, em,
-                     em_deriv, rij);
+    env_row_store<T>(j >= 0 ? xf + 3 * j : nullptr, xi, yi, zi, ti, av + 4 * s, sd + 4 * s, vec,
+                     rmin, rmax, o, em, em_deriv, rij);
     nlist[o] = j;
   }
 }

@@ -284,3 +284,55 @@ def test_external_nlist_candidate_counts(gb, oracle, dtype, inside, width, sel):
                                                          rcut, 0.5, list(sel))
     exp = oracle.format_nlist_pt(ext, typ, nl, nloc, rcut, list(sel))
     np.testing.assert_array_equal(got.cpu().numpy().reshape(nloc, -1), exp)
+
+
+def _check_lists(gb, oracle, coord, typ, box, dtype, sel, rcut=6.0):
+    nt, nnei = len(sel), sum(sel)
+    avg, std = np.zeros((nt, nnei * 4), dtype), np.ones((nt, nnei * 4), dtype)
+    em, _, _, nl, ec, et, emap = oracle.prod_env_mat_a_pbc(
+        coord, typ, box.reshape(-1).astype(dtype), avg, std, rcut, 0.5, list(sel), return_ext=True)
+    tdt = torch.float64 if dtype == np.float64 else torch.float32
+    plan = gb.NeighborPlan([len(typ)], box.reshape(1, 9), rcut, DEV, tdt)
+    D = lambda a: torch.tensor(a, device=DEV)
+    # statistics on a 16-byte boundary and one element off it
+    for off in (0, 1):
+        st = [D(np.concatenate([np.zeros(off, dtype), a.reshape(-1)]))[off:].view(nt, -1)
+              for a in (avg, std)]
+        r = gb.env_mat_packed(plan, D(coord), D(typ), *st, 0.5, list(sel), need_nlist_ext=True)
+        np.testing.assert_array_equal(r.nlist.cpu().numpy().reshape(-1), nl)
+        # the FP32 bound of test_ragged_batch_vs_oracle
+        tol = 1e-12 if dtype == np.float64 else 5e-6
+        np.testing.assert_allclose(r.em.cpu().numpy().reshape(-1), em, atol=tol, rtol=tol)
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("n0,n1", [(1, 1), (2, 0), (32, 5), (33, 34), (64, 33), (65, 64), (96, 31),
+                                   (97, 32), (98, 31), (128, 1), (129, 0), (90, 70)])
+def test_candidates_per_type(gb, oracle, dtype, n0, n1):
+    """A cluster across a box corner whose atoms all see one another: every
+    centre has n0 and n1 candidates of the two types, itself left out (the
+    rows at 4-key padding, 32, 64 and 96 of a type, 128 of all)."""
+    rng = np.random.default_rng(100 * n0 + n1)
+    v = rng.normal(size=(n0 + n1, 3))
+    v *= rng.uniform(0.6, 2.9, (n0 + n1, 1)) / np.linalg.norm(v, axis=1)[:, None]
+    typ = rng.permutation(np.repeat([0, 1], [n0, n1])).astype(np.int32)
+    _check_lists(gb, oracle, v.astype(dtype), typ, np.diag([26., 26., 26.]), dtype, (60, 100))
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("tilt", [0.0, 0.7])
+@pytest.mark.parametrize("edges", [(13.0, 19.5, 40.0), (6.1, 12.5, 5.0), (100.0, 7.0, 23.0)])
+def test_cells_beyond_the_cutoff(gb, oracle, dtype, tilt, edges):
+    """Boxes along the axes (stencil cells out of reach are skipped) and
+    tilted ones (all are searched); a third of the coordinates on cell and
+    half-cell faces, some outside the box."""
+    rng = np.random.default_rng(int(edges[0] * 10) + int(10 * tilt))
+    box = np.diag(edges) + tilt * np.tril(np.ones((3, 3)), -1)
+    n = max(8, int(0.05 * np.prod(edges)))
+    frac = rng.uniform(-0.3, 1.3, (n, 3))
+    half = 2 * np.maximum(1, np.floor(np.array(edges) / 6.0))
+    snap = rng.random((n, 3)) < 1 / 3
+    frac[snap] = (np.round(frac * half) / half)[snap]
+    coord = (frac @ box + rng.uniform(-1e-3, 1e-3, (n, 3)) * ~snap).astype(dtype)
+    typ = rng.integers(0, 2, n).astype(np.int32)
+    _check_lists(gb, oracle, coord, typ, box, dtype, (46, 92))
