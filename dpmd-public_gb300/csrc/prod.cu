@@ -66,32 +66,11 @@ __device__ __forceinline__ void scatter9(double* p, const double* t) {
 #pragma unroll
   for (int q = 0; q < 9; ++q) atomicAdd(p + q, t[q]);
 }
+// FP32: p is a padded 12-float row, 16-byte aligned
 __device__ __forceinline__ void scatter9(float* p, const float* t) {
-  // p is 4-byte aligned; split the row at its 8- and 16-byte boundaries
-  switch ((reinterpret_cast<uintptr_t>(p) >> 2) & 3) {
-    case 0:
-      red4(p, t[0], t[1], t[2], t[3]);
-      red4(p + 4, t[4], t[5], t[6], t[7]);
-      atomicAdd(p + 8, t[8]);
-      break;
-    case 1:
-      atomicAdd(p, t[0]);
-      red2(p + 1, t[1], t[2]);
-      red4(p + 3, t[3], t[4], t[5], t[6]);
-      red2(p + 7, t[7], t[8]);
-      break;
-    case 2:
-      red2(p, t[0], t[1]);
-      red4(p + 2, t[2], t[3], t[4], t[5]);
-      red2(p + 6, t[6], t[7]);
-      atomicAdd(p + 8, t[8]);
-      break;
-    default:
-      atomicAdd(p, t[0]);
-      red4(p + 1, t[1], t[2], t[3], t[4]);
-      red4(p + 5, t[5], t[6], t[7], t[8]);
-      break;
-  }
+  red4(p, t[0], t[1], t[2], t[3]);
+  red4(p + 4, t[4], t[5], t[6], t[7]);
+  atomicAdd(p + 8, t[8]);
 }
 
 // ---------------------------------------------------------- atomic mode --
@@ -103,6 +82,7 @@ __device__ __forceinline__ void scatter9(float* p, const float* t) {
 // (vector) reductions, F_i by one warp reduction per row; the frame virial
 // as per-lane partials in T over at most 8 rows, folded into a double on
 // lane 0 and added to the frame's accumulator when the frame changes.
+// Forces, and forces with virials; the virial alone: k_virial_pairs.
 template <typename T, int U, bool WV>
 struct ScatterChunk {
   T g[U][4], d[U][12], r[U][3];
@@ -157,6 +137,7 @@ constexpr int kScatterWarps = 4;
 // reductions of a warp go to 32 distinct rows, and their cost in the
 // load/store unit scales with the instructions, not the bytes (measured: the
 // two-instruction form spends about a quarter of the force call on them).
+// Atomic virial rows are padded to 12 floats for the same reason.
 template <typename T, bool F4>
 __device__ __forceinline__ void scatter_force(T* __restrict__ force, size_t row, const T* v) {
   if constexpr (F4) {
@@ -244,7 +225,7 @@ __global__ void __launch_bounds__(kScatterWarps * 32) k_scatter_atomic(
         for (int a = 0; a < 3; ++a)
 #pragma unroll
           for (int b = 0; b < 3; ++b) t[a * 3 + b] = v[a] * cur.r[u][b];
-        scatter9(atom_virial + ((size_t)f * nall + j) * 9, t);
+        scatter9(atom_virial + ((size_t)f * nall + j) * (F4 ? 12 : 9), t);
 #pragma unroll
         for (int q = 0; q < 9; ++q) vs[q] += t[q];
       }
@@ -273,6 +254,73 @@ __global__ void __launch_bounds__(kScatterWarps * 32) k_scatter_atomic(
   }
 }
 
+// The virial alone has no per-centre sum, so its pairs are taken flat: each
+// CTA a span of one frame's pairs, a thread every 256th of them.  The call is
+// bound by its loads (80 B a pair in FP32): 136 MB for 12,288 centres, 20 us
+// at 6.7 TB/s.  k_scatter_atomic's warps walk rows of 138 slots in chunks of
+// 64, the third chunk nearly empty and each waiting for the one before: the
+// call took 65 us there (59 with padded rows, the same with the reductions
+// left out), 42 us here; 122,880 centres: 250 us, 5.4 TB/s.  Two pairs a
+// thread in flight: 47; 32 or 48 warps an SM instead of 40: 45, 43.
+// Per-lane partials of the frame virial in T over at most kVirSpan pairs, a
+// warp sum in T, then doubles.
+constexpr int kVirThreads = 256;
+constexpr int kVirSpan = 16;  // pairs per thread, at most
+
+template <typename T>
+constexpr int kVirCtas = sizeof(T) == 4 ? 5 : 4;  // resident CTAs an SM
+
+template <typename T, bool F4>
+__global__ void __launch_bounds__(kVirThreads, kVirCtas<T>) k_virial_pairs(
+    T* __restrict__ atom_virial, double* __restrict__ vir_acc, const T* __restrict__ net,
+    const T* __restrict__ dR, const T* __restrict__ rij, const int* __restrict__ nlist, int nloc,
+    int nall, int nnei, int cpf, int span) {
+  __shared__ double s_v[kVirThreads / 32][9];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int f = blockIdx.x / cpf;
+  const size_t pairs = (size_t)nloc * nnei;
+  const size_t p0 = (size_t)(blockIdx.x - f * cpf) * span;
+  const int n = (int)min((size_t)span, pairs - p0);
+  T vs[9];
+#pragma unroll
+  for (int q = 0; q < 9; ++q) vs[q] = T(0);
+  for (int k = tid; k < n; k += kVirThreads) {
+    const size_t rs = (size_t)f * pairs + p0 + k;
+    const int j = __ldg(nlist + rs);
+    T g[4], d[12], r[3];
+    V4<T>::load4(net + rs * 4, g);
+    V4<T>::load4(dR + rs * 12, d);
+    V4<T>::load4(dR + rs * 12 + 4, d + 4);
+    V4<T>::load4(dR + rs * 12 + 8, d + 8);
+#pragma unroll
+    for (int b = 0; b < 3; ++b) r[b] = __ldg(rij + rs * 3 + b);
+    if (j < 0 || j >= nall) continue;
+    T t[9];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      const T v = g[0] * d[a] + g[1] * d[3 + a] + g[2] * d[6 + a] + g[3] * d[9 + a];
+#pragma unroll
+      for (int b = 0; b < 3; ++b) {
+        t[a * 3 + b] = v * r[b];
+        vs[a * 3 + b] += t[a * 3 + b];
+      }
+    }
+    scatter9(atom_virial + ((size_t)f * nall + j) * (F4 ? 12 : 9), t);
+  }
+#pragma unroll
+  for (int q = 0; q < 9; ++q) {
+    const T s = warp_sum(vs[q]);
+    if (lane == 0) s_v[warp][q] = (double)s;
+  }
+  __syncthreads();
+  if (tid < 9) {
+    double s = 0.;
+#pragma unroll
+    for (int w = 0; w < kVirThreads / 32; ++w) s += s_v[w][tid];
+    atomicAdd(vir_acc + (size_t)f * 9 + tid, s);
+  }
+}
+
 // padded FP32 force rows [n][4] -> the output's [n][3]
 __global__ void k_force4_compact(float* __restrict__ force, const float4* __restrict__ f4,
                                  size_t n) {
@@ -282,6 +330,17 @@ __global__ void k_force4_compact(float* __restrict__ force, const float4* __rest
   force[3 * t] = v.x;
   force[3 * t + 1] = v.y;
   force[3 * t + 2] = v.z;
+}
+
+// padded FP32 atomic virial rows [n][12] -> the output's [n][9], and the
+// frame virials (n9 = 9 nframes values; vir may be null)
+__global__ void k_vir12_compact(float* __restrict__ av, const float* __restrict__ v12, size_t n,
+                                float* __restrict__ vir, const double* __restrict__ acc, int n9) {
+  const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (vir && t < (size_t)n9) vir[t] = (float)acc[t];
+  if (t >= 9 * n) return;
+  const size_t r = t / 9;
+  av[t] = v12[t + 3 * r];
 }
 
 template <typename T>
@@ -577,6 +636,7 @@ size_t a256(size_t x) { return (x + 255) & ~(size_t)255; }
 struct ProdWs {
   double* vir_acc;
   float4* force4;    // atomic mode, FP32: padded force rows [nframes * nall]
+  float* vir12;      // atomic mode, FP32: padded atomic virial rows [nframes * nall][12]
   double* vir_part;  // deterministic frame-virial partials [nframes, nchunk, 9]
   int* cnt;
   int* start;
@@ -597,7 +657,11 @@ ProdWs carve_prod(void* base, int nframes, int nloc, int nall, int nnei, int det
     return r;
   };
   w.vir_acc = reinterpret_cast<double*>(take(sizeof(double) * 9 * (size_t)nframes));
-  if (!det) w.force4 = reinterpret_cast<float4*>(take(sizeof(float4) * (size_t)nframes * nall));
+  if (!det) {
+    // (directly after vir_acc: one clear for both)
+    w.vir12 = reinterpret_cast<float*>(take(sizeof(float) * 12 * (size_t)nframes * nall));
+    w.force4 = reinterpret_cast<float4*>(take(sizeof(float4) * (size_t)nframes * nall));
+  }
   if (det) {
     const size_t nchunk = (size_t)(nall + kVirChunk - 1) / kVirChunk;
     w.vir_part = reinterpret_cast<double*>(take(sizeof(double) * 9 * (size_t)nframes * nchunk));
@@ -653,29 +717,62 @@ unsigned scatter_grid(size_t rows) {
   return (unsigned)std::max<size_t>(1, std::min<size_t>((size_t)cap, need));
 }
 
+// The atomic mode's launches.  FP32: forces and atomic virials accumulate in
+// the padded rows of the workspace, then are compacted into the outputs;
+// FP64: in the outputs themselves.
 template <typename T>
-void launch_atomic(T* force, float4* force4, T* atom_virial, double* vir_acc, const T* net,
-                   const T* dR, const T* rij, const int* nlist, int nloc, int nall, int nnei,
-                   int nframes, cudaStream_t st) {
-  const size_t rows = (size_t)nframes * nloc;
-  // FP32: forces accumulate in the padded rows of the workspace (zeroed by
-  // the caller), then compacted into the output
+void launch_atomic(T* force, T* virial, T* atom_virial, const ProdWs& w, const T* net, const T* dR,
+                   const T* rij, const int* nlist, int nloc, int nall, int nnei, int nframes,
+                   cudaStream_t st) {
+  const size_t rows = (size_t)nframes * nloc, n = (size_t)nframes * nall;
+  const int n9 = 9 * nframes;
   constexpr bool F4 = sizeof(T) == 4;
-  T* fdst = F4 && force ? reinterpret_cast<T*>(force4) : force;
-  if (atom_virial)
+  T *fdst = force, *vdst = atom_virial;
+  if constexpr (F4) {
+    if (force) {
+      fdst = reinterpret_cast<T*>(w.force4);
+      cudaMemsetAsync(fdst, 0, sizeof(float4) * n, st);
+    }
+    if (atom_virial) {
+      vdst = w.vir12;
+      cudaMemsetAsync(w.vir_acc, 0,
+                      (size_t)((char*)(w.vir12 + 12 * n) - (char*)w.vir_acc), st);
+    }
+  } else {
+    if (force) cudaMemsetAsync(force, 0, sizeof(T) * 3 * n, st);
+    if (atom_virial) {
+      cudaMemsetAsync(w.vir_acc, 0, sizeof(double) * n9, st);
+      cudaMemsetAsync(atom_virial, 0, sizeof(T) * 9 * n, st);
+    }
+  }
+  if (atom_virial && !force) {
+    // one wave of resident CTAs where that keeps a thread within kVirSpan
+    // pairs (a thread's chain is shortest then: 42 us for 12,288 centres, 57
+    // with many short CTAs), several waves above
+    const size_t pairs = (size_t)nloc * nnei, total = pairs * nframes;
+    const size_t wave = 152 * (size_t)kVirCtas<T> * kVirThreads;
+    const int span = kVirThreads * (int)std::min<size_t>((total + wave - 1) / wave, kVirSpan);
+    const size_t cpf = (pairs + span - 1) / span;
+    k_virial_pairs<T, F4><<<(unsigned)(cpf * nframes), kVirThreads, 0, st>>>(
+        vdst, w.vir_acc, net, dR, rij, nlist, nloc, nall, nnei, (int)cpf, span);
+  } else if (atom_virial)
     k_scatter_atomic<T, ScatterU<T>::U, true, F4><<<scatter_grid<T, true>(rows),
                                                     kScatterWarps * 32, 0, st>>>(
-        fdst, atom_virial, vir_acc, net, dR, rij, nlist, nloc, nall, nnei, nframes);
+        fdst, vdst, w.vir_acc, net, dR, rij, nlist, nloc, nall, nnei, nframes);
   else
     k_scatter_atomic<T, ScatterU<T>::U, false, F4><<<scatter_grid<T, false>(rows),
                                                      kScatterWarps * 32, 0, st>>>(
         fdst, nullptr, nullptr, net, dR, rij, nlist, nloc, nall, nnei, nframes);
   if constexpr (F4) {
-    if (force) {
-      const size_t n = (size_t)nframes * nall;
+    if (force)
       k_force4_compact<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(
-          reinterpret_cast<float*>(force), force4, n);
-    }
+          reinterpret_cast<float*>(force), w.force4, n);
+    if (atom_virial)
+      k_vir12_compact<<<(unsigned)((std::max<size_t>(9 * n, n9) + 255) / 256), 256, 0, st>>>(
+          atom_virial, w.vir12, n, virial, w.vir_acc, n9);
+  } else {
+    if (virial)
+      k_vir_finish<T><<<(unsigned)((n9 + 255) / 256), 256, 0, st>>>(virial, w.vir_acc, n9);
   }
 }
 
@@ -706,12 +803,13 @@ int prod_launch(T* force, T* virial, T* atom_virial, const T* net, const T* dR, 
   ProdWs w = carve_prod(ws, nframes, nloc, nall, nnei, det);
   GBDP_REQUIRE(ws != nullptr || w.bytes == 0, "prod_force/virial: null workspace");
   GBDP_REQUIRE(ws_bytes >= w.bytes, "prod_force/virial: workspace %zu < %zu", ws_bytes, w.bytes);
-  // the FP32 atomic mode writes every force word from its padded rows
-  const bool f4 = !det && sizeof(T) == 4 && force;
+  // the atomic mode clears what it adds into, the FP32 form writing every
+  // word of the outputs from its padded rows
   const bool empty = nframes == 0 || nloc == 0 || nnei == 0;
-  if (force && (!f4 || empty))
-    cudaMemsetAsync(force, 0, sizeof(T) * (size_t)nframes * nall * 3, st);
-  if (atom_virial) cudaMemsetAsync(atom_virial, 0, sizeof(T) * (size_t)nframes * nall * 9, st);
+  if (det || empty) {
+    if (force) cudaMemsetAsync(force, 0, sizeof(T) * (size_t)nframes * nall * 3, st);
+    if (atom_virial) cudaMemsetAsync(atom_virial, 0, sizeof(T) * (size_t)nframes * nall * 9, st);
+  }
   if (empty) {
     if (virial) cudaMemsetAsync(virial, 0, sizeof(T) * (size_t)nframes * 9, st);
     GBDP_CHECK_LAUNCH("prod_force/virial");
@@ -721,16 +819,10 @@ int prod_launch(T* force, T* virial, T* atom_virial, const T* net, const T* dR, 
                "prod_force/virial: null input pointer");
   GBDP_REQUIRE(((uintptr_t)net & 15) == 0 && ((uintptr_t)dR & 15) == 0,
                "prod_force/virial: net_deriv and env_deriv must be 16-byte aligned");
-  // every word of `virial` is written below (k_vir_finish, or the fixed-order
-  // reduction), so it needs no zero fill; the double accumulators of the
-  // atomic mode only where a virial is asked for
+  // every word of `virial` is written below, so it needs no zero fill
   if (!det) {
-    if (atom_virial) cudaMemsetAsync(w.vir_acc, 0, sizeof(double) * 9 * nframes, st);
-    if (f4) cudaMemsetAsync(w.force4, 0, sizeof(float4) * (size_t)nframes * nall, st);
-    launch_atomic<T>(force, w.force4, atom_virial, w.vir_acc, net, dR, rij, nlist, nloc, nall,
-                     nnei, nframes, st);
-    if (virial) k_vir_finish<T><<<(unsigned)((9 * nframes + 255) / 256), 256, 0, st>>>(
-        virial, w.vir_acc, 9 * nframes);
+    launch_atomic<T>(force, virial, atom_virial, w, net, dR, rij, nlist, nloc, nall, nnei, nframes,
+                     st);
   } else {
     int rc = build_reverse(w, nlist, nloc, nall, nnei, nframes, st);
     if (rc) return rc;
@@ -764,8 +856,9 @@ int prod_virial_impl(T* virial, T* atom_virial, const T* net, const T* dR, const
   ProdWs w = carve_prod(ws, nframes, nloc, nall, nnei, det);
   GBDP_REQUIRE(ws != nullptr, "prod_virial_a: null workspace");
   GBDP_REQUIRE(ws_bytes >= w.bytes, "prod_virial_a: workspace %zu < %zu", ws_bytes, w.bytes);
-  cudaMemsetAsync(atom_virial, 0, sizeof(T) * (size_t)nframes * nall * 9, st);
-  if (nframes == 0 || nloc == 0 || nnei == 0) {
+  const bool empty = nframes == 0 || nloc == 0 || nnei == 0;
+  if (det || empty) cudaMemsetAsync(atom_virial, 0, sizeof(T) * (size_t)nframes * nall * 9, st);
+  if (empty) {
     cudaMemsetAsync(virial, 0, sizeof(T) * (size_t)nframes * 9, st);
     GBDP_CHECK_LAUNCH("prod_virial_a");
     return GBDP_OK;
@@ -774,11 +867,8 @@ int prod_virial_impl(T* virial, T* atom_virial, const T* net, const T* dR, const
   GBDP_REQUIRE(((uintptr_t)net & 15) == 0 && ((uintptr_t)dR & 15) == 0,
                "prod_virial_a: net_deriv and env_deriv must be 16-byte aligned");
   if (!det) {
-    cudaMemsetAsync(w.vir_acc, 0, sizeof(double) * 9 * nframes, st);
-    launch_atomic<T>(nullptr, nullptr, atom_virial, w.vir_acc, net, dR, rij, nlist, nloc, nall,
-                     nnei, nframes, st);
-    k_vir_finish<T><<<(unsigned)((9 * nframes + 255) / 256), 256, 0, st>>>(virial, w.vir_acc,
-                                                                             9 * nframes);
+    launch_atomic<T>(nullptr, virial, atom_virial, w, net, dR, rij, nlist, nloc, nall, nnei,
+                     nframes, st);
   } else {
     int rc = build_reverse(w, nlist, nloc, nall, nnei, nframes, st);
     if (rc) return rc;

@@ -198,3 +198,38 @@ def test_many_frames_force_fp32(gb, oracle):
     for k in range(nf):
         fo = oracle.prod_force_a(nets[k], emd, nl, nloc, nloc, nnei)
         np.testing.assert_allclose(f[k].cpu().numpy(), np.reshape(fo, -1), atol=2e-3, rtol=1e-4)
+
+
+@pytest.mark.parametrize("dtype", [torch.float64, torch.float32])
+@pytest.mark.parametrize("nf,nloc,nall,nnei", [
+    (1, 1, 1, 1), (3, 1, 4, 255), (2, 1, 3, 256), (5, 1, 2, 257), (7, 37, 50, 138),
+    (1, 1130, 1131, 138), (1, 1500, 1500, 138), (2, 25000, 25011, 130)])
+def test_virial_pairs_vs_fp64(gb, dtype, nf, nloc, nall, nnei):
+    """The flat virial at the edges of a CTA's span and of one wave (a frame
+    of one pair; 255 to 257; a wave of one pair a thread, two, and several
+    waves), with ghosts and padding.  Bounds: m additions of an atom's row
+    and eight roundings of a term, (m + 8) u of the sum of magnitudes; the
+    frame's, 16 additions a thread, five of the warp, eight of a term and the
+    result's, 32 u."""
+    ops = __import__("dpmd_public_gb300.ops", fromlist=["x"])
+    g = torch.Generator(device=DEV).manual_seed(nf * nloc + nnei)
+    R = lambda *s: torch.randn(*s, generator=g, device=DEV, dtype=dtype)
+    net, dr, rij = R(nf, nloc * nnei * 4), R(nf, nloc * nnei * 12), R(nf, nloc * nnei * 3)
+    nl = torch.randint(-1, nall, (nf, nloc * nnei), generator=g, device=DEV, dtype=torch.int32)
+    natoms = torch.tensor([nloc, nall, 0, 0], dtype=torch.int32)
+    v, av = ops.prod_virial_se_a_impl(net, dr, rij, nl, natoms, nnei, 0, False)
+    u = 2.0 ** (-24 if dtype == torch.float32 else -53)
+    for k in range(nf):
+        G, D, X = (q[k].double().view(-1, *s) for q, s in ((net, (4, 1)), (dr, (4, 3)), (rij, (1, 3))))
+        j = nl[k].long()
+        ok = (j >= 0).double().view(-1, 1)
+        term = ((G * D).sum(1)[:, :, None] * X).view(-1, 9) * ok
+        mag = ((G * D).abs().sum(1)[:, :, None] * X.abs()).view(-1, 9) * ok
+        z = lambda w: torch.zeros(nall, w, dtype=torch.float64, device=DEV)
+        row, rmag = (z(9).index_add_(0, j.clamp_min(0), q) for q in (term, mag))
+        m = z(1).index_add_(0, j.clamp_min(0), ok)
+        # (the 64-bit sums of this check round as well: twice the bound in FP64)
+        w = 2.0 if dtype == torch.float64 else 1.0
+        assert bool(((av[k].double().view(nall, 9) - row).abs() <= w * (m + 8) * u * rmag).all())
+        chain = 32 if dtype == torch.float32 else 64 + int(ok.sum().item()) ** 0.5
+        assert bool(((v[k].double() - term.sum(0)).abs() <= w * chain * u * mag.sum(0)).all())
