@@ -7,6 +7,7 @@
 
 #include <cstdio>
 #include <string>
+#include <utility>
 
 #include "../../include/gbdp.h"
 
@@ -34,6 +35,58 @@ int cuda_status(cudaError_t e, const char* where);
       return GBDP_ERR_INVALID;                 \
     }                                          \
   } while (0)
+
+// ----------------------------------------------------- dependent launches --
+// A chain of short kernels is bound by the hand-over from one to the next.
+// launch_dep launches with programmatic stream serialization: the kernel's
+// CTAs may start once every CTA of the kernel before it on the stream has
+// called grid_release (or ended), and its grid_wait returns when all earlier
+// work is complete and visible.  A kernel launched so calls grid_wait before
+// its first access to global memory and grid_release after it (a later
+// kernel that reads constant data ahead of its own wait may then rely on
+// everything before this kernel).  Any other predecessor on the stream, and
+// any other successor, is ordered as usual.  A step on 192 atoms from host
+// to host, 18 kernels and 6 memsets: 204 us; so launched, clears in the chain
+// and the short kernels at its end merged: 183.  12,288 atoms captured in a
+// graph: 487 and 476.
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_release() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+template <typename... P, typename... A>
+cudaError_t launch_dep(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
+                       A&&... args) {
+  cudaLaunchConfig_t lc = {};
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  lc.attrs = attr;
+  lc.numAttrs = 1;
+  lc.gridDim = grid;
+  lc.blockDim = block;
+  lc.dynamicSmemBytes = smem;
+  lc.stream = st;
+  return cudaLaunchKernelEx(&lc, kern, std::forward<A>(args)...);
+}
+
+// a[0, na) = b[0, nb) = 0
+template <typename T>
+__global__ void k_clear2(T* __restrict__ a, size_t na, T* __restrict__ b, size_t nb) {
+  grid_wait();
+  grid_release();
+  const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t < na) a[t] = T(0);
+  if (t < nb) b[t] = T(0);
+}
+
+// Clears by a kernel in the chain (a memset is not part of one).
+template <typename T>
+cudaError_t clear_dep(T* a, size_t na, T* b, size_t nb, cudaStream_t st) {
+  const size_t n = na > nb ? na : nb;
+  if (n == 0) return cudaSuccess;
+  return launch_dep(k_clear2<T>, dim3((unsigned)((n + 255) / 256)), dim3(256), 0, st, a, na, b, nb);
+}
 
 // ------------------------------------------------------------ warp helpers --
 template <typename T>

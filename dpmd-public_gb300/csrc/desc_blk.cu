@@ -104,6 +104,8 @@ __global__ void __launch_bounds__(W * 32, 32 / W)
     k_fwd_blk(const __grid_constant__ DescFwdArgs p, const __grid_constant__ TabSet<float> ts,
               int nloc, int M) {
   extern __shared__ __align__(32) unsigned char smem_raw[];
+  grid_wait();
+  grid_release();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int i = S == 1 ? blockIdx.x * W + warp : blockIdx.x;
   if (i >= nloc) return;  // S = 1: uniform over the warp; S > 1: the grid is exact
@@ -400,6 +402,8 @@ __global__ void __launch_bounds__(W * 32, bwd_warps(U) / W)
     k_bwd_blk(const __grid_constant__ DescBwdArgs p, const __grid_constant__ TabSet<float> ts,
               int nloc, int M, float inv_rw, int pf_dist) {
   extern __shared__ __align__(32) unsigned char smem_raw[];
+  grid_wait();
+  grid_release();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int i = S == 1 ? blockIdx.x * W + warp : blockIdx.x;
   if (i >= nloc) return;  // S = 1: uniform over the warp; S > 1: the grid is exact
@@ -731,7 +735,8 @@ void launch_fwd(const DescFwdArgs& a, const TabSet<float>& ts, int nloc, int M, 
   const int nnei = ts.sec[ts.ntypes];
   const size_t smem = (S == 1 ? W : 1) * fwd_bytes<S>(nnei, M);
   set_smem(kern, smem, 32 / W);
-  kern<<<(unsigned)(S == 1 ? (nloc + W - 1) / W : nloc), W * 32, smem, st>>>(a, ts, nloc, M);
+  launch_dep(kern, dim3((unsigned)(S == 1 ? (nloc + W - 1) / W : nloc)), dim3(W * 32), smem, st, a,
+             ts, nloc, M);
 }
 
 template <int NS>
@@ -767,8 +772,8 @@ void launch_bwd(const DescBwdArgs& a, const TabSet<float>& ts, int nloc, int M, 
     c_smem = smem;
     c_pf = sms * ctas * W;
   }
-  kern<<<(unsigned)(S == 1 ? (nloc + W - 1) / W : nloc), W * 32, smem, st>>>(
-      a, ts, nloc, M, 1.f / (a.rmax - a.rmin), c_pf);
+  launch_dep(kern, dim3((unsigned)(S == 1 ? (nloc + W - 1) / W : nloc)), dim3(W * 32), smem, st, a,
+             ts, nloc, M, 1.f / (a.rmax - a.rmin), c_pf);
 }
 
 template <int NK, int U>

@@ -134,6 +134,8 @@ __global__ void k_localize(const gbdp_nbr_frame* __restrict__ fr, int nframes, i
                            int* __restrict__ ext_map, int* __restrict__ atom_frame,
                            int* __restrict__ atom_cell, int* __restrict__ cell_count,
                            int* __restrict__ sub_count, int* __restrict__ atom_sub) {
+  grid_wait();
+  grid_release();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= nloc_total) return;
   const int f = find_frame_atom(fr, nframes, i);
@@ -244,6 +246,8 @@ __global__ void k_cell_scan(const gbdp_nbr_frame* __restrict__ fr,
                             int* __restrict__ status, const int* __restrict__ sub_count,
                             int* __restrict__ ext_sub) {
   __shared__ int warp_tot[32];
+  grid_wait();
+  grid_release();
   const gbdp_nbr_frame& g = fr[blockIdx.x];
   const int ncl = g.ncell[0] * g.ncell[1] * g.ncell[2];
   int carry = 0;
@@ -303,6 +307,8 @@ __global__ void k_cell_bucket(int nloc_total, const gbdp_nbr_frame* __restrict__
                               const int* __restrict__ atom_cell,
                               const int* __restrict__ cell_start, int* __restrict__ cell_fill,
                               int* __restrict__ bucket) {
+  grid_wait();
+  grid_release();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= nloc_total) return;
   const int c = atom_cell[i];
@@ -320,6 +326,8 @@ __global__ void k_cell_rank(int nloc_total, const gbdp_nbr_frame* __restrict__ f
                             const int* __restrict__ cell_count, const int* __restrict__ bucket,
                             int* __restrict__ cell_atoms, const int* __restrict__ atom_sub,
                             int* __restrict__ atom_xpos) {
+  grid_wait();
+  grid_release();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= nloc_total) return;
   const int c = atom_cell[i];
@@ -352,6 +360,8 @@ __global__ void k_ghost_fill(const gbdp_nbr_frame* __restrict__ fr, int nframes,
                              int* __restrict__ ext_type, int* __restrict__ ext_map,
                              typename XsOf<T>::type* __restrict__ xs,
                              const int* __restrict__ atom_xpos) {
+  grid_wait();
+  grid_release();
   const int ew = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (ew >= next_cell_total) return;
@@ -719,6 +729,8 @@ __global__ void __launch_bounds__(kEnvWarps * 32)
                 T* __restrict__ rij, int* __restrict__ nlist, int* __restrict__ nlist_ext,
                 int* __restrict__ status, VList vl) {
   extern __shared__ __align__(16) unsigned char smem[];
+  grid_wait();
+  grid_release();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int i = blockIdx.x * kEnvWarps + warp;
   if (i >= nloc_total) return;
@@ -1033,6 +1045,8 @@ __global__ void __launch_bounds__(kEnvWarps * 32)
                     T rmin, T rmax, T* __restrict__ em, T* __restrict__ em_deriv,
                     T* __restrict__ rij, int* __restrict__ nlist, int* __restrict__ status) {
   extern __shared__ __align__(16) unsigned char smem[];
+  grid_wait();
+  grid_release();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int i = blockIdx.x * kEnvWarps + warp;
   if (i >= nwork) return;
@@ -1264,25 +1278,25 @@ void env_ghosts(const EnvWs& w, T* ext_coord, int* ext_type, int* ext_map, int* 
                 const T* coord, const int* atype, const gbdp_nbr_plan* plan,
                 const gbdp_nbr_frame* frames, cudaStream_t stream) {
   const int nl = plan->nloc_total;
-  cudaMemsetAsync(w.status, 0, w.zero_bytes, stream);
   const int tb = 256;
-  k_localize<T><<<(nl + tb - 1) / tb, tb, 0, stream>>>(frames, plan->nframes, nl, coord, atype,
-                                                       ext_coord, ext_type, ext_map,
-                                                       w.atom_frame, w.atom_cell, w.cell_count,
-                                                       w.sub_count, w.atom_sub);
-  k_cell_scan<<<plan->nframes, 1024, 0, stream>>>(frames, w.cell_count, w.cell_start,
-                                                  w.ext_start, w.ext_cnt, w.ghost_start,
-                                                  ext_nall, w.status, w.sub_count, w.ext_sub);
-  k_cell_bucket<<<(nl + tb - 1) / tb, tb, 0, stream>>>(nl, frames, w.atom_frame, w.atom_cell,
-                                                       w.cell_start, w.cell_fill, w.bucket);
-  k_cell_rank<<<(nl + tb - 1) / tb, tb, 0, stream>>>(nl, frames, w.atom_frame, w.atom_cell,
-                                                     w.cell_start, w.cell_count, w.bucket,
-                                                     w.cell_atoms, w.atom_sub, w.atom_xpos);
+  const dim3 ga((nl + tb - 1) / tb);
+  // (zero_bytes: whole 256-byte pieces)
+  clear_dep<int>(reinterpret_cast<int*>(w.status), w.zero_bytes / 4, nullptr, 0, stream);
+  launch_dep(k_localize<T>, ga, dim3(tb), 0, stream, frames, plan->nframes, nl, coord, atype,
+             ext_coord, ext_type, ext_map, w.atom_frame, w.atom_cell, w.cell_count, w.sub_count,
+             w.atom_sub);
+  launch_dep(k_cell_scan, dim3(plan->nframes), dim3(1024), 0, stream, frames, w.cell_count,
+             w.cell_start, w.ext_start, w.ext_cnt, w.ghost_start, ext_nall, w.status, w.sub_count,
+             w.ext_sub);
+  launch_dep(k_cell_bucket, ga, dim3(tb), 0, stream, nl, frames, w.atom_frame, w.atom_cell,
+             w.cell_start, w.cell_fill, w.bucket);
+  launch_dep(k_cell_rank, ga, dim3(tb), 0, stream, nl, frames, w.atom_frame, w.atom_cell,
+             w.cell_start, w.cell_count, w.bucket, w.cell_atoms, w.atom_sub, w.atom_xpos);
   const int nec = plan->next_cell_total;
-  k_ghost_fill<T><<<(nec * 32 + tb - 1) / tb, tb, 0, stream>>>(
-      frames, plan->nframes, nec, w.cell_start, w.cell_count, w.cell_atoms, w.ext_start,
-      w.ghost_start, ext_coord, ext_type, ext_map,
-      static_cast<typename XsOf<T>::type*>(w.xs), w.atom_xpos);
+  launch_dep(k_ghost_fill<T>, dim3((nec * 32 + tb - 1) / tb), dim3(tb), 0, stream, frames,
+             plan->nframes, nec, w.cell_start, w.cell_count, w.cell_atoms, w.ext_start,
+             w.ghost_start, ext_coord, ext_type, ext_map,
+             static_cast<typename XsOf<T>::type*>(w.xs), w.atom_xpos);
 }
 
 // One launch of k_nlist_env in the given mode (candidates within rc).
@@ -1299,12 +1313,12 @@ void nlist_env_mode(const EnvWs& w, const gbdp_nbr_plan* plan, const gbdp_nbr_fr
   if (smem > 48 * 1024)
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   const bool cells = MODE != kEnvList;
-  kern<<<(nl + kEnvWarps - 1) / kEnvWarps, kEnvWarps * 32, smem, stream>>>(
-      nl, frames, w.atom_frame, cells ? w.atom_cell : nullptr, cells ? w.atom_sub : nullptr,
-      cells ? w.ext_sub : nullptr,
-      cells ? static_cast<const typename XsOf<T>::type*>(w.xs) : nullptr, ext_coord, ext_map,
-      atype, avg, stdv, si, rc * rc, (T)rcut_smth, (T)rmax, mc, em, em_deriv, rij, nlist,
-      nlist_ext, w.status, vl);
+  launch_dep(kern, dim3((nl + kEnvWarps - 1) / kEnvWarps), dim3(kEnvWarps * 32), smem, stream, nl,
+             frames, w.atom_frame, cells ? w.atom_cell : nullptr, cells ? w.atom_sub : nullptr,
+             cells ? w.ext_sub : nullptr,
+             cells ? static_cast<const typename XsOf<T>::type*>(w.xs) : nullptr, ext_coord,
+             ext_map, atype, avg, stdv, si, rc * rc, (T)rcut_smth, (T)rmax, mc, em, em_deriv, rij,
+             nlist, nlist_ext, w.status, vl);
 }
 
 template <typename T>
@@ -1453,7 +1467,7 @@ int env_nlist_launch(T* em, T* em_deriv, T* rij, int* nlist, int* status, const 
                "prod_env_mat_a_nlist: null required pointer");
   GBDP_REQUIRE(((uintptr_t)em & 15) == 0 && (!em_deriv || ((uintptr_t)em_deriv & 15) == 0),
                "prod_env_mat_a_nlist: em / em_deriv must be 16-byte aligned");
-  if (status) cudaMemsetAsync(status, 0, sizeof(int), stream);
+  if (status) clear_dep<int>(status, 1, nullptr, 0, stream);
   const int cap = (nnei_in + 7) & ~7;
   const size_t per_warp = (size_t)cap * sizeof(T) + (size_t)((si.nnei + 3) & ~3) * 4 + 2 * (size_t)cap;
   GBDP_REQUIRE((size_t)kEnvWarps * ((per_warp + 15) & ~(size_t)15) <= 200 * 1024,
@@ -1463,9 +1477,9 @@ int env_nlist_launch(T* em, T* em_deriv, T* rij, int* nlist, int* status, const 
   auto kern = k_nlist_env_ext<T>;
   if (smem > 48 * 1024)
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  kern<<<(unsigned)((nwork + kEnvWarps - 1) / kEnvWarps), kEnvWarps * 32, smem, stream>>>(
-      nloc, nall, nnei_in, (int)nwork, ext_coord, ext_type, nlist_in, avg, stdv, si, (T)rcut,
-      (T)rcut_smth, (T)rcut, em, em_deriv, rij, nlist, status);
+  launch_dep(kern, dim3((unsigned)((nwork + kEnvWarps - 1) / kEnvWarps)), dim3(kEnvWarps * 32),
+             smem, stream, nloc, nall, nnei_in, (int)nwork, ext_coord, ext_type, nlist_in, avg,
+             stdv, si, (T)rcut, (T)rcut_smth, (T)rcut, em, em_deriv, rij, nlist, status);
   GBDP_CHECK_LAUNCH("prod_env_mat_a_nlist");
   return GBDP_OK;
 }

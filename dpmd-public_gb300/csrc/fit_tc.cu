@@ -324,12 +324,6 @@ __device__ __forceinline__ void row_ld16(const float* chunk, int lane, float* v)
 
 // programmatic dependent launch: wait for the grid this one depends on (all
 // its writes visible); let the dependent grid be scheduled
-__device__ __forceinline__ void griddep_wait() {
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-}
-__device__ __forceinline__ void griddep_launch_dependents() {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-}
 
 // Per-warp epilogue progress, carried across the tiles a CTA processes:
 // chunks done (input and output staging buffers alternate by chunk) and
@@ -561,7 +555,7 @@ __global__ void __launch_bounds__(128, 1)
       tma_2d(st + 2 * A_TILE + B_TILE, &maps.b_lo[t], kb * TBK, n0, &full[kb]);
     }
     issued = pre;
-    griddep_wait();
+    grid_wait();
     for (int kb = 0; kb < nkb; ++kb) {
       const int s = kb % TSTAGES;
       const unsigned ph = (kb / TSTAGES) & 1u;
@@ -610,8 +604,8 @@ __global__ void __launch_bounds__(128, 1)
   tc_fence_after();
   // the next layer may start filling SMs as this grid's CTAs leave; this
   // thread's own reads of the previous layer's outputs come after its wait
-  griddep_launch_dependents();
-  griddep_wait();
+  grid_release();
+  grid_wait();
   float esum = 0.f;
   if (got) {
     static_assert(4 * EPI_WARP_BYTES <= TSTAGES * STAGE, "epilogue staging exceeds the stage buffers");
@@ -723,7 +717,7 @@ __global__ void __launch_bounds__(192, 1)
           tma_2d(st + 2 * A_TILE, &maps.b_hi[t], kb * TBK, n0, &full[kb]);
           tma_2d(st + 2 * A_TILE + B_TILE, &maps.b_lo[t], kb * TBK, n0, &full[kb]);
         }
-        griddep_wait();
+        grid_wait();
         for (int kb = 0; kb < pre; ++kb) {
           unsigned char* st = smem + kb * STAGE;
           tma_2d(st, &maps.a_hi, kb * TBK, row0, &full[kb]);
@@ -731,7 +725,7 @@ __global__ void __launch_bounds__(192, 1)
         }
         issued = pre;
       } else {
-        griddep_wait();
+        grid_wait();
       }
       int it = 0;
       for (int tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x, ++it) {
@@ -807,7 +801,7 @@ __global__ void __launch_bounds__(192, 1)
     }
   } else {
     // ---- epilogue warps: this warp's rows of each tile
-    griddep_wait();  // the previous layer's outputs visible to this thread
+    grid_wait();  // the previous layer's outputs visible to this thread
     const int ew = warp - 2, q = warp & 3;
     unsigned char* wsm = epi + ew * EPI_WARP_BYTES;
     uint64_t* ib = inbar + ew * 2;
@@ -820,7 +814,7 @@ __global__ void __launch_bounds__(192, 1)
       ++seen[j];
       tc_fence_after();
       // the next layer may start filling SMs once this CTA's last tile drains
-      if (tile + (int)gridDim.x >= ntiles) griddep_launch_dependents();
+      if (tile + (int)gridDim.x >= ntiles) grid_release();
       int row0, n0, nt, t;
       tile_at(tile, row0, n0, nt, t);
       const int yrow = row0 + q * 32;
@@ -917,7 +911,7 @@ __global__ void __launch_bounds__(320, 1)
       // ---- TMA producer: runs into the next tile's k-blocks as stages free up
       int issued = 0;
       bool ok = true;
-      griddep_wait();
+      grid_wait();
       for (int tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x) {
         int row0, n0, t;
         tile_at(tile, row0, n0, t);
@@ -981,7 +975,7 @@ __global__ void __launch_bounds__(320, 1)
     }
   } else {
     // ---- epilogue warps
-    griddep_wait();  // the row scales visible; earlier readers of T1 done
+    grid_wait();  // the row scales visible; earlier readers of T1 done
     const int q = warp & 3, half = (warp - 2) >> 2;
     constexpr int NCMAX = C::HALF / 16;
     int it = 0;
@@ -989,7 +983,7 @@ __global__ void __launch_bounds__(320, 1)
       if (!__all_sync(kFull, mbar_wait_bounded(tfull, (unsigned)it & 1u, ep.status))) break;
       tc_fence_after();
       // the next launch may start filling SMs once this CTA's last tile drains
-      if (tile + (int)gridDim.x >= ntiles) griddep_launch_dependents();
+      if (tile + (int)gridDim.x >= ntiles) grid_release();
       int row0, n0, t;
       tile_at(tile, row0, n0, t);
       const int r = q * 32 + lane, cl = half * C::HALF;
@@ -1118,7 +1112,7 @@ __global__ void __launch_bounds__(64 + B1_EPI_WARPS * 32, 1)
           ++issued;
           if (first) {  // the A tiles of the first stages follow the wait
             if (issued < S && kb + 1 < nkb) continue;
-            griddep_wait();
+            grid_wait();
             first = false;
             for (int k = 0; k < issued; ++k) {
               unsigned char* a = smem + k * STAGE;
@@ -1179,7 +1173,7 @@ __global__ void __launch_bounds__(64 + B1_EPI_WARPS * 32, 1)
   } else {
     // ---- epilogue warps (B1 reads nothing of the previous layers, but its
     //      output rows may still be read by launches before this one)
-    griddep_wait();
+    grid_wait();
     const int ew = warp - 2, q = warp & 3, half = ew >> 2;
     unsigned char* wsm = epi + ew * 2 * B1_CHUNK;
     int it = 0, nst = 0;
@@ -1189,7 +1183,7 @@ __global__ void __launch_bounds__(64 + B1_EPI_WARPS * 32, 1)
         break;
       tc_fence_after();
       // the next launch may start filling SMs once this CTA's last tile drains
-      if (tile + (int)gridDim.x >= ntiles) griddep_launch_dependents();
+      if (tile + (int)gridDim.x >= ntiles) grid_release();
       int row0, n0, t;
       tile_at(tile, row0, n0, t);
       const uint32_t tacc = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(j * 256 + half * 64);
@@ -1426,7 +1420,7 @@ __global__ void __launch_bounds__(64 + MID_WARPS * 32, 1)
     float4* g2 = p.g2p + (size_t)blockIdx.x * (FIT_W / 4) * TBM + r;
     unsigned accph = 0;
     bool ok = true;
-    griddep_wait();  // F1's T1 visible to this thread
+    grid_wait();  // F1's T1 visible to this thread
     for (int rb = blockIdx.x; rb < p.nblk && ok; rb += gridDim.x) {
       const int t = type_of(rb);
       const float4* t1 = p.t1p + (size_t)rb * (FIT_W / 4) * TBM + r;
@@ -1454,7 +1448,7 @@ __global__ void __launch_bounds__(64 + MID_WARPS * 32, 1)
         }
         accph ^= 1u;
         tc_fence_after();
-        if (l == 3 && rb + (int)gridDim.x >= p.nblk) griddep_launch_dependents();
+        if (l == 3 && rb + (int)gridDim.x >= p.nblk) grid_release();
         const float* cs = p.cs[t][l];
         const float osc = p.osc[t][l + 1];
 #pragma unroll 1
@@ -1547,6 +1541,8 @@ struct TcRows {
 
 __global__ void k_fit_tc_energy(float* __restrict__ e, const float* __restrict__ epart,
                                 int ntile_n, TcRows rw) {
+  grid_wait();
+  grid_release();
   const int r = blockIdx.x * blockDim.x + threadIdx.x;
   if (r >= rw.row_off[rw.ntypes]) return;
   int t = 0;
@@ -1768,7 +1764,9 @@ extern "C" int gbdp_fitting_tc_f32(float* e, float* dE_dD, const void* D_hi, con
   if (rc) return rc;
   int* status = reinterpret_cast<int*>(static_cast<char*>(workspace) + ws.bytes);
   cudaStream_t st = (cudaStream_t)stream;
-  cudaMemsetAsync(status, 0, sizeof(int) * 4, st);
+  // F1 reads weights ahead of its wait, which the clear's (before its
+  // release) covers
+  clear_dep<int>(status, 4, nullptr, 0, st);
   cudaFuncSetAttribute(k_fit_pers, cudaFuncAttributeMaxDynamicSharedMemorySize, PERS_SMEM);
   cudaFuncSetAttribute(k_fit_b1, cudaFuncAttributeMaxDynamicSharedMemorySize, B1_SMEM);
   // SM count of the device (initialised once, thread-safe)
@@ -1957,7 +1955,8 @@ extern "C" int gbdp_fitting_tc_f32(float* e, float* dE_dD, const void* D_hi, con
     rw.nrows[t] = nrows[t];
     rw.b_out[t] = nets[t].b_out;
   }
-  k_fit_tc_energy<<<(unsigned)((rows + 255) / 256), 256, 0, st>>>(e, ws.epart, base.ntile_n, rw);
+  launch_dep(k_fit_tc_energy, dim3((unsigned)((rows + 255) / 256)), dim3(256), 0, st, e, ws.epart,
+             base.ntile_n, rw);
   GBDP_CHECK_LAUNCH("fit_tc energy");
   return GBDP_OK;
 }

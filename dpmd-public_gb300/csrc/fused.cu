@@ -742,10 +742,21 @@ __global__ void k_fx_finish_inplace(double* __restrict__ buf, size_t n, int s) {
   }
 }
 
+// both after the FP32 backward in one launch of the chain
+__global__ void k_fx_finish2(float* __restrict__ out, const long long* __restrict__ acc, size_t n,
+                             int s, double* __restrict__ buf, size_t nb, int sb) {
+  grid_wait();
+  grid_release();
+  const size_t k = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (k < n) out[k] = (float)((double)acc[k] * pow2d(-s));
+  if (k < nb) buf[k] = (double)reinterpret_cast<const long long*>(buf)[k] * pow2d(-sb);
+}
+
+// one row a lane (r, of a warp's 32 in a row)
 template <typename T>
-__global__ void k_frame_energy(double* __restrict__ E, const T* __restrict__ ae,
-                               const int* __restrict__ frame_of_row, int nrows, int det) {
-  const int r = blockIdx.x * blockDim.x + threadIdx.x;
+__device__ __forceinline__ void add_rows(double* E, const T* __restrict__ ae,
+                                         const int* __restrict__ frame_of_row, int r, int nrows,
+                                         int det) {
   const int lane = threadIdx.x & 31;
   const int f = r < nrows ? frame_of_row[r] : -1;
   const double v = r < nrows ? (double)ae[r] : 0.;
@@ -767,13 +778,46 @@ __global__ void k_frame_energy(double* __restrict__ E, const T* __restrict__ ae,
 }
 
 template <typename T>
+__global__ void k_frame_energy(double* __restrict__ E, const T* __restrict__ ae,
+                               const int* __restrict__ frame_of_row, int nrows, int det) {
+  add_rows<T>(E, ae, frame_of_row, blockIdx.x * blockDim.x + threadIdx.x, nrows, det);
+}
+
+// Few rows: the clear, the sums and the read-back in one CTA, whose rows come
+// in passes of 1,024 (against three launches: 256 rows 7.1 and 9.2 us, 1,920
+// rows 9.2 and 11.2, 3,712 rows 15.3 and 11.2).
+constexpr int kEnergyRows = 2048, kEnergyThreads = 1024;
+
+template <typename T>
+__global__ void __launch_bounds__(kEnergyThreads) k_frame_energy_cta(
+    double* __restrict__ E, const T* __restrict__ ae, const int* __restrict__ frame_of_row,
+    int nrows, int nframes, int det) {
+  grid_wait();
+  grid_release();
+  for (int k = threadIdx.x; k < nframes; k += kEnergyThreads) E[k] = 0.;
+  __syncthreads();
+  for (int r0 = threadIdx.x & ~31; r0 < nrows; r0 += kEnergyThreads)
+    add_rows<T>(E, ae, frame_of_row, r0 + (threadIdx.x & 31), nrows, det);
+  if (!det) return;
+  __syncthreads();
+  for (int k = threadIdx.x; k < nframes; k += kEnergyThreads)
+    E[k] = (double)__ldcg(reinterpret_cast<const long long*>(E) + k) * pow2d(-kFxEnergy);
+}
+
+template <typename T>
 int frame_energy(double* E, const T* ae, const int* frame_of_row, int nrows, int nframes,
                  int det, cudaStream_t st) {
   GBDP_REQUIRE(nrows >= 0 && nframes >= 1, "frame_energy: nrows %d, nframes %d", nrows, nframes);
   GBDP_REQUIRE(E != nullptr, "frame_energy: null E");
+  GBDP_REQUIRE(nrows == 0 || (ae && frame_of_row), "frame_energy: null input");
+  if (nrows > 0 && nrows <= kEnergyRows) {
+    launch_dep(k_frame_energy_cta<T>, dim3(1), dim3(kEnergyThreads), 0, st, E, ae, frame_of_row,
+               nrows, nframes, det);
+    GBDP_CHECK_LAUNCH("frame_energy");
+    return GBDP_OK;
+  }
   cudaMemsetAsync(E, 0, sizeof(double) * (size_t)nframes, st);
   if (nrows == 0) return GBDP_OK;
-  GBDP_REQUIRE(ae && frame_of_row, "frame_energy: null input");
   k_frame_energy<T><<<(unsigned)((nrows + 255) / 256), 256, 0, st>>>(E, ae, frame_of_row, nrows,
                                                                      det);
   if (det) k_fx_finish_inplace<<<1, 256, 0, st>>>(E, (size_t)nframes, kFxEnergy);
@@ -1319,12 +1363,16 @@ extern "C" int gbdp_se_a_descriptor_bwd_blk_f32(
                       ext_coord, ext_map,  atype,    inv_std,
                       {atom_frame, frame_atom_off, frame_ext_off}, rcut_smth, rcut};
   return tune_run(kTuneBwd, 4, M, nnei, nloc, st, [&](int w) -> int {
-    cudaMemsetAsync(virial_acc, 0, sizeof(double) * 9 * (size_t)nframes, st);
-    if (!force_fx || nloc == 0)
-      cudaMemsetAsync(force, 0, sizeof(float) * 3 * (size_t)nloc, st);
+    const size_t nf = 3 * (size_t)nloc, nv = 9 * (size_t)nframes;
+    if (force_fx && nloc > 0)
+      clear_dep<long long>(force_fx, nf, reinterpret_cast<long long*>(virial_acc), nv, st);
     else
-      cudaMemsetAsync(force_fx, 0, sizeof(long long) * 3 * (size_t)nloc, st);
-    if (nloc == 0) return GBDP_OK;
+      clear_dep<int>(reinterpret_cast<int*>(force), nf, reinterpret_cast<int*>(virial_acc), 2 * nv,
+                     st);
+    if (nloc == 0) {
+      GBDP_CHECK_LAUNCH("se_a_descriptor_bwd");
+      return GBDP_OK;
+    }
     // untuned: two neighbours in flight while the SMs hold less than four
     // atoms each (192 atoms: 27.6 against 31.7 us; 768 atoms: 41.9 / 39.9)
     if (w == 0)
@@ -1332,11 +1380,9 @@ extern "C" int gbdp_se_a_descriptor_bwd_blk_f32(
     int rc = desc_bwd_blk(a, ts, nloc, M, code_warps(w), code_nbrs(w), st);
     if (rc) return rc;
     if (force_fx) {
-      const size_t nf = 3 * (size_t)nloc;
-      k_fx_finish<float><<<(unsigned)((nf + 255) / 256), 256, 0, st>>>(force, force_fx, nf,
-                                                                       FxScale<float>::force);
-      k_fx_finish_inplace<<<1, 256, 0, st>>>(virial_acc, 9 * (size_t)nframes,
-                                             FxScale<float>::virial);
+      launch_dep(k_fx_finish2, dim3((unsigned)((std::max(nf, nv) + 255) / 256)), dim3(256), 0, st,
+                 force, force_fx, nf, FxScale<float>::force, virial_acc, nv,
+                 FxScale<float>::virial);
     }
     GBDP_CHECK_LAUNCH("se_a_descriptor_bwd");
     return GBDP_OK;

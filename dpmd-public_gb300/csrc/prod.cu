@@ -152,6 +152,8 @@ __global__ void __launch_bounds__(kScatterWarps * 32) k_scatter_atomic(
     T* __restrict__ force, T* __restrict__ atom_virial, double* __restrict__ vir_acc,
     const T* __restrict__ net, const T* __restrict__ dR, const T* __restrict__ rij,
     const int* __restrict__ nlist, int nloc, int nall, int nnei, int nframes) {
+  grid_wait();
+  grid_release();
   __shared__ double s_vd[kScatterWarps][9];  // lane 0's double virial sums
   const int lane = threadIdx.x & 31;
   const long nw = (long)gridDim.x * kScatterWarps;
@@ -275,6 +277,8 @@ __global__ void __launch_bounds__(kVirThreads, kVirCtas<T>) k_virial_pairs(
     T* __restrict__ atom_virial, double* __restrict__ vir_acc, const T* __restrict__ net,
     const T* __restrict__ dR, const T* __restrict__ rij, const int* __restrict__ nlist, int nloc,
     int nall, int nnei, int cpf, int span) {
+  grid_wait();
+  grid_release();
   __shared__ double s_v[kVirThreads / 32][9];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int f = blockIdx.x / cpf;
@@ -324,6 +328,8 @@ __global__ void __launch_bounds__(kVirThreads, kVirCtas<T>) k_virial_pairs(
 // padded FP32 force rows [n][4] -> the output's [n][3]
 __global__ void k_force4_compact(float* __restrict__ force, const float4* __restrict__ f4,
                                  size_t n) {
+  grid_wait();
+  grid_release();
   const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= n) return;
   const float4 v = f4[t];
@@ -336,6 +342,8 @@ __global__ void k_force4_compact(float* __restrict__ force, const float4* __rest
 // frame virials (n9 = 9 nframes values; vir may be null)
 __global__ void k_vir12_compact(float* __restrict__ av, const float* __restrict__ v12, size_t n,
                                 float* __restrict__ vir, const double* __restrict__ acc, int n9) {
+  grid_wait();
+  grid_release();
   const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (vir && t < (size_t)n9) vir[t] = (float)acc[t];
   if (t >= 9 * n) return;
@@ -345,6 +353,8 @@ __global__ void k_vir12_compact(float* __restrict__ av, const float* __restrict_
 
 template <typename T>
 __global__ void k_vir_finish(T* __restrict__ virial, const double* __restrict__ acc, int n) {
+  grid_wait();
+  grid_release();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t < n) virial[t] = (T)acc[t];
 }
@@ -728,22 +738,16 @@ void launch_atomic(T* force, T* virial, T* atom_virial, const ProdWs& w, const T
   const int n9 = 9 * nframes;
   constexpr bool F4 = sizeof(T) == 4;
   T *fdst = force, *vdst = atom_virial;
+  // everything added into, cleared in one launch (FP64 with both: two)
   if constexpr (F4) {
-    if (force) {
-      fdst = reinterpret_cast<T*>(w.force4);
-      cudaMemsetAsync(fdst, 0, sizeof(float4) * n, st);
-    }
-    if (atom_virial) {
-      vdst = w.vir12;
-      cudaMemsetAsync(w.vir_acc, 0,
-                      (size_t)((char*)(w.vir12 + 12 * n) - (char*)w.vir_acc), st);
-    }
+    if (force) fdst = reinterpret_cast<T*>(w.force4);
+    if (atom_virial) vdst = w.vir12;
+    float* acc = reinterpret_cast<float*>(w.vir_acc);
+    clear_dep<float>(fdst, force ? 4 * n : 0, acc,
+                     atom_virial ? (size_t)(w.vir12 + 12 * n - acc) : 0, st);
   } else {
-    if (force) cudaMemsetAsync(force, 0, sizeof(T) * 3 * n, st);
-    if (atom_virial) {
-      cudaMemsetAsync(w.vir_acc, 0, sizeof(double) * n9, st);
-      cudaMemsetAsync(atom_virial, 0, sizeof(T) * 9 * n, st);
-    }
+    if (force) clear_dep<double>(force, 3 * n, nullptr, 0, st);
+    if (atom_virial) clear_dep<double>(atom_virial, 9 * n, w.vir_acc, n9, st);
   }
   if (atom_virial && !force) {
     // one wave of resident CTAs where that keeps a thread within kVirSpan
@@ -753,26 +757,27 @@ void launch_atomic(T* force, T* virial, T* atom_virial, const ProdWs& w, const T
     const size_t wave = 152 * (size_t)kVirCtas<T> * kVirThreads;
     const int span = kVirThreads * (int)std::min<size_t>((total + wave - 1) / wave, kVirSpan);
     const size_t cpf = (pairs + span - 1) / span;
-    k_virial_pairs<T, F4><<<(unsigned)(cpf * nframes), kVirThreads, 0, st>>>(
-        vdst, w.vir_acc, net, dR, rij, nlist, nloc, nall, nnei, (int)cpf, span);
+    launch_dep(k_virial_pairs<T, F4>, dim3((unsigned)(cpf * nframes)), dim3(kVirThreads), 0, st,
+               vdst, w.vir_acc, net, dR, rij, nlist, nloc, nall, nnei, (int)cpf, span);
   } else if (atom_virial)
-    k_scatter_atomic<T, ScatterU<T>::U, true, F4><<<scatter_grid<T, true>(rows),
-                                                    kScatterWarps * 32, 0, st>>>(
-        fdst, vdst, w.vir_acc, net, dR, rij, nlist, nloc, nall, nnei, nframes);
+    launch_dep(k_scatter_atomic<T, ScatterU<T>::U, true, F4>, dim3(scatter_grid<T, true>(rows)),
+               dim3(kScatterWarps * 32), 0, st, fdst, vdst, w.vir_acc, net, dR, rij, nlist, nloc,
+               nall, nnei, nframes);
   else
-    k_scatter_atomic<T, ScatterU<T>::U, false, F4><<<scatter_grid<T, false>(rows),
-                                                     kScatterWarps * 32, 0, st>>>(
-        fdst, nullptr, nullptr, net, dR, rij, nlist, nloc, nall, nnei, nframes);
+    launch_dep(k_scatter_atomic<T, ScatterU<T>::U, false, F4>, dim3(scatter_grid<T, false>(rows)),
+               dim3(kScatterWarps * 32), 0, st, fdst, nullptr, nullptr, net, dR, rij, nlist, nloc,
+               nall, nnei, nframes);
   if constexpr (F4) {
     if (force)
-      k_force4_compact<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(
-          reinterpret_cast<float*>(force), w.force4, n);
+      launch_dep(k_force4_compact, dim3((unsigned)((n + 255) / 256)), dim3(256), 0, st,
+                 reinterpret_cast<float*>(force), w.force4, n);
     if (atom_virial)
-      k_vir12_compact<<<(unsigned)((std::max<size_t>(9 * n, n9) + 255) / 256), 256, 0, st>>>(
-          atom_virial, w.vir12, n, virial, w.vir_acc, n9);
+      launch_dep(k_vir12_compact, dim3((unsigned)((std::max<size_t>(9 * n, n9) + 255) / 256)),
+                 dim3(256), 0, st, atom_virial, w.vir12, n, virial, w.vir_acc, n9);
   } else {
     if (virial)
-      k_vir_finish<T><<<(unsigned)((n9 + 255) / 256), 256, 0, st>>>(virial, w.vir_acc, n9);
+      launch_dep(k_vir_finish<T>, dim3((unsigned)((n9 + 255) / 256)), dim3(256), 0, st, virial,
+                 w.vir_acc, n9);
   }
 }
 
