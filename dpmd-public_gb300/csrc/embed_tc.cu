@@ -51,6 +51,7 @@ constexpr int kParW1 = 0, kParB1 = 64, kParB2 = 128, kParB3 = 192;
 
 constexpr int kRows = 128;
 constexpr int kSlot = 26624;   // one staged net, forward part (1024-aligned)
+constexpr size_t kFwdBytes = 2 * kSlot + 16384 + kRows * 16 + 64;  // the forward's shared memory
 constexpr int kMaxTypes = 8;
 
 struct EmbArgs {
@@ -230,8 +231,14 @@ struct Group {
 };
 __device__ __forceinline__ Group load_group(const int* __restrict__ units,
                                             const int* __restrict__ atype, int nunits, int g,
-                                            int warp, bool one_side) {
+                                            int warp, bool one_side, bool split = false) {
   Group r;
+  if (split) {  // warps 0 and 2: the unit's first atom, 1 and 3: its second
+    r.atom = units[2 * g + (warp & 1)];
+    r.ti[0] = r.ti[1] = atype[units[2 * g]];
+    r.both = true;
+    return r;
+  }
   const int u0 = 2 * g, u1 = u0 + 1;
   const int mine = u0 + (warp >> 1);
   r.atom = mine < nunits ? units[2 * mine + (warp & 1)] : -1;
@@ -289,10 +296,17 @@ __device__ __forceinline__ void epi3(uint32_t trow, const float* par, const floa
 // atoms: rows in ascending order in one chain of FMAs per column, broken
 // where (member of the unit) sel + row is a multiple of 128 (X feeds BF16
 // operands in the backward: another grouping would move their rounding).
-template <int N1, int N2, int N3>
+// SPLIT: one unit a CTA, for calls of up to a wave of units, whose time is the
+// chain of slabs: an atom's slabs go to two warps (0 and 2, 1 and 3), which
+// evaluate them side by side and then sum the rows of both in slab order,
+// one warp the even 32-column chunks, the other the odd ones (the same sums
+// bit for bit).
+template <int N1, int N2, int N3, bool SPLIT>
 __global__ void __launch_bounds__(128, 3) k_emb_fwd(const __grid_constant__ EmbArgs p) {
   static_assert(N1 <= 32 && N2 <= 64 && N3 <= 128 && N3 >= 1, "embedding widths");
   constexpr int NCH = (N3 + 31) / 32;  // 32-column chunks
+  grid_wait();
+  grid_release();
   extern __shared__ unsigned char smem_raw[];
   unsigned char* sm = reinterpret_cast<unsigned char*>(
       (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -303,6 +317,7 @@ __global__ void __launch_bounds__(128, 3) k_emb_fwd(const __grid_constant__ EmbA
   uint32_t* tslot = reinterpret_cast<uint32_t*>(bar + 1);
   int* cached = reinterpret_cast<int*>(tslot + 1);  // [2] net held by each slot
   int* nslab = cached + 2;                          // [4 warps] slabs of the section
+  float* odd = reinterpret_cast<float*>(sm + kFwdBytes);  // SPLIT: [4 warps] odd chunks
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int r = tid;  // this thread's tile row = TMEM lane
@@ -328,13 +343,21 @@ __global__ void __launch_bounds__(128, 3) k_emb_fwd(const __grid_constant__ EmbA
   unsigned phase = 0;
   bool alive = true;
   const float inv_nnei = 1.f / (float)p.nnei;
-  const int ngroups = (p.nunits + 1) >> 1;
+  const int ngroups = SPLIT ? p.nunits : (p.nunits + 1) >> 1;
+  // the pair of warps of one atom (SPLIT); this one's slabs are s0, s0 + ss, ..
+  constexpr int ss = SPLIT ? 2 : 1, NOWN = SPLIT ? (NCH + 1) / 2 : NCH;
+  const int s0 = SPLIT ? warp >> 1 : 0;
+  auto pair_sync = [&]() {
+    asm volatile("bar.sync %0, 64;" ::"r"(1 + (warp & 1)) : "memory");
+  };
 
   for (int g = blockIdx.x; g < ngroups && alive; g += gridDim.x) {
-    const Group gr = load_group(p.units, p.atype, p.nunits, g, warp, p.type_one_side);
-    float2 xt[NCH][2];  // this lane's columns of X (sums), components (0, 1), (2, 3)
+    const Group gr = load_group(p.units, p.atype, p.nunits, g, warp, p.type_one_side, SPLIT);
+    // this lane's columns of X (sums), components (0, 1), (2, 3): of chunk c,
+    // or (SPLIT) of chunk 2 c + s0
+    float2 xt[NOWN][2];
 #pragma unroll
-    for (int c = 0; c < NCH; ++c) xt[c][0] = xt[c][1] = make_float2(0.f, 0.f);
+    for (int c = 0; c < NOWN; ++c) xt[c][0] = xt[c][1] = make_float2(0.f, 0.f);
     for (int pass = 0; pass < (gr.both ? 1 : 2) && alive; ++pass) {
       const bool act = gr.atom >= 0 && (gr.both || (warp >> 1) == pass);
       for (int tj = 0; tj < p.ntypes && alive; ++tj) {
@@ -347,7 +370,8 @@ __global__ void __launch_bounds__(128, 3) k_emb_fwd(const __grid_constant__ EmbA
         const int neff = act ? distinct_rows(em, sel) : 0;
         if (lane == 0) nslab[warp] = (neff + 31) >> 5;
         __syncthreads();
-        const int nsl = max(max(nslab[0], nslab[1]), max(nslab[2], nslab[3]));
+        const int nsl =
+            (max(max(nslab[0], nslab[1]), max(nslab[2], nslab[3])) + ss - 1) / ss;
         if (cached[tj & 1] != net) {  // uniform: stage this net's weights and params
           const uint4* src = reinterpret_cast<const uint4*>(p.nets + (size_t)net * kNetBytes);
           uint4* dst = reinterpret_cast<uint4*>(slot);
@@ -359,18 +383,17 @@ __global__ void __launch_bounds__(128, 3) k_emb_fwd(const __grid_constant__ EmbA
         __syncthreads();  // nslab and cached read before they change again
         const float* par = reinterpret_cast<const float*>(slot + kNetPar);
         const uint32_t b2 = smem_addr(slot + kNetB2), b3 = smem_addr(slot + kNetB3);
-        float2 acc[NCH][2];
+        float2 acc[NOWN][2];
 #pragma unroll
-        for (int c = 0; c < NCH; ++c) acc[c][0] = acc[c][1] = make_float2(0.f, 0.f);
+        for (int c = 0; c < NOWN; ++c) acc[c][0] = acc[c][1] = make_float2(0.f, 0.f);
         auto flush = [&](int c) {
           xt[c][0] = make_float2(xt[c][0].x + acc[c][0].x, xt[c][0].y + acc[c][0].y);
           xt[c][1] = make_float2(xt[c][1].x + acc[c][1].x, xt[c][1].y + acc[c][1].y);
           acc[c][0] = acc[c][1] = make_float2(0.f, 0.f);
         };
         float4 e = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (lane < neff) e = __ldg(em + lane);
+        if (32 * s0 + lane < neff) e = __ldg(em + 32 * s0 + lane);
         for (int sl = 0; sl < nsl && alive; ++sl) {
-          const int nrow = min(32, neff - 32 * sl);  // live rows of this warp (may be <= 0)
           rsm[r] = e;
           // ---- layer 1 (FP32): h1 = tanh(s w1 + b1), all N1 columns per thread
           float h1[N1];
@@ -380,7 +403,7 @@ __global__ void __launch_bounds__(128, 3) k_emb_fwd(const __grid_constant__ EmbA
           st_half<N1, 0>(atile, r, h1);
           st_half<N1, 1>(atile, r, h1);
           // the next slab's row
-          const int jn = 32 * (sl + 1) + lane;
+          const int jn = 32 * (ss * (sl + 1) + s0) + lane;
           e = jn < neff ? __ldg(em + jn) : make_float4(0.f, 0.f, 0.f, 0.f);
           fence_proxy_async_smem();
           tc_fence_before();
@@ -437,100 +460,135 @@ __global__ void __launch_bounds__(128, 3) k_emb_fwd(const __grid_constant__ EmbA
           if (!alive) break;
           tc_fence_after();
           // ---- epilogue 3 and G^T R, 32 columns at a time: a lane per column
-          //      over the warp's rows, through the warp's quarter of A (MMA 3
-          //      is done with it)
-          if (nrow > 0) {  // uniform over the warp
-            const float4* R = rsm + warp * 32;
-            const int pos = (warp & 1) * sel + 32 * sl;
+          //      over a slab's rows, through the warp's quarter of A (MMA 3 is
+          //      done with it)
+          // rows of slab `s` (G chunk in G, env rows in R) onto the owned
+          // chunk c, up to the row that stands for the equal rest
+          auto add_slab = [&](int c, int s, const float* G, const float4* R, float& gt) {
+            const int nrow = min(32, neff - 32 * s);
+            const int pos = (warp & 1) * sel + 32 * s;
             const int brk = (128 - (pos & 127)) & 127;  // row before which the chain breaks
-            const bool tail = 32 * sl + nrow == neff;   // the last row stands for the equal rest
-            const int plain = tail ? nrow - 1 : nrow;
-            float gt[NCH];
-            auto chunk = [&](int c) {
-              auto rows = [&](int lo, int hi) {
+            const int plain = 32 * s + nrow == neff ? nrow - 1 : nrow;
+            auto rows = [&](int lo, int hi) {
 #pragma unroll 4
-                for (int rr = lo; rr < hi; ++rr) {
-                  const float gv = gbuf[rr * 32 + ((((lane >> 2) ^ (rr & 7)) << 2) | (lane & 3))];
-                  const float4 q = R[rr];
-                  acc[c][0] = __ffma2_rn(lo2(q), dup2(gv), acc[c][0]);
-                  acc[c][1] = __ffma2_rn(hi2(q), dup2(gv), acc[c][1]);
-                }
-              };
-              if (brk < plain) {
-                rows(0, brk);
-                flush(c);
-                rows(brk, plain);
-              } else {
-                rows(0, plain);
+              for (int rr = lo; rr < hi; ++rr) {
+                const float gv = G[rr * 32 + ((((lane >> 2) ^ (rr & 7)) << 2) | (lane & 3))];
+                const float4 q = R[rr];
+                acc[c][0] = __ffma2_rn(lo2(q), dup2(gv), acc[c][0]);
+                acc[c][1] = __ffma2_rn(hi2(q), dup2(gv), acc[c][1]);
               }
-              const int rr = nrow - 1;
-              gt[c] = gbuf[rr * 32 + ((((lane >> 2) ^ (rr & 7)) << 2) | (lane & 3))];
             };
-            __syncwarp();
+            if (brk < plain) {
+              rows(0, brk);
+              flush(c);
+              rows(brk, plain);
+            } else {
+              rows(0, plain);
+            }
+            const int rr = nrow - 1;
+            gt = G[rr * 32 + ((((lane >> 2) ^ (rr & 7)) << 2) | (lane & 3))];
+          };
+          // the last row of slab `s` for itself and the equal rest
+          auto add_rest = [&](int s, const float4* R, const float* gt) {
+            const float4 q = R[neff - 32 * s - 1];
+            const bool one = q.y == 0.f && q.z == 0.f && q.w == 0.f;  // a padding row
+            int at = (warp & 1) * sel + neff - 1;
+            for (int left = sel - neff + 1; left > 0;) {
+              if ((at & 127) == 0)
+#pragma unroll
+                for (int c = 0; c < NOWN; ++c) flush(c);
+              const int n = min(left, 128 - (at & 127));
+              if (one) {
+                for (int k = 0; k < n; ++k)
+#pragma unroll
+                  for (int c = 0; c < NOWN; ++c) acc[c][0].x = fmaf(q.x, gt[c], acc[c][0].x);
+              } else {
+                for (int k = 0; k < n; ++k)
+#pragma unroll
+                  for (int c = 0; c < NOWN; ++c) {
+                    acc[c][0] = __ffma2_rn(lo2(q), dup2(gt[c]), acc[c][0]);
+                    acc[c][1] = __ffma2_rn(hi2(q), dup2(gt[c]), acc[c][1]);
+                  }
+              }
+              at += n;
+              left -= n;
+            }
+          };
+          if constexpr (!SPLIT) {
+            const int nrow = min(32, neff - 32 * sl);  // live rows of this warp
+            if (nrow > 0) {  // uniform over the warp
+              const float4* R = rsm + warp * 32;
+              float gt[NCH];
+              __syncwarp();
+              epi3<N2, N3, 0>(trow, par, h2, gbuf);
+              __syncwarp();
+              add_slab(0, sl, gbuf, R, gt[0]);
+              if constexpr (NCH > 1) {
+                __syncwarp();
+                epi3<N2, N3, 1>(trow, par, h2, gbuf);
+                __syncwarp();
+                add_slab(1, sl, gbuf, R, gt[1]);
+              }
+              if constexpr (NCH > 2) {
+                __syncwarp();
+                epi3<N2, N3, 2>(trow, par, h2, gbuf);
+                __syncwarp();
+                add_slab(2, sl, gbuf, R, gt[2]);
+              }
+              if constexpr (NCH > 3) {
+                __syncwarp();
+                epi3<N2, N3, 3>(trow, par, h2, gbuf);
+                __syncwarp();
+                add_slab(3, sl, gbuf, R, gt[3]);
+              }
+              if (32 * sl + nrow == neff) add_rest(sl, R, gt);
+              __syncwarp();
+            }
+          } else if (32 * ss * sl < neff) {  // uniform over the pair
+            const int w0 = warp & 1, w1 = w0 + 2, sE = 2 * sl, sO = sE + 1;
+            const bool two = 32 * sO < neff;
+            // even chunks in a warp's quarter of A, odd ones in its odd buffer
+            const float* b0 = s0 ? odd + w0 * 1024 : reinterpret_cast<float*>(atile + w0 * 4096);
+            const float* b1 = s0 ? odd + w1 * 1024 : reinterpret_cast<float*>(atile + w1 * 4096);
+            float gt[NOWN] = {};
             epi3<N2, N3, 0>(trow, par, h2, gbuf);
-            __syncwarp();
-            chunk(0);
-            if constexpr (NCH > 1) {
-              __syncwarp();
-              epi3<N2, N3, 1>(trow, par, h2, gbuf);
-              __syncwarp();
-              chunk(1);
+            if constexpr (NCH > 1) epi3<N2, N3, 1>(trow, par, h2, odd + warp * 1024);
+            pair_sync();
+            if (s0 < NCH) {
+              add_slab(0, sE, b0, rsm + w0 * 32, gt[0]);
+              if (two) add_slab(0, sO, b1, rsm + w1 * 32, gt[0]);
             }
             if constexpr (NCH > 2) {
-              __syncwarp();
+              pair_sync();
               epi3<N2, N3, 2>(trow, par, h2, gbuf);
-              __syncwarp();
-              chunk(2);
-            }
-            if constexpr (NCH > 3) {
-              __syncwarp();
-              epi3<N2, N3, 3>(trow, par, h2, gbuf);
-              __syncwarp();
-              chunk(3);
-            }
-            if (tail) {
-              const float4 q = R[nrow - 1];
-              const bool one = q.y == 0.f && q.z == 0.f && q.w == 0.f;  // a padding row
-              int at = (warp & 1) * sel + neff - 1;
-              for (int left = sel - neff + 1; left > 0;) {
-                if ((at & 127) == 0)
-#pragma unroll
-                  for (int c = 0; c < NCH; ++c) flush(c);
-                const int n = min(left, 128 - (at & 127));
-                if (one) {
-                  for (int k = 0; k < n; ++k)
-#pragma unroll
-                    for (int c = 0; c < NCH; ++c) acc[c][0].x = fmaf(q.x, gt[c], acc[c][0].x);
-                } else {
-                  for (int k = 0; k < n; ++k)
-#pragma unroll
-                    for (int c = 0; c < NCH; ++c) {
-                      acc[c][0] = __ffma2_rn(lo2(q), dup2(gt[c]), acc[c][0]);
-                      acc[c][1] = __ffma2_rn(hi2(q), dup2(gt[c]), acc[c][1]);
-                    }
-                }
-                at += n;
-                left -= n;
+              if constexpr (NCH > 3) epi3<N2, N3, 3>(trow, par, h2, odd + warp * 1024);
+              pair_sync();
+              if (2 + s0 < NCH) {
+                add_slab(1, sE, b0, rsm + w0 * 32, gt[1]);
+                if (two) add_slab(1, sO, b1, rsm + w1 * 32, gt[1]);
               }
             }
-            __syncwarp();
+            if (32 * (two ? sO : sE) + 32 >= neff)
+              add_rest(two ? sO : sE, rsm + (two ? w1 : w0) * 32, gt);
+            pair_sync();  // the buffers read before they are filled again
           }
           tc_fence_before();
         }
 #pragma unroll
-        for (int c = 0; c < NCH; ++c) flush(c);
+        for (int c = 0; c < NOWN; ++c) flush(c);
       }
     }
     if (!alive) break;
     // ---- X and D of this warp's atom
     if (gr.atom >= 0) {
       const size_t row = p.drow ? (size_t)p.drow[gr.atom] : (size_t)gr.atom;
-      float4* xT = reinterpret_cast<float4*>(gbuf);
+      // (SPLIT: the pair shares xT and the rows of D)
+      float4* xT = reinterpret_cast<float4*>(atile + (SPLIT ? warp & 1 : warp) * 4096);
       float nk = 0.f, na = 0.f;
       __syncwarp();
 #pragma unroll
-      for (int c = 0; c < NCH; ++c) {
-        const int m = 32 * c + lane;
+      for (int c = 0; c < NOWN; ++c) {
+        const int m = 32 * (ss * c + s0) + lane;
         if (m < N3) {
           const float4 x = make_float4(xt[c][0].x * inv_nnei, xt[c][0].y * inv_nnei,
                                        xt[c][1].x * inv_nnei, xt[c][1].y * inv_nnei);
@@ -545,7 +603,17 @@ __global__ void __launch_bounds__(128, 3) k_emb_fwd(const __grid_constant__ EmbA
           if (m < p.A) na = fmaxf(na, q);
         }
       }
-      __syncwarp();
+      if constexpr (SPLIT)
+        pair_sync();
+      else
+        __syncwarp();
+      if constexpr (SPLIT)
+        for (int m = lane; m < N3; m += 32) {
+          const float4 x = xT[m];
+          const float q = x.x * x.x + x.y * x.y + x.z * x.z + x.w * x.w;
+          nk = fmaxf(nk, q);
+          if (m < p.A) na = fmaxf(na, q);
+        }
       auto dval = [&](int m, int a) {
         const float4 u = xT[m], w = xT[a];
         return fmaf(u.w, w.w, fmaf(u.z, w.z, fmaf(u.y, w.y, fmaf(u.x, w.x, 0.f))));
@@ -561,20 +629,23 @@ __global__ void __launch_bounds__(128, 3) k_emb_fwd(const __grid_constant__ EmbA
         const float sc = f16_scale_for(sqrtf(nk * na) * 1.0001f);
         __half* dh = static_cast<__half*>(p.D) + row * (size_t)N3 * p.A;
         __half* dl = static_cast<__half*>(p.D_lo) + row * (size_t)N3 * p.A;
-        for (int at = 4 * lane; at < N3 * p.A; at += 128) {
+        for (int at = 4 * (lane + 32 * s0); at < N3 * p.A; at += 128 * ss) {
           const int m = at / p.A, a = at - m * p.A;
           const float v[4] = {dval(m, a), dval(m, a + 1), dval(m, a + 2), dval(m, a + 3)};
           st_split4_f16(dh + at, dl + at, v, sc);
         }
-        if (lane == 0) p.D_rs[row] = 1.f / sc;
+        if (lane == 0 && s0 == 0) p.D_rs[row] = 1.f / sc;
       } else {
         float* d = static_cast<float*>(p.D) + row * (size_t)N3 * p.A;
-        for (int at = lane; at < N3 * p.A; at += 32) {
+        for (int at = lane + 32 * s0; at < N3 * p.A; at += 32 * ss) {
           const int m = at / p.A;
           d[at] = dval(m, at - m * p.A);
         }
       }
-      __syncwarp();
+      if constexpr (SPLIT)
+        pair_sync();
+      else
+        __syncwarp();
     }
   }
   tc_fence_before();
@@ -639,6 +710,8 @@ __host__ __device__ constexpr size_t dx16_warp_bytes(int N3) {
 __global__ void __launch_bounds__(kDxWarps * 32)
     k_emb_dx16(float* __restrict__ dxs, const float* __restrict__ dD, const float* __restrict__ X,
                const int* __restrict__ drow, int nloc, int N3, float inv_nnei) {
+  grid_wait();
+  grid_release();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int atom = blockIdx.x * kDxWarps + warp;
@@ -775,8 +848,12 @@ __device__ __forceinline__ void bepi3(uint32_t trow, const float* par, const flo
   }
 }
 
-template <int N1, int N2, int N3>
+// SPLIT as in k_emb_fwd: every row's gradient is its own, so the warps of an
+// atom need nothing of each other.
+template <int N1, int N2, int N3, bool SPLIT>
 __global__ void __launch_bounds__(128, 2) k_emb_bwd(const __grid_constant__ EmbBwdArgs p) {
+  grid_wait();
+  grid_release();
   extern __shared__ unsigned char smem_raw[];
   unsigned char* sm = reinterpret_cast<unsigned char*>(
       (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -812,13 +889,16 @@ __global__ void __launch_bounds__(128, 2) k_emb_bwd(const __grid_constant__ EmbB
 
   const uint32_t aaddr = smem_addr(atile);
   float4* dx = dxsm + warp * 128;
-  const int ngroups = (p.nunits + 1) >> 1;
+  const int ngroups = SPLIT ? p.nunits : (p.nunits + 1) >> 1;
+  // this warp's slabs of its atom's section: s0, s0 + ss, ..
+  constexpr int ss = SPLIT ? 2 : 1;
+  const int s0 = SPLIT ? warp >> 1 : 0;
 
   for (int tj = 0; tj < p.ntypes && alive; ++tj) {
     const int sel = p.sec[tj + 1] - p.sec[tj];
     if (sel == 0) continue;
     for (int g = blockIdx.x; g < ngroups && alive; g += gridDim.x) {
-      const Group gr = load_group(p.units, p.atype, p.nunits, g, warp, p.type_one_side);
+      const Group gr = load_group(p.units, p.atype, p.nunits, g, warp, p.type_one_side, SPLIT);
       for (int pass = 0; pass < (gr.both ? 1 : 2) && alive; ++pass) {
         const bool act = gr.atom >= 0 && (gr.both || (warp >> 1) == pass);
         const int net = p.type_one_side ? tj : tj * p.ntypes + gr.ti[pass];
@@ -833,7 +913,8 @@ __global__ void __launch_bounds__(128, 2) k_emb_bwd(const __grid_constant__ EmbB
             dx[m] = make_float4(d[0], d[N3], d[2 * N3], d[3 * N3]);
           }
         __syncthreads();  // (and the previous group is done with the shared buffers)
-        const int nsl = max(max(nslab[0], nslab[1]), max(nslab[2], nslab[3]));
+        const int nsl =
+            (max(max(nslab[0], nslab[1]), max(nslab[2], nslab[3])) + ss - 1) / ss;
         if (cached[0] != net) {
           const uint4* src = reinterpret_cast<const uint4*>(p.nets + (size_t)net * kNetBytes);
           uint4* dst = reinterpret_cast<uint4*>(slot);
@@ -847,12 +928,13 @@ __global__ void __launch_bounds__(128, 2) k_emb_bwd(const __grid_constant__ EmbB
         const uint32_t b2 = smem_addr(slot + kNetB2), b3 = smem_addr(slot + kNetB3);
         const uint32_t b3t = smem_addr(slot + kNetB3T), b2t = smem_addr(slot + kNetB2T);
         float4 en = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (lane < neff) en = __ldg(em + lane);
+        if (32 * s0 + lane < neff) en = __ldg(em + 32 * s0 + lane);
         for (int sl = 0; sl < nsl && alive; ++sl) {
-          const int j = 32 * sl + lane;
+          const int slab = ss * sl + s0;
+          const int j = 32 * slab + lane;
           const bool live = j < neff;
           const float4 e = en;
-          en = j + 32 < neff ? __ldg(em + j + 32) : make_float4(0.f, 0.f, 0.f, 0.f);
+          en = j + 32 * ss < neff ? __ldg(em + j + 32 * ss) : make_float4(0.f, 0.f, 0.f, 0.f);
           // ---- forward recompute: layer 1, MMA 2, epilogue 2, MMA 3
           float h1[N1];
   #pragma unroll
@@ -994,7 +1076,7 @@ __global__ void __launch_bounds__(128, 2) k_emb_bwd(const __grid_constant__ EmbB
             const float4 o = make_float4(ds + dr[0], dr[1], dr[2], dr[3]);
             if (live) out[j] = o;
             // the last row's gradient is that of the equal rows after it too
-            const int tl = neff - 1 - 32 * sl;
+            const int tl = neff - 1 - 32 * slab;
             if (tl >= 0 && tl < 32) {  // uniform over the warp
               const float4 q = make_float4(
                   __shfl_sync(kFull, o.x, tl), __shfl_sync(kFull, o.y, tl),
@@ -1014,15 +1096,26 @@ __global__ void __launch_bounds__(128, 2) k_emb_bwd(const __grid_constant__ EmbB
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 256;" ::"r"(tmem) : "memory");
 }
 
+// A unit a CTA while all of them are resident at once, two an SM (forward and
+// backward, 120 atoms: 70 us with two units a CTA, 56 so; 450 atoms: 78, 66).
+// Above that two units a CTA: half the tiles are then taken per SM and the
+// warps' work, not the chain, bounds the call.
+inline bool split_units(int nunits, int& sms) {
+  int dev = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  return nunits <= 2 * sms;
+}
+
 // 92 KiB: two CTAs per SM (2 x 256 TMEM columns)
 template <int N3>
 constexpr size_t bwd_smem() {
   return 1024 + kBwdSlot + 32768 + 4 * 128 * 16 + 64;
 }
 
-template <int N1, int N2, int N3>
-int emb_bwd_launch(const EmbBwdArgs& a, cudaStream_t st) {
-  auto kern = k_emb_bwd<N1, N2, N3>;
+template <int N1, int N2, int N3, bool SPLIT>
+int emb_bwd_launch(const EmbBwdArgs& a, int sms, cudaStream_t st) {
+  auto kern = k_emb_bwd<N1, N2, N3, SPLIT>;
   constexpr size_t smem = bwd_smem<N3>();
   static const cudaError_t attr = [&] {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -1035,22 +1128,21 @@ int emb_bwd_launch(const EmbBwdArgs& a, cudaStream_t st) {
   // two CTAs per SM: registers by __launch_bounds__(128, 2), shared memory
   // below half an SM's
   static_assert(2 * (smem + 1024) <= 228 * 1024, "two CTAs per SM");
-  int dev = 0, sms = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const int grid = std::max(1, std::min(2 * sms, (a.nunits + 1) / 2));
-  kern<<<grid, 128, smem, st>>>(a);
+  const int grid = std::max(1, SPLIT ? a.nunits : std::min(2 * sms, (a.nunits + 1) / 2));
+  launch_dep(kern, dim3(grid), dim3(128), smem, st, a);
   GBDP_CHECK_LAUNCH("embed_bwd_tc");
   return GBDP_OK;
 }
 
 // 72 KiB: three CTAs per SM (3 x 128 TMEM columns)
-constexpr size_t fwd_smem() { return 1024 + 2 * kSlot + 16384 + kRows * 16 + 64; }
+// (SPLIT: 16 KiB more, two an SM)
+template <bool SPLIT>
+constexpr size_t fwd_smem() { return 1024 + kFwdBytes + (SPLIT ? 16384 : 0); }
 
-template <int N1, int N2, int N3>
-int emb_fwd_launch(const EmbArgs& a, cudaStream_t st) {
-  auto kern = k_emb_fwd<N1, N2, N3>;
-  constexpr size_t smem = fwd_smem();
+template <int N1, int N2, int N3, bool SPLIT>
+int emb_fwd_launch(const EmbArgs& a, int sms, cudaStream_t st) {
+  auto kern = k_emb_fwd<N1, N2, N3, SPLIT>;
+  constexpr size_t smem = fwd_smem<SPLIT>();
   // the largest shared-memory carveout, so that three CTAs fit an SM
   static const cudaError_t attr = [&] {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -1062,12 +1154,9 @@ int emb_fwd_launch(const EmbArgs& a, cudaStream_t st) {
   if (attr != cudaSuccess) return cuda_status(attr, "embed_fwd_tc attribute");
   // three CTAs per SM: registers by __launch_bounds__(128, 3), shared memory
   // below a third of an SM's
-  static_assert(3 * (smem + 1024) <= 228 * 1024, "three CTAs per SM");
-  int dev = 0, sms = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const int grid = std::max(1, std::min(3 * sms, (a.nunits + 1) / 2));
-  kern<<<grid, 128, smem, st>>>(a);
+  static_assert((SPLIT ? 2 : 3) * (smem + 1024) <= 228 * 1024, "CTAs per SM");
+  const int grid = std::max(1, SPLIT ? a.nunits : std::min(3 * sms, (a.nunits + 1) / 2));
+  launch_dep(kern, dim3(grid), dim3(128), smem, st, a);
   GBDP_CHECK_LAUNCH("embed_fwd_tc");
   return GBDP_OK;
 }
@@ -1122,8 +1211,14 @@ extern "C" int gbdp_embed_fwd_tc_bf16(float* X, void* D, void* D_lo, float* D_rs
   GBDP_REQUIRE(a.sec[ntypes] == nnei, "embed_fwd_tc: sum(sel) %d != nnei %d", a.sec[ntypes], nnei);
   if (nunits == 0) return GBDP_OK;
   const cudaStream_t st = (cudaStream_t)stream;
-  if (n1 == 25 && n2 == 50 && n3 == 100) return emb_fwd_launch<25, 50, 100>(a, st);
-  if (n1 == 3 && n2 == 6 && n3 == 12) return emb_fwd_launch<3, 6, 12>(a, st);
+  int sms = 0;
+  const bool split = split_units(nunits, sms);
+  if (n1 == 25 && n2 == 50 && n3 == 100)
+    return split ? emb_fwd_launch<25, 50, 100, true>(a, sms, st)
+                 : emb_fwd_launch<25, 50, 100, false>(a, sms, st);
+  if (n1 == 3 && n2 == 6 && n3 == 12)
+    return split ? emb_fwd_launch<3, 6, 12, true>(a, sms, st)
+                 : emb_fwd_launch<3, 6, 12, false>(a, sms, st);
   set_error("embed_fwd_tc: embedding widths %d-%d-%d not built (25-50-100, 3-6-12)", n1, n2, n3);
   return GBDP_ERR_INVALID;
 }
@@ -1172,11 +1267,17 @@ extern "C" int gbdp_embed_bwd_tc_bf16(float* net_deriv, float* dx_work, const fl
   const size_t shm = sizeof(float) * (size_t)(4 * n3 + n3 * (axis + 1) + 4 * axis);
   GBDP_REQUIRE(shm <= 48 * 1024, "embed_bwd_tc: N3 * axis too large");
   if (axis == 16 && ((uintptr_t)dD & 15) == 0 && kDxWarps * dx16_warp_bytes(n3) <= 48 * 1024)
-    k_emb_dx16<<<(unsigned)((nloc + kDxWarps - 1) / kDxWarps), kDxWarps * 32,
-                 kDxWarps * dx16_warp_bytes(n3), st>>>(dx_work, dD, X, drow, nloc, n3,
-                                                       1.f / (float)nnei);
+    launch_dep(k_emb_dx16, dim3((unsigned)((nloc + kDxWarps - 1) / kDxWarps)), dim3(kDxWarps * 32),
+               kDxWarps * dx16_warp_bytes(n3), st, dx_work, dD, X, drow, nloc, n3,
+               1.f / (float)nnei);
   else
     k_emb_dx<<<nloc, 128, shm, st>>>(dx_work, dD, X, drow, n3, axis, 1.f / (float)nnei);
   GBDP_CHECK_LAUNCH("embed_dx");
-  return w25 ? emb_bwd_launch<25, 50, 100>(a, st) : emb_bwd_launch<3, 6, 12>(a, st);
+  int sms = 0;
+  const bool split = split_units(nunits, sms);
+  if (w25)
+    return split ? emb_bwd_launch<25, 50, 100, true>(a, sms, st)
+                 : emb_bwd_launch<25, 50, 100, false>(a, sms, st);
+  return split ? emb_bwd_launch<3, 6, 12, true>(a, sms, st)
+               : emb_bwd_launch<3, 6, 12, false>(a, sms, st);
 }

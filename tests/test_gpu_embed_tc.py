@@ -157,3 +157,44 @@ def test_equal_rows_and_slabs(setup, one_side, mols):
     Dr = torch.einsum("ncm,nca->nma", Xr, Xr[:, :, :cfg.axis_neuron]).reshape(b.nloc, -1)
     ref = torch.autograd.grad(Dr, x, b.dD[b.drow.long()])[0]
     assert float((net - ref).abs().max()) <= 2e-2 * float(ref.abs().max())
+
+
+@pytest.mark.parametrize("one_side", [True, False])
+def test_one_and_two_units_a_block_agree(setup, one_side):
+    """Few units take a block each, an atom's slabs on two warps; many, two
+    a block: the same bits, X, D and dE/d(env matrix), for 41 molecules by
+    themselves (62 units) and as the first of 210 (315)."""
+    se_a, water, cfg0, m64, _, _ = setup
+    import dataclasses
+
+    cfg = dataclasses.replace(cfg0, type_one_side=one_side)
+    mdl = importlib.import_module("dpmd_public_gb300.model")
+    m = se_a.SeAModel(cfg, mdl.init_params(cfg, 3), m64.davg.cpu().numpy(),
+                      m64.dstd.cpu().numpy(), DEV, torch.float32)
+    g = torch.Generator(device=DEV).manual_seed(5)
+    em = torch.randn(630, cfg.nnei, 4, generator=g, device=DEV)
+    dD = torch.randn(630, cfg.neuron[-1] * cfg.axis_neuron, generator=g, device=DEV) * 0.05
+    cut = torch.randint(1, 46, (630, 2), generator=g, device=DEV).tolist()
+    for i, ks in enumerate(cut):  # equal rows from a random place on
+        for t in range(2):
+            em[i, cfg.sec[t] + ks[t] * (t + 1):cfg.sec[t + 1]] = torch.tensor([-0.4, 0., 0., 0.],
+                                                                              device=DEV)
+    got = []
+    for mols in (41, 210):
+        n = 3 * mols
+        b = m.batch([np.tile(np.array([0, 1, 1], np.int32), mols)],
+                    np.diag([60.0] * 3).reshape(1, 9))
+        b.ensure_plain_tc(m)
+        b.dD.zero_()
+        b.dD[b.drow.long()] = dD[:n]
+        e = em[:n].contiguous()
+        m.embed_tc_forward(b, e)
+        net = m.embed_tc_backward(b, e)
+        torch.cuda.synchronize()
+        assert int(b.emb_status.item()) == 0
+        D = b.D[b.drow.long()]
+        lo = getattr(b, "D_lo", None)
+        parts = [b.X, net, D] + ([] if lo is None else [lo[b.drow.long()], b.D_rs[b.drow.long()]])
+        got.append([q[:123].clone() for q in parts])
+    for a, c in zip(*got):
+        assert torch.equal(a, c)
