@@ -278,3 +278,32 @@ def test_fused_deterministic_mode(mods, built, dtype):
     g.replay()
     torch.cuda.synchronize()
     assert torch.equal(out[1], F) and torch.equal(out[0], E) and torch.equal(out[2], V)
+
+
+@pytest.mark.parametrize("dtype", [torch.float64, torch.float32])
+@pytest.mark.parametrize("det", [0, 1])
+@pytest.mark.parametrize("nrows,nframes", [(1, 1), (33, 40), (2047, 3), (2048, 300), (2049, 3),
+                                           (5000, 17)])
+def test_frame_energies(mods, dtype, det, nrows, nframes):
+    """Rows of frames in any order and padding rows (frame -1), at the row
+    counts where one block takes over from a grid, over an output that held
+    other values: sums within n u of the magnitudes' (u = 2^-53), plus the
+    fixed point's half step a row (2^-31) in the deterministic mode."""
+    import importlib
+
+    L = importlib.import_module("dpmd_public_gb300._lib")
+    lib = L.load()
+    g = torch.Generator(device=DEV).manual_seed(nrows)
+    ae = torch.randn(nrows, generator=g, device=DEV, dtype=dtype)
+    f = torch.randint(-1, nframes, (nrows,), generator=g, device=DEV, dtype=torch.int32)
+    E = torch.full((nframes,), 7.0, device=DEV, dtype=torch.float64)
+    fn = lib.gbdp_frame_energy_f64 if dtype == torch.float64 else lib.gbdp_frame_energy_f32
+    rc = fn(E.data_ptr(), ae.data_ptr(), f.data_ptr(), nrows, nframes, det,
+            torch.cuda.current_stream().cuda_stream)
+    assert rc == 0
+    ok = (f >= 0).double()
+    z = torch.zeros(nframes, device=DEV, dtype=torch.float64)
+    ref = z.clone().index_add_(0, f.clamp_min(0).long(), ae.double() * ok)
+    mag = z.clone().index_add_(0, f.clamp_min(0).long(), ae.double().abs() * ok)
+    bound = 2 * nrows * 2.0 ** -53 * mag + (nrows * 2.0 ** -31 if det else 0.0)
+    assert bool(((E - ref).abs() <= bound).all())
