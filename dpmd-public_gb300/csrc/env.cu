@@ -709,13 +709,15 @@ struct VList {
 //              written to the Verlet list; nothing else
 enum { kEnvCells = 0, kEnvList = 1, kEnvBuild = 2 };
 
-// A warp per centre, bound by instruction issue (72 % of the slots, 0.22 ms
-// for 51,304 atoms; some 3,800 warp instructions a centre: 40 % the cell
-// search, a quarter each the ordering and the rows).  On 125,000 atoms of
+// A warp per centre, bound by instruction issue (75 % of the slots; 135 us for
+// 37,830 atoms, some 3,200 warp instructions a centre; before, of 3,800, 40 %
+// the cell search and a quarter each the ordering and the rows).  On 125,000 atoms of
 // ragged water the neighbour part of a step took 640 us with every half cell
 // of the stencil searched, the types sorted by networks and the statistics
-// loaded one value at a time, and 548 us now; of the three alone, searching
-// every cell again gives 628, sorting 661, single loads 557.
+// loaded one value at a time, and 522 us now; at 548 us, searching every cell
+// again gave 628, sorting 661, single loads 557 (launching the chain of
+// kernels as dependents took another 18 off, reading the box's shape from
+// FP32 instead of FP64 8).
 
 template <typename T, int MODE>
 __global__ void __launch_bounds__(kEnvWarps * 32)
@@ -819,8 +821,8 @@ __global__ void __launch_bounds__(kEnvWarps * 32)
     uf[d] = (float)(d == 0 ? xi : d == 1 ? yi : zi) * (g.recf[4 * d] * nf) -
             (float)(F[d] - fs[d] * g.ngcell[d]);
     mf[d] = 1e-3f + 1e-6f * nf;
-    diag = diag && g.boxf[4 * d] > 0.f && g.box[3 * d + (d + 1) % 3] == 0. &&
-           g.box[3 * d + (d + 2) % 3] == 0.;
+    diag = diag && g.boxf[4 * d] > 0.f && g.boxf[3 * d + (d + 1) % 3] == 0.f &&
+           g.boxf[3 * d + (d + 2) % 3] == 0.f;
   }
   const float far2 = diag ? rc2f * 1.0001f : FLT_MAX;
   const int sy = 2 * hw[1] + 1, sz = 2 * hw[2] + 1;
