@@ -1008,7 +1008,9 @@ def graph_kernels(graph):
         nm = (name.value or b"?").decode(errors="replace")
         if "gbdp" in nm:
             ours += 1
-            m = re.search(r"(k_[a-z0-9_]+)", nm)
+            # (the mangled name of a kernel of namespace gbdp's anonymous one
+            # may follow a file name that holds "k_" too: the last match)
+            m = re.search(r".*\d(k_[a-z0-9_]+)", nm) or re.search(r"(k_[a-z0-9_]+)", nm)
             short = m.group(1) if m else nm
             names[short] = names.get(short, 0) + 1
         else:
@@ -1300,24 +1302,24 @@ PART_KERNEL = {"env_nlist": "k_nlist_env (+ cell build and ghost fill)",
                "desc_fwd": "k_fwd_blk", "desc_bwd": "k_bwd_blk"}
 
 # dram__bytes_read.sum + dram__bytes_write.sum per local atom, from one ncu
-# capture of the 12,288-atom step (profiles/k_desc_fwd_bwd_12288.md,
-# profiles/k_fit_tc_12288.md: the six fitting GEMM launches summed), scaled
-# to a launch by the atoms it processes (the traffic of these kernels grows
-# in proportion to the atoms)
-NCU_TRAFFIC_ATOM = {"desc_bwd": 133.1e6 / 12288, "desc_fwd": 65.7e6 / 12288,
-                    "fitting_gemm": 6 * 40.6e6 / 12288}
-NCU_TRAFFIC_SRC = "ncu capture of the 12,288-atom step, scaled by atoms"
+# capture of a 48-frame ragged step of 37,830 atoms (profiles/
+# step_kernels_ragged48.md; the fitting's three launches summed), scaled to a
+# launch by the atoms it processes (the traffic of these kernels grows in
+# proportion to the atoms)
+NCU_TRAFFIC_ATOM = {"desc_bwd": 417.2e6 / 37830, "desc_fwd": 320.4e6 / 37830,
+                    "fitting_gemm": 566.7e6 / 37830}
+NCU_TRAFFIC_SRC = "ncu capture of a 37,830-atom ragged step, scaled by atoms"
 
 
 def roofline(name, t, nat, cfg, peaks, fit_mode):
     ms = t["ms"]
     if name == "fitting_gemm":
         tc = fit_mode == "tc-f16x3"
-        nl = 6 if tc else 1
+        nl = 3 if tc else 1
         flops = _fit_flops(cfg) * nat
         ach = flops / (ms * 1e-3) / 1e12
         peak = peaks["bf16_tflops"]
-        out = {"kernel": "k_fit_tc + k_fit_pers" if tc else f"cuBLAS ({fit_mode}) + k_fit_*", "bound": "tensor",
+        out = {"kernel": "k_fit_f1 + k_fit_mid + k_fit_b1" if tc else f"cuBLAS ({fit_mode}) + k_fit_*", "bound": "tensor",
                "achieved": ach, "peak": peak, "unit": "TFLOP/s", "frac": ach / peak,
                "traffic": NCU_TRAFFIC_ATOM[name] * nat / nl if tc else None,
                "traffic_src": NCU_TRAFFIC_SRC if tc else None,

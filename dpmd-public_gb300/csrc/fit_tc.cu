@@ -23,12 +23,13 @@
 // kb % 3, the two small cross terms to a fourth accumulator, and the
 // epilogue adds the four in IEEE FP32.
 //
-// One kernel computes a 128-row tile of C = A B for one layer (tile widths
-// per layer in the TcCfg configurations below); its fused
+// A kernel computes 128-row tiles of C = A B; its fused
 // epilogue applies the layer's activation (forward) or gradient chain
 // (backward) and writes the next GEMM's A operand already split, so the
 // whole per-type fitting net (deepmd/pt/model/task/fitting.py:734-899,
-// layer semantics deepmd/dpmodel/utils/network.py) is six launches:
+// layer semantics deepmd/dpmodel/utils/network.py) is six layers, from 30 row
+// blocks on in three launches (k_fit_f1; k_fit_mid for F2, F3, B3 and B2;
+// k_fit_b1), below in six of k_fit_tc (narrow tiles):
 //   F1  T1 = tanh(D W1 + b1)                    -> H1 = T1 (split)
 //   F2  T2 = tanh(H1 W2 + b2), H2 = T2 idt2 + T1 (split)
 //   F3  T3 = tanh(H2 W3 + b3), H3 = T3 idt3 + H2, e += H3 w_out,
@@ -70,8 +71,8 @@ constexpr int A_TILE = TBM * TBK * 2;  // 16 KiB
 //              per SM, a second CTA's epilogue overlapping the first's main
 //              loop measured faster than the persistent kernel (about 21 us
 //              against 25-27 us a layer).
-// B1 runs on the persistent kernel k_fit_pers (with 128 x 80 tiles on the
-// 12,288-row step: 64 us per tile-CTA -> 49 us persistent).
+// Where F1, the K-240 layers and B1 have kernels of their own (k_fit_f1,
+// k_fit_mid, k_fit_b1) these two serve what those leave.
 template <int TBN_, int STAGES_, int NACC_>
 struct TcCfg {
   static constexpr int TBN = TBN_, STAGES = STAGES_, NACC = NACC_;
