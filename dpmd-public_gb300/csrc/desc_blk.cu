@@ -16,9 +16,9 @@
 // k_bwd_blk.  As k_desc_bwd: 16 lanes per neighbour, U x 2 neighbours in
 // flight per warp; dE/dD is read once, coalesced, for both products of dX.
 //
-// Both run one warp per atom, or (S = 4, small batches) the four warps of a
-// CTA on one atom's neighbours, so that the serial walk over the neighbours
-// is a quarter as long and a few hundred atoms still fill the SMs.
+// Both run one warp per atom, or (S = 4 and, forward, 8: small batches) the
+// warps of a CTA on one atom's neighbours, so that the serial walk over the
+// neighbours is that much shorter and a few hundred atoms still fill the SMs.
 //
 // Bounds and measurements (water, M = 100; against the k-planar kernels).
 // 125,000 atoms in 160 frames: forward 1,178 -> 1,008 us (L1: without the kept
@@ -715,8 +715,11 @@ __global__ void __launch_bounds__(W * 32, bwd_warps(U) / W)
 // slots, the barriers and the sums across warps cost more.  Measured on
 // water, shared / own, us: forward 192 atoms 18.4 / 24.4, 1200: 24.4 / 30.5,
 // 1800: 36.7 / 31.3; backward 192: 31.7 / 48.1, 768: 39.9 / 50.1, 1200: 52.2
-// / 52.2, 1800: 58.3 / 54.2.
-constexpr int kShareFwd = 152 * 10, kShareBwd = 152 * 8;
+// / 52.2, 1800: 58.3 / 54.2.  The forward takes eight warps an atom while all
+// CTAs are resident at once, four an SM (eight / four, us: 48 atoms 14.5 /
+// 19.0, 192: 14.5 / 18.6, 600: 16.6 / 20.5, 1200: 27.0 / 24.5; the backward,
+// two CTAs an SM, gains at most 2 us up to 300 atoms and loses 6 at 600).
+constexpr int kShareFwd8 = 152 * 4, kShareFwd = 152 * 10, kShareBwd = 152 * 8;
 
 // shared memory of a launch, and the smallest shared-memory carveout that
 // holds the resident CTAs: the rest of the unified L1 caches table rows
@@ -746,6 +749,8 @@ void fwd_width(const DescFwdArgs& a, const TabSet<float>& ts, int nloc, int M, i
     launch_fwd<NS, 1, 1>(a, ts, nloc, M, st);
   else if (W == 2)
     launch_fwd<NS, 2, 1>(a, ts, nloc, M, st);
+  else if (nloc <= kShareFwd8)
+    launch_fwd<NS, 8, 8>(a, ts, nloc, M, st);
   else if (nloc < kShareFwd)
     launch_fwd<NS, 4, 4>(a, ts, nloc, M, st);
   else

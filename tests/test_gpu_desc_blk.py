@@ -56,6 +56,13 @@ def test_widths(gb, mods, mols, width, sel):
     _check(gb, mods, mols, width, sel)
 
 
+@pytest.mark.parametrize("width,sel", [(16, (46, 92)), (20, (5, 7)), (36, (46, 92)), (128, (46, 92))])
+def test_widths_between(gb, mods, width, sel):
+    """900 atoms: four warps an atom in both directions (fewer take eight in
+    the forward, more a warp an atom)."""
+    _check(gb, mods, 300, width, sel)
+
+
 def _descriptor(gb, m, dtype, form, b, em, dD, X=None):
     """X, D (X is None) or force, virial of one kernel form."""
     import ctypes
