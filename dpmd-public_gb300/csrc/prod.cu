@@ -654,6 +654,7 @@ struct ProdWs {
   int* bsum;
   int* pairs_a;
   int* pairs_b;
+  size_t no_vir12;   // bytes without the last, for calls that need no vir12
   size_t bytes;
 };
 
@@ -666,12 +667,11 @@ ProdWs carve_prod(void* base, int nframes, int nloc, int nall, int nnei, int det
     off += a256(n);
     return r;
   };
+  if (!det) w.force4 = reinterpret_cast<float4*>(take(sizeof(float4) * (size_t)nframes * nall));
   w.vir_acc = reinterpret_cast<double*>(take(sizeof(double) * 9 * (size_t)nframes));
-  if (!det) {
-    // (directly after vir_acc: one clear for both)
+  w.no_vir12 = off;
+  if (!det)  // (directly after vir_acc: one clear for both)
     w.vir12 = reinterpret_cast<float*>(take(sizeof(float) * 12 * (size_t)nframes * nall));
-    w.force4 = reinterpret_cast<float4*>(take(sizeof(float4) * (size_t)nframes * nall));
-  }
   if (det) {
     const size_t nchunk = (size_t)(nall + kVirChunk - 1) / kVirChunk;
     w.vir_part = reinterpret_cast<double*>(take(sizeof(double) * 9 * (size_t)nframes * nchunk));
@@ -807,10 +807,11 @@ int prod_launch(T* force, T* virial, T* atom_virial, const T* net, const T* dR, 
                nnei, nframes);
   ProdWs w = carve_prod(ws, nframes, nloc, nall, nnei, det);
   GBDP_REQUIRE(ws != nullptr || w.bytes == 0, "prod_force/virial: null workspace");
-  GBDP_REQUIRE(ws_bytes >= w.bytes, "prod_force/virial: workspace %zu < %zu", ws_bytes, w.bytes);
+  const bool empty = nframes == 0 || nloc == 0 || nnei == 0;
+  const size_t need = det || (sizeof(T) == 4 && atom_virial && !empty) ? w.bytes : w.no_vir12;
+  GBDP_REQUIRE(ws_bytes >= need, "prod_force/virial: workspace %zu < %zu", ws_bytes, need);
   // the atomic mode clears what it adds into, the FP32 form writing every
   // word of the outputs from its padded rows
-  const bool empty = nframes == 0 || nloc == 0 || nnei == 0;
   if (det || empty) {
     if (force) cudaMemsetAsync(force, 0, sizeof(T) * (size_t)nframes * nall * 3, st);
     if (atom_virial) cudaMemsetAsync(atom_virial, 0, sizeof(T) * (size_t)nframes * nall * 9, st);
@@ -860,8 +861,9 @@ int prod_virial_impl(T* virial, T* atom_virial, const T* net, const T* dR, const
                "prod_virial_a: bad sizes");
   ProdWs w = carve_prod(ws, nframes, nloc, nall, nnei, det);
   GBDP_REQUIRE(ws != nullptr, "prod_virial_a: null workspace");
-  GBDP_REQUIRE(ws_bytes >= w.bytes, "prod_virial_a: workspace %zu < %zu", ws_bytes, w.bytes);
   const bool empty = nframes == 0 || nloc == 0 || nnei == 0;
+  const size_t need = det || (sizeof(T) == 4 && !empty) ? w.bytes : w.no_vir12;
+  GBDP_REQUIRE(ws_bytes >= need, "prod_virial_a: workspace %zu < %zu", ws_bytes, need);
   if (det || empty) cudaMemsetAsync(atom_virial, 0, sizeof(T) * (size_t)nframes * nall * 9, st);
   if (empty) {
     cudaMemsetAsync(virial, 0, sizeof(T) * (size_t)nframes * 9, st);

@@ -233,3 +233,29 @@ def test_virial_pairs_vs_fp64(gb, dtype, nf, nloc, nall, nnei):
         assert bool(((av[k].double().view(nall, 9) - row).abs() <= w * (m + 8) * u * rmag).all())
         chain = 32 if dtype == torch.float32 else 64 + int(ok.sum().item()) ** 0.5
         assert bool(((v[k].double() - term.sum(0)).abs() <= w * chain * u * mag.sum(0)).all())
+
+
+def test_workspace_by_call(gb):
+    """The padded atomic virial rows are asked for by the FP32 virial alone: a
+    force call takes a workspace without them, the virial call refuses it."""
+    import ctypes
+
+    L = __import__("dpmd_public_gb300._lib", fromlist=["x"])
+    lib = L.load()
+    n, nnei = 10, 4
+    full = int(lib.gbdp_prod_workspace_bytes(1, n, n, nnei, 0))
+    part = full - -(-48 * n // 256) * 256
+    z = lambda k: torch.zeros(k, device=DEV)
+    f, v, av = z(3 * n), z(9), z(9 * n)
+    net, dr, rij = z(n * nnei * 4), z(n * nnei * 12), z(n * nnei * 3)
+    nl = torch.zeros(n * nnei, device=DEV, dtype=torch.int32)
+    ws = torch.empty(full, device=DEV, dtype=torch.uint8)
+    st = torch.cuda.current_stream().cuda_stream
+    P = lambda t: t.data_ptr()
+    force = lambda b: lib.gbdp_prod_force_a_f32(P(f), P(net), P(dr), P(nl), n, n, nnei, 1, 0, P(ws),
+                                                ctypes.c_size_t(b), st)
+    virial = lambda b: lib.gbdp_prod_virial_a_f32(P(v), P(av), P(net), P(dr), P(rij), P(nl), n, n,
+                                                  nnei, 1, 0, P(ws), ctypes.c_size_t(b), st)
+    assert force(full) == 0 and virial(full) == 0 and force(part) == 0
+    assert virial(part) != 0 and force(255) != 0
+    torch.cuda.synchronize()
