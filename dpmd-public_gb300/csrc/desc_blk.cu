@@ -718,7 +718,7 @@ __global__ void __launch_bounds__(W * 32, bwd_warps(U) / W)
 // / 52.2, 1800: 58.3 / 54.2.  The forward takes eight warps an atom while all
 // CTAs are resident at once, four an SM (eight / four, us: 48 atoms 14.5 /
 // 19.0, 192: 14.5 / 18.6, 600: 16.6 / 20.5, 1200: 27.0 / 24.5; the backward,
-// two CTAs an SM, gains at most 2 us up to 300 atoms and loses 6 at 600).
+// two CTAs an SM, would gain under 1 us up to 300 atoms and lose 6 at 600).
 constexpr int kShareFwd8 = 152 * 4, kShareFwd = 152 * 10, kShareBwd = 152 * 8;
 
 // shared memory of a launch, and the smallest shared-memory carveout that
