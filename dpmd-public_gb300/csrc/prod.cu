@@ -66,10 +66,16 @@ __device__ __forceinline__ void scatter9(double* p, const double* t) {
 #pragma unroll
   for (int q = 0; q < 9; ++q) atomicAdd(p + q, t[q]);
 }
-// FP32: p is a padded 12-float row, 16-byte aligned
+// FP32: p is a padded 12-float row, on a 16-byte boundary where the workspace
+// starts on one (the same for every row of a launch), else on an 8-byte one
 __device__ __forceinline__ void scatter9(float* p, const float* t) {
-  red4(p, t[0], t[1], t[2], t[3]);
-  red4(p + 4, t[4], t[5], t[6], t[7]);
+  if ((reinterpret_cast<uintptr_t>(p) & 15) == 0) {
+    red4(p, t[0], t[1], t[2], t[3]);
+    red4(p + 4, t[4], t[5], t[6], t[7]);
+  } else {
+#pragma unroll
+    for (int q = 0; q < 8; q += 2) red2(p + q, t[q], t[q + 1]);
+  }
   atomicAdd(p + 8, t[8]);
 }
 
@@ -798,6 +804,14 @@ void launch_vir_reduce(T* virial, const T* atom_virial, const ProdWs& w, int nal
   k_vir_final<T><<<nframes, 32, 0, st>>>(virial, w.vir_part, nchunk);
 }
 
+// The virials' accumulators are doubles; FP32 atomic forces are added 16 bytes
+// at a time.
+template <typename T>
+bool ws_aligned(const void* ws, int det, bool force, bool virial) {
+  const int a = sizeof(T) == 4 && !det && force ? 16 : virial ? 8 : 4;
+  return ((uintptr_t)ws & (a - 1)) == 0;
+}
+
 template <typename T>
 int prod_launch(T* force, T* virial, T* atom_virial, const T* net, const T* dR, const T* rij,
                 const int* nlist, int nloc, int nall, int nnei, int nframes, int det, void* ws,
@@ -825,6 +839,8 @@ int prod_launch(T* force, T* virial, T* atom_virial, const T* net, const T* dR, 
                "prod_force/virial: null input pointer");
   GBDP_REQUIRE(((uintptr_t)net & 15) == 0 && ((uintptr_t)dR & 15) == 0,
                "prod_force/virial: net_deriv and env_deriv must be 16-byte aligned");
+  GBDP_REQUIRE(ws_aligned<T>(ws, det, force, atom_virial),
+               "prod_force/virial: workspace not 8-byte aligned (16 for FP32 atomic forces)");
   // every word of `virial` is written below, so it needs no zero fill
   if (!det) {
     launch_atomic<T>(force, virial, atom_virial, w, net, dR, rij, nlist, nloc, nall, nnei, nframes,
@@ -873,6 +889,7 @@ int prod_virial_impl(T* virial, T* atom_virial, const T* net, const T* dR, const
   GBDP_REQUIRE(net && dR && rij && nlist, "prod_virial_a: null input pointer");
   GBDP_REQUIRE(((uintptr_t)net & 15) == 0 && ((uintptr_t)dR & 15) == 0,
                "prod_virial_a: net_deriv and env_deriv must be 16-byte aligned");
+  GBDP_REQUIRE(ws_aligned<T>(ws, det, false, true), "prod_virial_a: workspace not 8-byte aligned");
   if (!det) {
     launch_atomic<T>(nullptr, virial, atom_virial, w, net, dR, rij, nlist, nloc, nall, nnei,
                      nframes, st);

@@ -315,7 +315,8 @@ GBDP_API int gbdp_env_status(const void* workspace, gbdp_stream stream);
  * neighbour list (bitwise reproducible); 0 scatters with atomics (FP32
  * forces accumulate in 16-byte padded rows of the workspace, one vector
  * reduction a pair, then are compacted into `force`, FP32 atomic virials in
- * 48-byte rows; the workspace size below includes those rows).
+ * 48-byte rows; the workspace size below includes those rows).  The workspace
+ * is 8-byte aligned for a virial, 16-byte for FP32 atomic forces.
  * ---------------------------------------------------------------------- */
 GBDP_API size_t gbdp_prod_workspace_bytes(int nframes, int nloc, int nall, int nnei, int deterministic);
 GBDP_API int gbdp_prod_force_a_f32(float* force, const float* net_deriv, const float* env_deriv,

@@ -165,3 +165,22 @@ def test_descriptor_split_needs_row_scales(gb):
     rc = lib.gbdp_se_a_descriptor_fwd_split_f32(fake, fake, fake, None, fake, fake, None, tabs,
                                                info, 2, sel, 1, 8, 100, 16, None)
     assert rc != 0 and b"D_rscale" in lib.gbdp_last_error()
+
+
+def test_prod_workspace_alignment_is_checked(gb):
+    """A workspace that the atomic additions could not address is refused
+    before anything is launched: FP32 forces 16 bytes, virials 8 (the pointers
+    are only looked at)."""
+    lib = gb._lib.load()
+    p = 1 << 20
+    for sfx in ("f32", "f64"):
+        force = getattr(lib, "gbdp_prod_force_a_" + sfx)
+        virial = getattr(lib, "gbdp_prod_virial_a_" + sfx)
+        both = getattr(lib, "gbdp_prod_force_virial_a_" + sfx)
+        bad = [virial(p, p, p, p, p, p, 2, 2, 4, 1, 0, p + 4, ctypes.c_size_t(1 << 20), None),
+               both(p, p, p, p, p, p, p, 2, 2, 4, 1, 0, p + 4, ctypes.c_size_t(1 << 20), None)]
+        if sfx == "f32":
+            bad.append(force(p, p, p, p, 2, 2, 4, 1, 0, p + 8, ctypes.c_size_t(1 << 20), None))
+        for rc in bad:
+            assert rc == gb._lib.GBDP_OK - 1
+        assert b"aligned" in lib.gbdp_last_error()

@@ -259,3 +259,37 @@ def test_workspace_by_call(gb):
     assert force(full) == 0 and virial(full) == 0 and force(part) == 0
     assert virial(part) != 0 and force(255) != 0
     torch.cuda.synchronize()
+
+
+@pytest.mark.parametrize("off", [0, 8])
+def test_virial_workspace_on_8_bytes(gb, off):
+    """The FP32 virial takes a workspace on any 8-byte boundary: the padded
+    rows, 16-byte aligned or not, against FP64.  Bounds as in
+    test_virial_pairs_vs_fp64."""
+    import ctypes
+
+    L = __import__("dpmd_public_gb300._lib", fromlist=["x"])
+    lib = L.load()
+    n, nall, nnei = 37, 50, 138
+    g = torch.Generator(device=DEV).manual_seed(17)
+    R = lambda *s: torch.randn(*s, generator=g, device=DEV)
+    net, dr, rij = R(n * nnei, 4), R(n * nnei, 12), R(n * nnei, 3)
+    nl = torch.randint(0, nall, (n * nnei,), generator=g, device=DEV, dtype=torch.int32)
+    v, av = torch.full((9,), 7.0, device=DEV), torch.full((nall, 9), 7.0, device=DEV)
+    wsb = int(lib.gbdp_prod_workspace_bytes(1, n, nall, nnei, 0))
+    ws = torch.empty(wsb + 16, device=DEV, dtype=torch.uint8)
+    assert ws.data_ptr() % 16 == 0
+    P = lambda t: t.data_ptr()
+    L.check(lib.gbdp_prod_virial_a_f32(P(v), P(av), P(net), P(dr), P(rij), P(nl), n, nall, nnei, 1,
+                                       0, P(ws) + off, ctypes.c_size_t(wsb),
+                                       torch.cuda.current_stream().cuda_stream), "virial")
+    torch.cuda.synchronize()
+    G, D, X = net.double()[:, :, None], dr.double().view(-1, 4, 3), rij.double()[:, None]
+    term, mag = (((a * b).sum(1)[:, :, None] * c).view(-1, 9)
+                 for a, b, c in ((G, D, X), (G.abs(), D.abs(), X.abs())))
+    z = lambda w: torch.zeros(nall, w, dtype=torch.float64, device=DEV)
+    row, rmag = (z(9).index_add_(0, nl.long(), q) for q in (term, mag))
+    m = z(1).index_add_(0, nl.long(), torch.ones_like(term[:, :1]))
+    u = 2.0 ** -24
+    assert bool(((av.double() - row).abs() <= (m + 8) * u * rmag).all())
+    assert bool(((v.double() - term.sum(0)).abs() <= 32 * u * mag.sum(0)).all())
