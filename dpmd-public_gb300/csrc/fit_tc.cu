@@ -1761,6 +1761,8 @@ extern "C" int gbdp_fitting_tc_f32(float* e, float* dE_dD, const void* D_hi, con
                "fit_tc: workspace %zu < %zu", workspace_bytes,
                gbdp_fitting_tc_workspace_bytes((int)rows));
   if (rows == 0) return GBDP_OK;
+  // (k_fit_f1 and k_fit_mid address it in 16-byte pieces, the others by TMA)
+  GBDP_REQUIRE(((uintptr_t)workspace & 15) == 0, "fit_tc: workspace not 16-byte aligned");
   int rc = get_encode();
   if (rc) return rc;
   int* status = reinterpret_cast<int*>(static_cast<char*>(workspace) + ws.bytes);

@@ -539,6 +539,7 @@ GBDP_API int gbdp_se_a_descriptor_bwd_blk_f32(
  *                  of these from the parameters)
  *   b[l]; idt[l] (NULL for layer 0); w_out [240]; b_out on the host.
  * Outputs: e [rows] per-row energy (0 on padding rows), dE_dD [rows, 1600].
+ * workspace: 16-byte aligned.
  * ---------------------------------------------------------------------- */
 typedef struct gbdp_fit_tc_net {
   const void* w_hi[3];

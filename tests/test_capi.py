@@ -184,3 +184,24 @@ def test_prod_workspace_alignment_is_checked(gb):
         for rc in bad:
             assert rc == gb._lib.GBDP_OK - 1
         assert b"aligned" in lib.gbdp_last_error()
+
+
+def test_fitting_workspace_alignment_is_checked(gb):
+    """A workspace off a 16-byte boundary is refused before any launch, for few
+    and for many row blocks (no pointer is followed: only device ones are
+    given)."""
+    L = gb._lib
+    lib = L.load()
+    p = 1 << 20
+    net = L.FitTcNet()
+    for k in ("w_hi", "w_lo", "wt_hi", "wt_lo", "cs_fwd", "cs_bwd", "b", "idt"):
+        setattr(net, k, (ctypes.c_void_p * 3)(p, p, p))
+    net.w_out = p
+    net.act_scale = (ctypes.c_float * 5)(1, 1, 1, 1, 1)
+    for rows in (128, 31 * 128):
+        n, off = (ctypes.c_int * 1)(rows), (ctypes.c_int * 2)(0, rows)
+        for a in (4, 8):
+            rc = lib.gbdp_fitting_tc_f32(p, p, p, p, p, 1, n, off, ctypes.byref(net), p + a,
+                                         ctypes.c_size_t(1 << 30), None)
+            assert rc == L.GBDP_OK - 1
+            assert b"workspace not 16-byte aligned" in lib.gbdp_last_error()
