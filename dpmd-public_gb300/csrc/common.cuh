@@ -45,7 +45,12 @@ int cuda_status(cudaError_t e, const char* where);
 // its first access to global memory and grid_release after it (a later
 // kernel that reads constant data ahead of its own wait may then rely on
 // everything before this kernel).  Any other predecessor on the stream, and
-// any other successor, is ordered as usual.  A step on 192 atoms from host
+// any other successor, is ordered as usual.  What the kernel directly before
+// writes is thus not constant while this one runs: it is read by plain loads
+// after the wait, never through the read-only path (no const __restrict__
+// parameter, __ldg or ld.global.nc, which promise the opposite and which no
+// fence holds back), in asm as volatile with a memory clobber.  What was
+// written before that kernel began is complete when this one begins.  A step on 192 atoms from host
 // to host, 18 kernels and 6 memsets: 204 us; so launched, clears in the chain
 // and the short kernels at its end merged: 183.  12,288 atoms captured in a
 // graph: 487 and 476.

@@ -153,7 +153,7 @@ __global__ void __launch_bounds__(W * 32, 32 / W)
           const int j = b + lane;
           bool hit = false;
           if (j < ns) {
-            const float4 e = ld_stream4(e0 + 4 * j);
+            const float4 e = ld_prev4(e0 + 4 * j);
             hit = e.x == last && e.y == 0.f && e.z == 0.f && e.w == 0.f;
             float x = e.x;
             const int idx = locate_row(inf, x);
@@ -443,8 +443,8 @@ __global__ void __launch_bounds__(W * 32, bwd_warps(U) / W)
     for (int u = 0; u < NX; ++u) {
       const int k = tid + NT * u;
       if (k < M)
-        v[u] = make_float4(ld_stream(Xi + k), ld_stream(Xi + M + k), ld_stream(Xi + 2 * M + k),
-                           ld_stream(Xi + 3 * M + k));
+        v[u] = make_float4(ld_prev(Xi + k), ld_prev(Xi + M + k), ld_prev(Xi + 2 * M + k),
+                           ld_prev(Xi + 3 * M + k));
     }
 #pragma unroll
     for (int u = 0; u < NX; ++u) {
@@ -485,7 +485,7 @@ __global__ void __launch_bounds__(W * 32, bwd_warps(U) / W)
 #pragma unroll
       for (int u = 0; u < BT; ++u) {
         const int k = (it0 + S * u) * 8 + (lane >> 2);
-        g[u] = k < M ? ld_stream4(g_i + k * kAxis + 4 * q) : make_float4(0.f, 0.f, 0.f, 0.f);
+        g[u] = k < M ? ld_prev4(g_i + k * kAxis + 4 * q) : make_float4(0.f, 0.f, 0.f, 0.f);
       }
 #pragma unroll
       for (int u = 0; u < BT; ++u) {
@@ -571,7 +571,7 @@ __global__ void __launch_bounds__(W * 32, bwd_warps(U) / W)
         if (S > 1 && chunk % S != w) continue;
         const int j = b + lane;
         if (j < nv) {
-          const float4 e = ld_stream4(p.em + ((size_t)i * nnei + s0 + j) * 4);
+          const float4 e = ld_prev4(p.em + ((size_t)i * nnei + s0 + j) * 4);
           float x = e.x;
           const int idx = locate_row(inf, x);
           sl.em[s0 + j] = e;

@@ -198,9 +198,9 @@ struct Skip {
 // rows of section [s0, s0 + ns) of an atom to evaluate: 1 + the last row that
 // differs from the section's last row, plus one for the equal rest (NaN
 // differs from itself: every row)
-__device__ __forceinline__ int distinct_rows(const float4* __restrict__ em, int ns) {
+__device__ __forceinline__ int distinct_rows(const float4* em, int ns) {
   const int lane = threadIdx.x & 31;
-  const float4 last = __ldg(em + ns - 1);
+  const float4 last = em[ns - 1];
   int top = -1;
   for (int b = 0; b < ns; b += 128) {
     bool ne[4];
@@ -209,7 +209,7 @@ __device__ __forceinline__ int distinct_rows(const float4* __restrict__ em, int 
       const int j = b + 32 * u + lane;
       ne[u] = false;
       if (j < ns) {
-        const float4 e = __ldg(em + j);
+        const float4 e = em[j];
         ne[u] = !(e.x == last.x && e.y == last.y && e.z == last.z && e.w == last.w);
       }
     }
@@ -392,7 +392,7 @@ __global__ void __launch_bounds__(128, 3) k_emb_fwd(const __grid_constant__ EmbA
           acc[c][0] = acc[c][1] = make_float2(0.f, 0.f);
         };
         float4 e = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (32 * s0 + lane < neff) e = __ldg(em + 32 * s0 + lane);
+        if (32 * s0 + lane < neff) e = em[32 * s0 + lane];
         for (int sl = 0; sl < nsl && alive; ++sl) {
           rsm[r] = e;
           // ---- layer 1 (FP32): h1 = tanh(s w1 + b1), all N1 columns per thread
@@ -404,7 +404,7 @@ __global__ void __launch_bounds__(128, 3) k_emb_fwd(const __grid_constant__ EmbA
           st_half<N1, 1>(atile, r, h1);
           // the next slab's row
           const int jn = 32 * (ss * (sl + 1) + s0) + lane;
-          e = jn < neff ? __ldg(em + jn) : make_float4(0.f, 0.f, 0.f, 0.f);
+          e = jn < neff ? em[jn] : make_float4(0.f, 0.f, 0.f, 0.f);
           fence_proxy_async_smem();
           tc_fence_before();
           __syncthreads();
@@ -708,7 +708,7 @@ __host__ __device__ constexpr size_t dx16_warp_bytes(int N3) {
   return (size_t)N3 * 16 + ((size_t)N3 * 17 * 4 + 15) / 16 * 16;  // X^T, then dD (odd row stride)
 }
 __global__ void __launch_bounds__(kDxWarps * 32)
-    k_emb_dx16(float* __restrict__ dxs, const float* __restrict__ dD, const float* __restrict__ X,
+    k_emb_dx16(float* __restrict__ dxs, const float* dD, const float* X,
                const int* __restrict__ drow, int nloc, int N3, float inv_nnei) {
   grid_wait();
   grid_release();
@@ -928,13 +928,13 @@ __global__ void __launch_bounds__(128, 2) k_emb_bwd(const __grid_constant__ EmbB
         const uint32_t b2 = smem_addr(slot + kNetB2), b3 = smem_addr(slot + kNetB3);
         const uint32_t b3t = smem_addr(slot + kNetB3T), b2t = smem_addr(slot + kNetB2T);
         float4 en = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (32 * s0 + lane < neff) en = __ldg(em + 32 * s0 + lane);
+        if (32 * s0 + lane < neff) en = em[32 * s0 + lane];
         for (int sl = 0; sl < nsl && alive; ++sl) {
           const int slab = ss * sl + s0;
           const int j = 32 * slab + lane;
           const bool live = j < neff;
           const float4 e = en;
-          en = j + 32 * ss < neff ? __ldg(em + j + 32 * ss) : make_float4(0.f, 0.f, 0.f, 0.f);
+          en = j + 32 * ss < neff ? em[j + 32 * ss] : make_float4(0.f, 0.f, 0.f, 0.f);
           // ---- forward recompute: layer 1, MMA 2, epilogue 2, MMA 3
           float h1[N1];
   #pragma unroll

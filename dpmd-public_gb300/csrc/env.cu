@@ -240,10 +240,10 @@ __device__ __forceinline__ void ext_cell_source(const gbdp_nbr_frame& g, int e, 
 
 // ---------------------------------------------------------- k_cell_scan --
 __global__ void k_cell_scan(const gbdp_nbr_frame* __restrict__ fr,
-                            const int* __restrict__ cell_count, int* __restrict__ cell_start,
+                            const int* cell_count, int* __restrict__ cell_start,
                             int* __restrict__ ext_start, int* __restrict__ ext_cnt,
                             int* __restrict__ ghost_start, int* __restrict__ ext_nall,
-                            int* __restrict__ status, const int* __restrict__ sub_count,
+                            int* __restrict__ status, const int* sub_count,
                             int* __restrict__ ext_sub) {
   __shared__ int warp_tot[32];
   grid_wait();
@@ -305,7 +305,7 @@ __global__ void k_cell_scan(const gbdp_nbr_frame* __restrict__ fr,
 __global__ void k_cell_bucket(int nloc_total, const gbdp_nbr_frame* __restrict__ fr,
                               const int* __restrict__ atom_frame,
                               const int* __restrict__ atom_cell,
-                              const int* __restrict__ cell_start, int* __restrict__ cell_fill,
+                              const int* cell_start, int* __restrict__ cell_fill,
                               int* __restrict__ bucket) {
   grid_wait();
   grid_release();
@@ -323,7 +323,7 @@ __global__ void k_cell_rank(int nloc_total, const gbdp_nbr_frame* __restrict__ f
                             const int* __restrict__ atom_frame,
                             const int* __restrict__ atom_cell,
                             const int* __restrict__ cell_start,
-                            const int* __restrict__ cell_count, const int* __restrict__ bucket,
+                            const int* __restrict__ cell_count, const int* bucket,
                             int* __restrict__ cell_atoms, const int* __restrict__ atom_sub,
                             int* __restrict__ atom_xpos) {
   grid_wait();
@@ -354,12 +354,12 @@ template <typename T>
 __global__ void k_ghost_fill(const gbdp_nbr_frame* __restrict__ fr, int nframes,
                              int next_cell_total, const int* __restrict__ cell_start,
                              const int* __restrict__ cell_count,
-                             const int* __restrict__ cell_atoms,
+                             const int* cell_atoms,
                              const int* __restrict__ ext_start,
                              const int* __restrict__ ghost_start, T* __restrict__ ext_coord,
                              int* __restrict__ ext_type, int* __restrict__ ext_map,
                              typename XsOf<T>::type* __restrict__ xs,
-                             const int* __restrict__ atom_xpos) {
+                             const int* atom_xpos) {
   grid_wait();
   grid_release();
   const int ew = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -724,8 +724,8 @@ __global__ void __launch_bounds__(kEnvWarps * 32)
     k_nlist_env(int nloc_total, const gbdp_nbr_frame* __restrict__ fr,
                 const int* __restrict__ atom_frame, const int* __restrict__ atom_cell,
                 const int* __restrict__ atom_sub, const int* __restrict__ ext_sub,
-                const typename XsOf<T>::type* __restrict__ xs, const T* __restrict__ ext_coord,
-                const int* __restrict__ ext_map, const int* __restrict__ atype,
+                const typename XsOf<T>::type* xs, const T* ext_coord,
+                const int* ext_map, const int* __restrict__ atype,
                 const T* __restrict__ avg, const T* __restrict__ stdv, SecInfo si, float rc2f,
                 T rmin, T rmax, int max_cand, T* __restrict__ em, T* __restrict__ em_deriv,
                 T* __restrict__ rij, int* __restrict__ nlist, int* __restrict__ nlist_ext,
@@ -1041,8 +1041,8 @@ __host__ __device__ constexpr size_t nlist_ext_warp_bytes(int nnei_in, int nnei)
 
 template <typename T>
 __global__ void __launch_bounds__(kEnvWarps * 32)
-    k_nlist_env_ext(int nloc, int nall, int nnei_in, int nwork, const T* __restrict__ ext_coord,
-                    const int* __restrict__ ext_type, const int* __restrict__ nlist_in,
+    k_nlist_env_ext(int nloc, int nall, int nnei_in, int nwork, const T* ext_coord,
+                    const int* ext_type, const int* nlist_in,
                     const T* __restrict__ avg, const T* __restrict__ stdv, SecInfo si, T rcut,
                     T rmin, T rmax, T* __restrict__ em, T* __restrict__ em_deriv,
                     T* __restrict__ rij, int* __restrict__ nlist, int* __restrict__ status) {

@@ -1540,7 +1540,7 @@ struct TcRows {
   int ntypes;
 };
 
-__global__ void k_fit_tc_energy(float* __restrict__ e, const float* __restrict__ epart,
+__global__ void k_fit_tc_energy(float* __restrict__ e, const float* epart,
                                 int ntile_n, TcRows rw) {
   grid_wait();
   grid_release();

@@ -743,7 +743,7 @@ __global__ void k_fx_finish_inplace(double* __restrict__ buf, size_t n, int s) {
 }
 
 // both after the FP32 backward in one launch of the chain
-__global__ void k_fx_finish2(float* __restrict__ out, const long long* __restrict__ acc, size_t n,
+__global__ void k_fx_finish2(float* __restrict__ out, const long long* acc, size_t n,
                              int s, double* __restrict__ buf, size_t nb, int sb) {
   grid_wait();
   grid_release();
@@ -754,7 +754,7 @@ __global__ void k_fx_finish2(float* __restrict__ out, const long long* __restric
 
 // one row a lane (r, of a warp's 32 in a row)
 template <typename T>
-__device__ __forceinline__ void add_rows(double* E, const T* __restrict__ ae,
+__device__ __forceinline__ void add_rows(double* E, const T* ae,
                                          const int* __restrict__ frame_of_row, int r, int nrows,
                                          int det) {
   const int lane = threadIdx.x & 31;
@@ -790,7 +790,7 @@ constexpr int kEnergyRows = 2048, kEnergyThreads = 1024;
 
 template <typename T>
 __global__ void __launch_bounds__(kEnergyThreads) k_frame_energy_cta(
-    double* __restrict__ E, const T* __restrict__ ae, const int* __restrict__ frame_of_row,
+    double* __restrict__ E, const T* ae, const int* __restrict__ frame_of_row,
     int nrows, int nframes, int det) {
   grid_wait();
   grid_release();

@@ -124,6 +124,22 @@ __device__ __forceinline__ double ld_stream(const double* p) {
   return v;
 }
 
+// The same for data of the kernel launched directly before (dependent
+// launches): plain loads, after the wait.
+__device__ __forceinline__ float4 ld_prev4(const float* p) {
+  float4 v;
+  asm volatile("ld.global.L1::no_allocate.v4.f32 {%0, %1, %2, %3}, [%4];"
+               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+               : "l"(p)
+               : "memory");
+  return v;
+}
+__device__ __forceinline__ float ld_prev(const float* p) {
+  float v;
+  asm volatile("ld.global.L1::no_allocate.f32 %0, [%1];" : "=f"(v) : "l"(p) : "memory");
+  return v;
+}
+
 // a row of 4 values read twice by the same warp: first out of L1
 __device__ __forceinline__ float4 ld_first4(const float* p) {
   float4 v;

@@ -332,7 +332,7 @@ __global__ void __launch_bounds__(kVirThreads, kVirCtas<T>) k_virial_pairs(
 }
 
 // padded FP32 force rows [n][4] -> the output's [n][3]
-__global__ void k_force4_compact(float* __restrict__ force, const float4* __restrict__ f4,
+__global__ void k_force4_compact(float* __restrict__ force, const float4* f4,
                                  size_t n) {
   grid_wait();
   grid_release();
@@ -346,8 +346,8 @@ __global__ void k_force4_compact(float* __restrict__ force, const float4* __rest
 
 // padded FP32 atomic virial rows [n][12] -> the output's [n][9], and the
 // frame virials (n9 = 9 nframes values; vir may be null)
-__global__ void k_vir12_compact(float* __restrict__ av, const float* __restrict__ v12, size_t n,
-                                float* __restrict__ vir, const double* __restrict__ acc, int n9) {
+__global__ void k_vir12_compact(float* __restrict__ av, const float* v12, size_t n,
+                                float* __restrict__ vir, const double* acc, int n9) {
   grid_wait();
   grid_release();
   const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -358,7 +358,7 @@ __global__ void k_vir12_compact(float* __restrict__ av, const float* __restrict_
 }
 
 template <typename T>
-__global__ void k_vir_finish(T* __restrict__ virial, const double* __restrict__ acc, int n) {
+__global__ void k_vir_finish(T* __restrict__ virial, const double* acc, int n) {
   grid_wait();
   grid_release();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
