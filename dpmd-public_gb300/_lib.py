@@ -91,6 +91,7 @@ _SIGS = {
     "gbdp_fitting_tc_status": (_I, [_P, _I, _P]),
     "gbdp_set_autotune": (None, [_I]),
     "gbdp_autotune_report": (_I, [ctypes.c_char_p, _I]),
+    "gbdp_autotune_set": (_I, [_I] * 8),
     "gbdp_embed_tc_net_bytes": (_Z, []),
     "gbdp_embed_fwd_tc_bf16": (_I, [_P] * 8 + [_I, _P, _I, _P] + [_I] * 7 + [_P, _P]),
     "gbdp_embed_bwd_tc_bf16": (_I, [_P] * 8 + [_I, _P, _I, _P] + [_I] * 7 + [_P, _P]),

@@ -719,6 +719,8 @@ __global__ void __launch_bounds__(W * 32, bwd_warps(U) / W)
 // CTAs are resident at once, four an SM (eight / four, us: 48 atoms 14.5 /
 // 19.0, 192: 14.5 / 18.6, 600: 16.6 / 20.5, 1200: 27.0 / 24.5; the backward,
 // two CTAs an SM, would gain under 1 us up to 300 atoms and lose 6 at 600).
+// The line is on the number of atoms alone, never on the tuner's choice: an
+// atom's sums are grouped by the warps that share it.
 constexpr int kShareFwd8 = 152 * 4, kShareFwd = 152 * 10, kShareBwd = 152 * 8;
 
 // shared memory of a launch, and the smallest shared-memory carveout that
@@ -745,14 +747,14 @@ void launch_fwd(const DescFwdArgs& a, const TabSet<float>& ts, int nloc, int M, 
 template <int NS>
 void fwd_width(const DescFwdArgs& a, const TabSet<float>& ts, int nloc, int M, int W,
                cudaStream_t st) {
-  if (W == 1)
-    launch_fwd<NS, 1, 1>(a, ts, nloc, M, st);
-  else if (W == 2)
-    launch_fwd<NS, 2, 1>(a, ts, nloc, M, st);
-  else if (nloc <= kShareFwd8)
+  if (nloc <= kShareFwd8)
     launch_fwd<NS, 8, 8>(a, ts, nloc, M, st);
   else if (nloc < kShareFwd)
     launch_fwd<NS, 4, 4>(a, ts, nloc, M, st);
+  else if (W == 1)
+    launch_fwd<NS, 1, 1>(a, ts, nloc, M, st);
+  else if (W == 2)
+    launch_fwd<NS, 2, 1>(a, ts, nloc, M, st);
   else
     launch_fwd<NS, 4, 1>(a, ts, nloc, M, st);
 }
@@ -784,12 +786,12 @@ void launch_bwd(const DescBwdArgs& a, const TabSet<float>& ts, int nloc, int M, 
 template <int NK, int U>
 void bwd_width(const DescBwdArgs& a, const TabSet<float>& ts, int nloc, int M, int W,
                cudaStream_t st) {
-  if (W == 1)
+  if (nloc < kShareBwd)
+    launch_bwd<NK, 4, 4, U>(a, ts, nloc, M, st);
+  else if (W == 1)
     launch_bwd<NK, 1, 1, U>(a, ts, nloc, M, st);
   else if (W == 2)
     launch_bwd<NK, 2, 1, U>(a, ts, nloc, M, st);
-  else if (nloc < kShareBwd)
-    launch_bwd<NK, 4, 4, U>(a, ts, nloc, M, st);
   else
     launch_bwd<NK, 4, 1, U>(a, ts, nloc, M, st);
 }
@@ -809,6 +811,9 @@ __global__ void k_table_blocked(float* __restrict__ dst, const float* __restrict
 }
 
 }  // namespace
+
+int desc_fwd_share(int nloc) { return nloc <= kShareFwd8 ? 8 : nloc < kShareFwd ? 4 : 1; }
+int desc_bwd_share(int nloc) { return nloc < kShareBwd ? 4 : 1; }
 
 int desc_fwd_blk(const DescFwdArgs& a, const TabSet<float>& ts, int nloc, int M, int W,
                  cudaStream_t st) {

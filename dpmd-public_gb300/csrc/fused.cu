@@ -872,14 +872,19 @@ int make_tabset(TabSet<T>& ts, const T* const* tables, const T* infos, int ntype
 // so only the launch shape changes: a small batch fills more SMs with
 // smaller CTAs), bits 3-4 for the backward the neighbours in flight per
 // 16-lane group minus one (1 or 2: more loads in flight per warp against
-// fewer resident warps).  With autotuning on (gbdp_set_autotune), the first
-// call for a shape key (kernel, dtype, M, nnei, floor(log2 nloc)) that is
-// not under stream capture times every choice with CUDA events on the
-// caller's stream (three runs each, the minimum) and keeps the fastest;
-// later calls with that key use it.  The cache is the library's only mutable
-// global state and sits behind a mutex.  Without a tuned entry the choice is
-// 4 warps, 1 neighbour in flight.
-enum { kTuneFwd = 0, kTuneBwd = 1 };
+// fewer resident warps).  Every choice gives the same bits: how many warps
+// share an atom, which regroups sums, is the kernels' rule on nloc and no
+// choice (on blocked tables; where they share one the code's warps have no
+// meaning).  With autotuning on (gbdp_set_autotune), the first call for a
+// shape key (kernel, dtype, M, nnei, floor(log2 nloc), warps that share an
+// atom) that is not under stream capture times every choice with CUDA events
+// on the caller's stream (three runs each, the minimum) and keeps the
+// fastest; later calls with that key use it.  The cache is the library's only
+// mutable global state and sits behind a mutex.  Without a tuned entry the
+// choice is 4 warps and 1 neighbour in flight (on blocked tables 2 with few
+// atoms).
+enum { kTuneFwd = 0, kTuneBwd = 1, kTuneFwdBlk = 2, kTuneBwdBlk = 3 };
+inline bool tune_is_bwd(int kid) { return kid & 1; }
 constexpr int kTuneMax = 6;
 constexpr int kTuneFwdCodes[3] = {1, 2, 4};
 constexpr int kTuneBwdCodes[6] = {1, 2, 4, 1 | 8, 2 | 8, 4 | 8};
@@ -891,13 +896,17 @@ struct TuneEntry {
   float ms[kTuneMax];
 };
 std::mutex g_tune_mu;
-std::map<std::array<int, 5>, TuneEntry> g_tune;
+using TuneKey = std::array<int, 6>;
+std::map<TuneKey, TuneEntry> g_tune;
 std::atomic<int> g_autotune{0};
 
-std::array<int, 5> tune_key(int kid, int tsize, int M, int nnei, int nloc) {
+TuneKey tune_key(int kid, int tsize, int M, int nnei, int nloc) {
   int lg = 0;
   while (lg < 30 && (1 << (lg + 1)) <= nloc) ++lg;
-  return {kid, tsize, M, nnei, lg};
+  const int share = kid == kTuneFwdBlk   ? desc_fwd_share(nloc)
+                    : kid == kTuneBwdBlk ? desc_bwd_share(nloc)
+                                         : 1;
+  return {kid, tsize, M, nnei, lg, share};
 }
 
 int tuned_code(int kid, int tsize, int M, int nnei, int nloc, int dflt) {
@@ -920,9 +929,9 @@ int tune_run(int kid, int tsize, int M, int nnei, int nloc, cudaStream_t st, F&&
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     if (!have && cudaStreamIsCapturing(st, &cs) == cudaSuccess &&
         cs == cudaStreamCaptureStatusNone) {
-      const int* codes = kid == kTuneFwd ? kTuneFwdCodes : kTuneBwdCodes;
+      const int* codes = tune_is_bwd(kid) ? kTuneBwdCodes : kTuneFwdCodes;
       // the FP64 backward is built for one neighbour in flight only
-      const int nc = kid == kTuneFwd ? 3 : (tsize == 4 ? 6 : 3);
+      const int nc = tune_is_bwd(kid) && tsize == 4 ? 6 : 3;
       cudaEvent_t e0, e1;
       cudaEventCreate(&e0);
       cudaEventCreate(&e1);
@@ -1322,8 +1331,8 @@ extern "C" int gbdp_se_a_descriptor_fwd_blk_f32(
                "se_a descriptor fwd: nnei %d needs %zu bytes of shared memory", nnei,
                (size_t)kFWarps * wb);
   const DescFwdArgs a{X, D, D_lo, D_rscale, em, atype, d_row};
-  return tune_run(kTuneFwd, 4, M, nnei, nloc, st, [&](int w) -> int {
-    if (w == 0) w = tuned_code(kTuneFwd, 4, M, nnei, nloc, kFWarps);
+  return tune_run(kTuneFwdBlk, 4, M, nnei, nloc, st, [&](int w) -> int {
+    if (w == 0) w = tuned_code(kTuneFwdBlk, 4, M, nnei, nloc, kFWarps);
     return desc_fwd_blk(a, ts, nloc, M, code_warps(w), st);
   });
 }
@@ -1362,7 +1371,7 @@ extern "C" int gbdp_se_a_descriptor_bwd_blk_f32(
                       dE_dD,   d_row,      em,       nlist_ext,
                       ext_coord, ext_map,  atype,    inv_std,
                       {atom_frame, frame_atom_off, frame_ext_off}, rcut_smth, rcut};
-  return tune_run(kTuneBwd, 4, M, nnei, nloc, st, [&](int w) -> int {
+  return tune_run(kTuneBwdBlk, 4, M, nnei, nloc, st, [&](int w) -> int {
     const size_t nf = 3 * (size_t)nloc, nv = 9 * (size_t)nframes;
     if (force_fx && nloc > 0)
       clear_dep<long long>(force_fx, nf, reinterpret_cast<long long*>(virial_acc), nv, st);
@@ -1376,7 +1385,7 @@ extern "C" int gbdp_se_a_descriptor_bwd_blk_f32(
     // untuned: two neighbours in flight while the SMs hold less than four
     // atoms each (192 atoms: 27.6 against 31.7 us; 768 atoms: 41.9 / 39.9)
     if (w == 0)
-      w = tuned_code(kTuneBwd, 4, M, nnei, nloc, nloc < 152 * 4 ? kBWarps | 8 : kBWarps);
+      w = tuned_code(kTuneBwdBlk, 4, M, nnei, nloc, nloc < 152 * 4 ? kBWarps | 8 : kBWarps);
     int rc = desc_bwd_blk(a, ts, nloc, M, code_warps(w), code_nbrs(w), st);
     if (rc) return rc;
     if (force_fx) {
@@ -1391,6 +1400,23 @@ extern "C" int gbdp_se_a_descriptor_bwd_blk_f32(
 
 extern "C" void gbdp_set_autotune(int on) { g_autotune.store(on ? 1 : 0); }
 
+extern "C" int gbdp_autotune_set(int backward, int blocked, int fp64, int last_layer_size, int nnei,
+                                 int nloc, int warps, int nbrs) {
+  GBDP_REQUIRE(!(blocked && fp64), "autotune_set: blocked tables are FP32");
+  GBDP_REQUIRE(warps == 0 || warps == 1 || warps == 2 || warps == 4,
+               "autotune_set: %d warps (1, 2 or 4; 0: none kept)", warps);
+  GBDP_REQUIRE(nbrs == 1 || (nbrs == 2 && backward && !fp64),
+               "autotune_set: %d neighbours in flight (FP32 backward: 1 or 2; else 1)", nbrs);
+  const int kid = (blocked ? kTuneFwdBlk : kTuneFwd) + (backward ? 1 : 0);
+  const TuneKey key = tune_key(kid, fp64 ? 8 : 4, last_layer_size, nnei, nloc);
+  std::lock_guard<std::mutex> lk(g_tune_mu);
+  if (warps == 0)
+    g_tune.erase(key);
+  else
+    g_tune[key] = TuneEntry{warps | (nbrs - 1) << 3, 0, {}};
+  return GBDP_OK;
+}
+
 extern "C" int gbdp_autotune_report(char* buf, int len) {
   std::string out;
   {
@@ -1400,9 +1426,12 @@ extern "C" int gbdp_autotune_report(char* buf, int len) {
       const auto& k = kv.first;
       const auto& e = kv.second;
       int w = snprintf(line, sizeof(line), "%s f%d M=%d nnei=%d nloc=2^%d warps=%d",
-                       k[0] == kTuneFwd ? "se_a_descriptor_fwd" : "se_a_descriptor_bwd",
+                       tune_is_bwd(k[0]) ? "se_a_descriptor_bwd" : "se_a_descriptor_fwd",
                        8 * k[1], k[2], k[3], k[4], code_warps(e.code));
-      if (k[0] == kTuneBwd) w += snprintf(line + w, sizeof(line) - w, " nbrs=%d", code_nbrs(e.code));
+      if (tune_is_bwd(k[0]))
+        w += snprintf(line + w, sizeof(line) - w, " nbrs=%d", code_nbrs(e.code));
+      if (k[0] >= kTuneFwdBlk)
+        w += snprintf(line + w, sizeof(line) - w, " table=blocked share=%d", k[5]);
       w += snprintf(line + w, sizeof(line) - w, " ms=");
       for (int c = 0; c < e.n; ++c)
         w += snprintf(line + w, sizeof(line) - w, c ? ",%.4f" : "%.4f", e.ms[c]);

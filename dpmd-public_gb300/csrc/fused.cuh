@@ -218,8 +218,11 @@ __device__ __forceinline__ int filled_prefix(const int* __restrict__ nl, int ns)
 }
 
 
-// desc_blk.cu: the descriptor on blocked tables, warps per CTA W (1, 2, 4;
-// 4 warps share an atom in small batches), U neighbours in flight per group
+// desc_blk.cu: the descriptor on blocked tables, warps per CTA W (1, 2 or 4,
+// one atom each; without meaning where warps share an atom), U neighbours in
+// flight per group; and the warps that share an atom, by the number of atoms
+int desc_fwd_share(int nloc);
+int desc_bwd_share(int nloc);
 int desc_fwd_blk(const DescFwdArgs& a, const TabSet<float>& ts, int nloc, int M, int W,
                  cudaStream_t st);
 int desc_bwd_blk(const DescBwdArgs& a, const TabSet<float>& ts, int nloc, int M, int W, int U,

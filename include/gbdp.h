@@ -576,20 +576,28 @@ GBDP_API void gbdp_fitting_tc_set_persistent_min_tiles(int tiles_per_sm);
 
 /* ---- launch-shape autotuning ----------------------------------------------
  * The fused descriptor kernels (the gbdp_se_a_descriptor_ fwd and bwd entry
- * points) run 1, 2 or 4 warps per CTA, one centre atom each (on blocked
- * tables the 4 warps share an atom in small batches), and the FP32 backward 1
- * or 2 neighbours in flight per 16-lane group.  With autotuning on, the first
- * call for a shape key
- * (kernel, dtype, last_layer_size, nnei, floor(log2 nloc)) that is not under
- * stream capture times every choice on the caller's stream (it synchronises
- * that stream) and keeps the fastest in a mutex-guarded cache; later calls
- * with that key, captured or not, use it.  Off by default (4 per CTA, 1
- * neighbour in flight).
+ * points) run 1, 2 or 4 warps per CTA, one centre atom each, and the FP32
+ * backward 1 or 2 neighbours in flight per 16-lane group; every choice gives
+ * the same bits (on blocked tables 4 or 8 warps share an atom in small
+ * batches: by the number of atoms, whatever the choice).  With autotuning on,
+ * the first call for a shape key (kernel, dtype, last_layer_size, nnei,
+ * floor(log2 nloc), warps that share an atom) that is not under stream
+ * capture times every choice on the caller's stream (it synchronises that
+ * stream) and keeps the fastest in a mutex-guarded cache; later calls with
+ * that key, captured or not, use it.  Off by default (4 per CTA, 1 neighbour
+ * in flight, on blocked tables 2 with few atoms).
  * No reference counterpart.  gbdp_autotune_report writes one line per tuned
  * key into buf (NUL-terminated, at most len bytes) and returns the full
  * length. */
 GBDP_API void gbdp_set_autotune(int on);
 GBDP_API int gbdp_autotune_report(char* buf, int len);
+/* Keep a launch shape without timing it, as if the tuner had chosen it for the
+ * key that the sizes fall in (a choice carried over from an earlier run); in
+ * use whether autotuning is on or not.  backward, blocked, fp64: the kernel
+ * (0 / 1 each; blocked tables are FP32); warps 1, 2 or 4, or 0 to keep none;
+ * nbrs 1, or 2 for the FP32 backward. */
+GBDP_API int gbdp_autotune_set(int backward, int blocked, int fp64, int last_layer_size, int nnei,
+                               int nloc, int warps, int nbrs);
 
 /* ---- uncompressed embedding net on the tensor cores (BF16) ----------------
  * Replaces the plain-form embedding of DescrptBlockSeA.forward

@@ -307,3 +307,31 @@ def test_frame_energies(mods, dtype, det, nrows, nframes):
     mag = z.clone().index_add_(0, f.clamp_min(0).long(), ae.double().abs() * ok)
     bound = 2 * nrows * 2.0 ** -53 * mag + (nrows * 2.0 ** -31 if det else 0.0)
     assert bool(((E - ref).abs() <= bound).all())
+
+
+@pytest.mark.parametrize("n", [4, 7, 8])
+def test_tuned_shapes_give_the_same_bits(mods, built, n):
+    """The launch shapes the tuner chooses between (1, 2 or 4 warps, 1 or 2
+    neighbours in flight) give a deterministic step the same bits, where warps
+    share an atom (192 and 1,029 atoms) and where each has its own (1,536): the
+    tuner's choice is by time, so results that depended on it
+    would not be the same on every run."""
+    L = __import__("dpmd_public_gb300._lib", fromlist=["x"])
+    se_a, mdl, water = mods
+    cfg, m64, m32 = built
+    lib = L.load()
+    frame = water.water_frame(n, 3.105 * n, 40 + n)
+    b = m32.batch([frame[1]], frame[2][None])
+    coord = torch.tensor(frame[0], dtype=torch.float32, device=DEV)
+    key = (0, cfg.neuron[-1], sum(cfg.sel), b.nloc)
+    run = lambda: tuple(x.clone() for x in m32.step_fused(b, coord, deterministic=True))
+    ref = run()
+    try:
+        for bwd, warps, nbrs in [(0, 1, 1), (0, 2, 1), (0, 4, 1)] + [
+                (1, w, u) for w in (1, 2, 4) for u in (1, 2)]:
+            L.check(lib.gbdp_autotune_set(bwd, 1, *key, warps, nbrs), "autotune_set")
+            for x, y in zip(run(), ref):
+                assert torch.equal(x, y), (bwd, warps, nbrs)
+    finally:
+        for bwd in (0, 1):
+            L.check(lib.gbdp_autotune_set(bwd, 1, *key, 0, 1), "autotune_set")
