@@ -125,6 +125,76 @@ def _check(gb, mods, mols, width, sel):
             assert err <= tol * float(ref.abs().max()), (form, name, err)
 
 
+@pytest.mark.parametrize("mols", [13, 202, 203, 405, 406, 506, 507, 666])
+@pytest.mark.parametrize("width,sel", [(100, (46, 92)), (48, (64, 31))])
+def test_launch_shapes(gb, mods, mols, width, sel):
+    """Every shape the tuner may keep, not only the untuned one, on both sides
+    of the sharing lines (608, 1,520; backward 1,216 atoms): the bounds of the
+    module, and D's FP16 parts against the FP32 form's D (a row's parts hold
+    22 bits under a scale bounded by |X_k| |X_a|, 2^-21 of it)."""
+    L = gb._lib
+    lib = L.load()
+    m64, m32 = _models(mods, width, sel)
+    b, em = _env_rows(mods, m32, mols)
+    X, D = _descriptor(gb, m64, torch.float64, "f64", b, em.double(), None)
+    dD = torch.randn(D.shape, generator=torch.Generator(device=DEV).manual_seed(mols), device=DEV)
+    F, V = _descriptor(gb, m64, torch.float64, "f64", b, em.double(), dD.double(),
+                       X.float().double())
+    key = (0, width, sum(sel), b.nloc)
+    near = lambda got, ref, tol: float((got.double() - ref).abs().max()) <= tol * float(ref.abs().max())
+    try:
+        for warps in (1, 2, 4):
+            L.check(lib.gbdp_autotune_set(0, 1, *key, warps, 1), "autotune_set")
+            x, d = _descriptor(gb, m32, torch.float32, "blk", b, em, None)
+            assert near(x, X, 2e-5) and near(d, D, 2e-5), warps
+            xs, hi, lo, rs = _split_fwd(gb, m32, b, em)
+            assert torch.equal(xs, x), warps
+            nk = x.double().square().sum(1)
+            bound = (nk.amax(1) * nk[:, :16].amax(1)).sqrt()[:, None]
+            got = (hi.double() + lo.double()) * rs.double()[:, None]
+            assert bool(((got - d.double()).abs() <= 2.0 ** -21 * bound).all()), warps
+            for nbrs in (1, 2):
+                L.check(lib.gbdp_autotune_set(1, 1, *key, warps, nbrs), "autotune_set")
+                f, v = _descriptor(gb, m32, torch.float32, "blk", b, em, dD, X.float())
+                assert near(f, F, 2e-5) and near(v, V, 2e-4), (warps, nbrs)
+    finally:
+        for bwd in (0, 1):
+            L.check(lib.gbdp_autotune_set(bwd, 1, *key, 0, 1), "autotune_set")
+
+
+def _split_fwd(gb, m, b, em):
+    """X and D's FP16 parts with the rows' inverse scales."""
+    import ctypes
+
+    L = gb._lib
+    cfg = m.cfg
+    P = lambda t: ctypes.c_void_p(t.data_ptr())
+    M = cfg.neuron[-1]
+    tabs = [m._blocked(t) for t in m.tables]
+    ptrs = (ctypes.c_void_p * len(tabs))(*[t.data_ptr() for t in tabs])
+    X = torch.empty(b.nloc, 4, M, device=DEV)
+    hi, lo = (torch.empty(b.nloc, M * 16, dtype=torch.float16, device=DEV) for _ in range(2))
+    rs = torch.empty(b.nloc, device=DEV)
+    L.check(L.load().gbdp_se_a_descriptor_fwd_blk_f32(
+        P(X), P(hi), P(lo), P(rs), P(em), P(b.atype), None, ptrs, m._tab_infos, cfg.ntypes, m._sel_c,
+        int(cfg.type_one_side), b.nloc, M, 16,
+        ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)), "fwd")
+    torch.cuda.synchronize()
+    return X, hi, lo, rs
+
+
+def _env_rows(mods, m32, mols):
+    """A batch of one frame of mols molecules and its env rows."""
+    water = mods[2]
+    side = int(np.ceil(mols ** (1 / 3) - 1e-9))
+    box = float(np.float32(water.water_box_for(max(mols, 8))))
+    c, t, _ = water.water_frame(side, box, 40 + mols, n_mol=mols)
+    b = m32.batch([t], np.diag([box] * 3).reshape(1, 9))
+    m32.step_fused(b, torch.tensor(c.astype(np.float32), device=DEV))
+    assert b.status() == 0
+    return b, b.env.em
+
+
 @pytest.mark.parametrize("m", [100, 37, 16, 128])
 def test_table_to_blocked_layout(gb, m):
     L = gb._lib
