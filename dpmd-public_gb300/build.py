@@ -72,6 +72,8 @@ def _compile(src: str, extra: list[str]) -> str:
 
 
 def _torch_flags():
+    import sysconfig
+
     import torch
     import torch.utils.cpp_extension as ce
 
@@ -80,7 +82,8 @@ def _torch_flags():
     abi = int(torch._C._GLIBCXX_USE_CXX11_ABI)
     cuda_inc = os.path.join(os.path.dirname(os.path.dirname(nvcc())), "include")
     return (["-O2", "-std=c++17", "-fPIC", f"-D_GLIBCXX_USE_CXX11_ABI={abi}",
-             "-I" + os.path.join(ROOT, "include"), "-I" + cuda_inc] + inc,
+             "-I" + os.path.join(ROOT, "include"), "-I" + cuda_inc,
+             "-I" + sysconfig.get_paths()["include"]] + inc,
             [f"-L{lib}", f"-Wl,-rpath,{lib}", "-ltorch", "-ltorch_cpu", "-lc10", "-lc10_cuda"])
 
 
@@ -125,6 +128,8 @@ def build(force: bool = False, verbose_ptxas: bool = False) -> str:
         out = TORCH_LIBS[src]
         cmd = [shutil.which("g++") or "g++", "-shared", "-o", out + ".tmp", obj, "-L" + HERE,
                "-Wl,-rpath,$ORIGIN", "-lgbdp"] + ldflags
+        if src.endswith("torch_native.cpp"):  # raises Python exceptions
+            cmd.append("-ltorch_python")
         r = subprocess.run(cmd, capture_output=True, text=True)
         if r.returncode != 0:
             raise RuntimeError(f"link of {os.path.basename(out)} failed:\n{r.stderr[-4000:]}")

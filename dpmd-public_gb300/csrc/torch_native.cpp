@@ -13,12 +13,26 @@
 //   env_mat       ProdEnvMatA, internal periodic mode
 //                 (source/op/tf/prod_env_mat_multi_device.cc:11-28)
 //   env_mat_nlist prod_env_mat_a from an external list (forward_lower)
+#include <torch/csrc/Exceptions.h>
+
 #include <memory>
 #include <mutex>
 
 #include "torch_tab.h"
 
 namespace {
+
+// Library errors reach Python as the operators' own exception type (GbdpError)
+// from the backward passes too, where no Python frame of ops.py stands between
+// the autograd engine and the caller.
+PyObject* g_error_type = nullptr;
+
+struct LibraryError : public torch::PyTorchError {
+  explicit LibraryError(const std::string& m) : torch::PyTorchError(m) {}
+  PyObject* python_type() override { return g_error_type ? g_error_type : PyExc_RuntimeError; }
+};
+
+void raise_library_error(const std::string& msg) { throw LibraryError(msg); }
 
 gbdp_stream stream_of(const Tensor& t) { return cur_stream(t); }
 
@@ -396,6 +410,12 @@ std::vector<Tensor> env_mat_nlist(const Tensor& coord_in, const Tensor& type_in,
 }
 
 }  // namespace
+
+// (called once at load, with the GIL held; the class is kept for good)
+extern "C" void gbdp_native_set_error_type(PyObject* type) {
+  Py_XINCREF(type);
+  g_error_type = type;
+}
 
 TORCH_LIBRARY(gbdp_native, m) {
   m.def("tab(Tensor table, Tensor table_info, Tensor em_x, Tensor em, int last_layer_size) -> Tensor",

@@ -13,6 +13,11 @@
 
 namespace {
 
+void raise_library_error(const std::string& msg) {
+  TORCH_CHECK(false, msg);
+  std::terminate();  // not reached
+}
+
 std::vector<Tensor> tabulate_fusion_se_a(const Tensor& table, const Tensor& table_info,
                                          const Tensor& em_x, const Tensor& em,
                                          int64_t last_layer_size) {

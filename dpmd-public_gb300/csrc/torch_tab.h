@@ -22,8 +22,13 @@ using torch::Tensor;
 using torch::autograd::AutogradContext;
 using torch::autograd::variable_list;
 
+// raises the library's last error as the including side's exception
+[[noreturn]] void raise_library_error(const std::string& msg);
+
 void check_rc(int rc, const char* what) {
-  TORCH_CHECK(rc == GBDP_OK, what, " failed (", rc, "): ", gbdp_last_error());
+  if (rc != GBDP_OK)
+    raise_library_error(std::string(what) + " failed (" + std::to_string(rc) +
+                        "): " + gbdp_last_error());
 }
 
 void need_cuda(const Tensor& t) {

@@ -134,7 +134,7 @@ def tabulate_grad_grad(table, table_info, em_x, em, dz_dem_x, dz_dem, last_layer
 # csrc/torch_native.cpp: the operators below and their autograd in C++ (the
 # host work of a small training batch went into Python autograd functions and
 # ctypes calls).  Its errors are raised as GbdpError where they are the
-# library's own (a status code or a device status).
+# library's own (a status code or a device status), in backward passes too.
 NATIVE_PATH = os.path.join(os.path.dirname(os.path.abspath(__file__)), "libgbdp_torch_gb300.so")
 _native = None
 
@@ -148,6 +148,9 @@ def native():
             raise RuntimeError(
                 f"{NATIVE_PATH} is missing: build it with __graft_entry__.build()")
         torch.ops.load_library(NATIVE_PATH)
+        set_type = ctypes.PyDLL(NATIVE_PATH).gbdp_native_set_error_type
+        set_type.argtypes, set_type.restype = [ctypes.py_object], None
+        set_type(L.GbdpError)
         ns = torch.ops.gbdp_native
         _native = types.SimpleNamespace(**{n: getattr(ns, n).default for n in (
             "tab", "prod_force", "prod_virial", "env_mat", "env_mat_nlist")})

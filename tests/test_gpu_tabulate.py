@@ -229,3 +229,31 @@ def test_split_edges_vs_oracle(oracle, dtype, nloc, nnei, M, shift):
     close(gm, rm)
     close(ops.tabulate_grad_grad(tab, inf, ex, emt, dev(dzx), dev(dzm), M),
           oracle.tabulate_fusion_se_a_grad_grad(table, info, x1, em, dzx, dzm, M))
+
+
+@pytest.mark.parametrize("second", [False, True])
+def test_library_error_in_backward(gb, second):
+    """A library error inside a backward pass (here a table that came back
+    from a saved-tensor hook on a 4-byte boundary, which the library refuses)
+    is the operators' own exception, as in the forward."""
+    on = [False]
+
+    def unpack(t):
+        if not (on[0] and t.dim() == 2 and t.is_cuda and t.shape[1] == 48):
+            return t
+        raw = torch.empty(t.numel() + 1, device=t.device)
+        return raw[1:].view(t.shape).copy_(t)
+
+    info = torch.tensor([0.0, 1.0, 2.0, 0.5, 0.5, 5.0], dtype=torch.float64)
+    table = torch.rand(8, 48, device=DEV)
+    em_x = torch.rand(12, 1, device=DEV, requires_grad=True)
+    em = torch.rand(3, 4, 4, device=DEV, requires_grad=True)
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: t, unpack):
+        y = torch.ops.deepmd.tabulate_fusion_se_a(table, info, em_x, em, 8)[0]
+        if second:
+            dy = torch.ones_like(y, requires_grad=True)
+            gx, gm = torch.autograd.grad(y, (em_x, em), dy, create_graph=True)
+            y = gx.sum() + gm.sum()
+    on[0] = True
+    with pytest.raises(gb._lib.GbdpError, match="tabulate_fusion_se_a_grad.* failed"):
+        torch.autograd.grad(y.sum(), dy if second else em)
