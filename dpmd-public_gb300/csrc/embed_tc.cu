@@ -491,7 +491,10 @@ __global__ void __launch_bounds__(128, 3) k_emb_fwd(const __grid_constant__ EmbA
           // the last row of slab `s` for itself and the equal rest
           auto add_rest = [&](int s, const float4* R, const float* gt) {
             const float4 q = R[neff - 32 * s - 1];
-            const bool one = q.y == 0.f && q.z == 0.f && q.w == 0.f;  // a padding row
+            // a padding row; 0 G is no 0 where G is not finite
+            bool one = q.y == 0.f && q.z == 0.f && q.w == 0.f;
+#pragma unroll
+            for (int c = 0; c < NOWN; ++c) one = one && fabsf(gt[c]) < INFINITY;
             int at = (warp & 1) * sel + neff - 1;
             for (int left = sel - neff + 1; left > 0;) {
               if ((at & 127) == 0)

@@ -198,3 +198,33 @@ def test_one_and_two_units_a_block_agree(setup, one_side):
         got.append([q[:123].clone() for q in parts])
     for a, c in zip(*got):
         assert torch.equal(a, c)
+
+
+@pytest.mark.parametrize("mols", [2, 210])
+def test_nan_in_a_padding_row(setup, mols):
+    """A row with s = NaN (0 / 0 in the statistics) makes every component of
+    its atom's X NaN, its zero components too (0 NaN = NaN in the sum over the
+    rows), also where the row is padding and evaluated for the equal rest; other
+    atoms keep their bits."""
+    se_a, water, cfg, m64, _, _ = setup
+    mdl = importlib.import_module("dpmd_public_gb300.model")
+    m = se_a.SeAModel(cfg, mdl.init_params(cfg, 3), m64.davg.cpu().numpy(),
+                      m64.dstd.cpu().numpy(), DEV, torch.float32)
+    n = 3 * mols
+    b = m.batch([np.tile(np.array([0, 1, 1], np.int32), mols)], np.diag([60.0] * 3).reshape(1, 9))
+    b.ensure_plain_tc(m)
+    g = torch.Generator(device=DEV).manual_seed(2)
+    em = torch.randn(n, cfg.nnei, 4, generator=g, device=DEV)
+    for t in range(2):
+        em[:, cfg.sec[t] + 20:cfg.sec[t + 1]] = torch.tensor([-0.4, 0., 0., 0.], device=DEV)
+    m.embed_tc_forward(b, em)
+    clean = b.X.clone()
+    bad = torch.zeros(n, dtype=torch.bool, device=DEV)
+    for i, t in ((0, 0), (4, 1), (n - 1, 0)):
+        em[i, cfg.sec[t + 1] - 1, 0] = float("nan")
+        bad[i] = True
+    m.embed_tc_forward(b, em)
+    torch.cuda.synchronize()
+    assert int(b.emb_status.item()) == 0
+    assert bool(torch.isnan(b.X[bad]).all())
+    assert torch.equal(b.X[~bad], clean[~bad])
