@@ -361,13 +361,16 @@ __global__ void __launch_bounds__(kTabWarps * 32)
       const Row4<T> e = s_row[warp][jj];
       T p[4] = {T(0), T(0), T(0), T(0)}, px = T(0);
       // no branch between the steps, so that several steps' loads are in
-      // flight: a lane past the width reads the last output against dy = 0
+      // flight: a lane past the width (in the last step) reads the last
+      // output and drops it (against dy = 0 alone an infinite one would be
+      // 0 inf = NaN)
 #pragma unroll
       for (int q = 0; q < NK; ++q) {
         Coef<T> c;
         load_coef<T>(c, row, min(t + G * q, Mc - 1));
         T v, d;
         tab_val_slope(c, xp, v, d);
+        if (q == NK - 1 && t + G * q >= Mc) v = d = T(0);
 #pragma unroll
         for (int m = 0; m < 4; ++m) p[m] += v * g[q][m];
         px += d * dot4(e, g[q]);
@@ -547,33 +550,23 @@ int tab_grad(T* dy_dem_x, T* dy_dem, const T* table, const T* info, const T* em_
 #define GBDP_TAB_GRAD(N)                                                                       \
   launch_grad<T, N>(st, dy_dem_x, dy_dem, table, ti, em_x, em, dy, nloc, nnei, M, kb,          \
                     is_sorted != 0, vec)
-    if constexpr (G == 16) {
-      switch (nk) {
-        case 1: GBDP_TAB_GRAD(1); break;
-        case 2: GBDP_TAB_GRAD(2); break;
-        case 3: GBDP_TAB_GRAD(3); break;
-        case 4: GBDP_TAB_GRAD(4); break;
-        case 5: GBDP_TAB_GRAD(5); break;
-        case 6: GBDP_TAB_GRAD(6); break;
-        case 7: GBDP_TAB_GRAD(7); break;
-        default: GBDP_TAB_GRAD(8); break;
-      }
-    } else {
-      if (nk <= 2)
-        GBDP_TAB_GRAD(2);
-      else if (nk <= 4)
-        GBDP_TAB_GRAD(4);
-      else if (nk <= 6)
-        GBDP_TAB_GRAD(6);
-      else if (nk <= 8)
-        GBDP_TAB_GRAD(8);
-      else if (nk <= 10)
-        GBDP_TAB_GRAD(10);
-      else if (nk <= 13)
-        GBDP_TAB_GRAD(13);
-      else
-        GBDP_TAB_GRAD(16);
+#define GBDP_TAB_GRAD2(N)              \
+  case N: GBDP_TAB_GRAD(N); break;     \
+  case N + 1: GBDP_TAB_GRAD(N + 1); break;
+    switch (nk) {
+      GBDP_TAB_GRAD2(1)
+      GBDP_TAB_GRAD2(3)
+      GBDP_TAB_GRAD2(5)
+      GBDP_TAB_GRAD2(7)
+      default:
+        if constexpr (G == 8) switch (nk) {
+            GBDP_TAB_GRAD2(9)
+            GBDP_TAB_GRAD2(11)
+            GBDP_TAB_GRAD2(13)
+            GBDP_TAB_GRAD2(15)
+          }
     }
+#undef GBDP_TAB_GRAD2
 #undef GBDP_TAB_GRAD
   }
   GBDP_CHECK_LAUNCH("tabulate_fusion_se_a_grad");

@@ -257,3 +257,23 @@ def test_library_error_in_backward(gb, second):
     on[0] = True
     with pytest.raises(gb._lib.GbdpError, match="tabulate_fusion_se_a_grad.* failed"):
         torch.autograd.grad(y.sum(), dy if second else em)
+
+
+@pytest.mark.parametrize("dtype", [torch.float64, torch.float32])
+@pytest.mark.parametrize("M", [1, 33, 82, 90, 100, 129])
+def test_infinite_output_in_the_gradient(dtype, M):
+    """An output whose polynomial is infinite (its constant term; the last one,
+    which the lanes past the width read as well) gives dy_dem an infinity of
+    dy's sign, not NaN, and leaves dy_dem_x finite."""
+    ops = __import__("dpmd_public_gb300.ops", fromlist=["x"])
+    g = torch.Generator(device=DEV).manual_seed(M)
+    R = lambda *s: torch.rand(*s, generator=g, device=DEV, dtype=dtype)
+    info = torch.tensor([0.0, 1.0, 2.0, 0.25, 0.25, 5.0], dtype=torch.float64)
+    table = R(8, M * 6)
+    table[:, 6 * (M - 1)] = float("inf")
+    nloc, nnei = 5, 7
+    dy = R(nloc, 4, M) - 0.5
+    gx, gm = ops.tabulate_grad(table, info, R(nloc * nnei, 1) * 2, R(nloc, nnei, 4), dy)
+    assert bool(torch.isfinite(gx).all())
+    sign = torch.sign(dy[:, None, :, M - 1]).expand(nloc, nnei, 4)
+    assert torch.equal(gm, sign * float("inf"))
