@@ -67,6 +67,7 @@ _SIGS = {
     "gbdp_nbr_plan_make": (_I, [_P, _P, _I, _P, _P, _F, _I]),
     "gbdp_env_workspace_bytes": (_Z, [_P, _I]),
     "gbdp_env_status": (_I, [_P, _P]),
+    "gbdp_prod_call_workspace_bytes": (_Z, [_I] * 7),
     "gbdp_prod_workspace_bytes": (_Z, [_I, _I, _I, _I, _I]),
     "gbdp_prod_env_mat_a_noalloc_f32": (_I, [_P] * 16 + [_F, _P, _I, _P]),
     "gbdp_fitting_workspace_bytes": (_Z, [_I, _P, _I, _P]),

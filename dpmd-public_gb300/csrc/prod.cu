@@ -865,6 +865,12 @@ extern "C" size_t gbdp_prod_workspace_bytes(int nframes, int nloc, int nall, int
   return carve_prod(nullptr, nframes, nloc, nall, nnei, deterministic).bytes;
 }
 
+extern "C" size_t gbdp_prod_call_workspace_bytes(int nframes, int nloc, int nall, int nnei,
+                                                 int deterministic, int fp64, int virial) {
+  const ProdWs w = carve_prod(nullptr, nframes, nloc, nall, nnei, deterministic);
+  return deterministic || (virial && !fp64) ? w.bytes : w.no_vir12;
+}
+
 namespace gbdp {
 namespace {
 // The virial op alone (no force output requested by the caller): the atomic

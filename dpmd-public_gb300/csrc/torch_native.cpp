@@ -77,7 +77,7 @@ Tensor force_call(const Tensor& net_in, const Tensor& der_in, const Tensor& nl_i
   const Tensor net = net_in.contiguous(), der = der_in.to(net.scalar_type()).contiguous(),
                nl = i32(nl_in);
   Tensor force = torch::empty({d.nf, (int64_t)d.nall * 3}, net.options());
-  const size_t wsb = gbdp_prod_workspace_bytes(d.nf, d.nloc, d.nall, d.nnei, 0);
+  const size_t wsb = gbdp_prod_call_workspace_bytes(d.nf, d.nloc, d.nall, d.nnei, 0, f64, 0);
   const Tensor ws = bytes(wsb, net);
   int rc;
   if (f64)
@@ -105,7 +105,7 @@ std::vector<Tensor> virial_call(const Tensor& net_in, const Tensor& der_in, cons
                rij = rij_in.to(st).contiguous(), nl = i32(nl_in);
   Tensor vir = torch::empty({d.nf, 9}, net.options());
   Tensor av = torch::empty({d.nf, (int64_t)d.nall * 9}, net.options());
-  const size_t wsb = gbdp_prod_workspace_bytes(d.nf, d.nloc, d.nall, d.nnei, 0);
+  const size_t wsb = gbdp_prod_call_workspace_bytes(d.nf, d.nloc, d.nall, d.nnei, 0, f64, 1);
   const Tensor ws = bytes(wsb, net);
   int rc;
   if (f64)

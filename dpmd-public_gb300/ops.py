@@ -359,7 +359,8 @@ def prod_force_se_a_impl(net_deriv, in_deriv, nlist, natoms, n_a_sel: int, n_r_s
     dt = net_deriv.dtype
     force = torch.empty((nf, nall * 3), dtype=dt, device=net_deriv.device)
     lib = L.load()
-    wsb = int(lib.gbdp_prod_workspace_bytes(nf, nloc, nall, nnei, int(deterministic)))
+    wsb = int(lib.gbdp_prod_call_workspace_bytes(nf, nloc, nall, nnei, int(deterministic),
+                                                 int(dt == torch.float64), 0))
     ws = torch.empty(max(wsb, 1), dtype=torch.uint8, device=net_deriv.device)
     fn = getattr(lib, f"gbdp_prod_force_a_{L.sfx(dt)}")
     net_deriv = net_deriv.contiguous()
@@ -381,7 +382,8 @@ def prod_virial_se_a_impl(net_deriv, in_deriv, rij, nlist, natoms, n_a_sel: int,
     virial = torch.empty((nf, 9), dtype=dt, device=net_deriv.device)
     atom_virial = torch.empty((nf, nall * 9), dtype=dt, device=net_deriv.device)
     lib = L.load()
-    wsb = int(lib.gbdp_prod_workspace_bytes(nf, nloc, nall, nnei, int(deterministic)))
+    wsb = int(lib.gbdp_prod_call_workspace_bytes(nf, nloc, nall, nnei, int(deterministic),
+                                                 int(dt == torch.float64), 1))
     ws = torch.empty(max(wsb, 1), dtype=torch.uint8, device=net_deriv.device)
     fn = getattr(lib, f"gbdp_prod_virial_a_{L.sfx(dt)}")
     net_deriv = net_deriv.contiguous()
@@ -409,7 +411,8 @@ def prod_force_virial_se_a_impl(net_deriv, in_deriv, rij, nlist, natoms, n_a_sel
     virial = torch.empty((nf, 9), dtype=dt, device=dev)
     atom_virial = torch.empty((nf, nall * 9), dtype=dt, device=dev)
     lib = L.load()
-    wsb = int(lib.gbdp_prod_workspace_bytes(nf, nloc, nall, nnei, int(deterministic)))
+    wsb = int(lib.gbdp_prod_call_workspace_bytes(nf, nloc, nall, nnei, int(deterministic),
+                                                 int(dt == torch.float64), 1))
     ws = torch.empty(max(wsb, 1), dtype=torch.uint8, device=dev)
     fn = getattr(lib, f"gbdp_prod_force_virial_a_{L.sfx(dt)}")
     net_deriv = net_deriv.contiguous()

@@ -319,6 +319,10 @@ GBDP_API int gbdp_env_status(const void* workspace, gbdp_stream stream);
  * is 8-byte aligned for a virial, 16-byte for FP32 atomic forces.
  * ---------------------------------------------------------------------- */
 GBDP_API size_t gbdp_prod_workspace_bytes(int nframes, int nloc, int nall, int nnei, int deterministic);
+/* What one call needs of it: without the padded virial rows for a force alone
+ * (virial 0) and in FP64. */
+GBDP_API size_t gbdp_prod_call_workspace_bytes(int nframes, int nloc, int nall, int nnei,
+                                               int deterministic, int fp64, int virial);
 GBDP_API int gbdp_prod_force_a_f32(float* force, const float* net_deriv, const float* env_deriv,
                           const int* nlist, int nloc, int nall, int nnei, int nframes,
                           int deterministic, void* workspace, size_t workspace_bytes,

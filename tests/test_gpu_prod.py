@@ -293,3 +293,33 @@ def test_virial_workspace_on_8_bytes(gb, off):
     u = 2.0 ** -24
     assert bool(((av.double() - row).abs() <= (m + 8) * u * rmag).all())
     assert bool(((v.double() - term.sum(0)).abs() <= 32 * u * mag.sum(0)).all())
+
+
+@pytest.mark.parametrize("dtype,virial", [(torch.float32, False), (torch.float64, False),
+                                          (torch.float64, True)])
+def test_workspace_of_a_call(dtype, virial):
+    """Calls that have no padded virial rows allocate no room for them: beside
+    its outputs a force call, and any FP64 call, takes 16 bytes an atom and
+    the frame's accumulator (blocks of the allocator: 2 MiB pieces)."""
+    n, nnei = 200_000, 1
+    z = lambda k: torch.zeros(1, k, device=DEV, dtype=dtype)
+    nl = torch.zeros(1, n * nnei, device=DEV, dtype=torch.int32)
+    natoms = torch.tensor([n, n, 0, 0], dtype=torch.int32)
+    net, dr, rij = z(n * nnei * 4), z(n * nnei * 12), z(n * nnei * 3)
+    ops = __import__("dpmd_public_gb300.ops", fromlist=["x"])
+    out_bytes = (9 if virial else 3) * n * net.element_size()
+    for form in ("op", "impl"):
+        if virial:
+            call = (lambda: torch.ops.deepmd.prod_virial_se_a(net, dr, rij, nl, natoms, nnei, 0)) \
+                if form == "op" else \
+                (lambda: ops.prod_virial_se_a_impl(net, dr, rij, nl, natoms, nnei, 0))
+        else:
+            call = (lambda: torch.ops.deepmd.prod_force_se_a(net, dr, nl, natoms, nnei, 0)) \
+                if form == "op" else \
+                (lambda: ops.prod_force_se_a_impl(net, dr, nl, natoms, nnei, 0))
+        torch.cuda.synchronize()
+        base = torch.cuda.memory_allocated()
+        torch.cuda.reset_peak_memory_stats()
+        call()
+        torch.cuda.synchronize()
+        assert torch.cuda.max_memory_allocated() - base <= out_bytes + 16 * n + (2 << 20), form
