@@ -194,3 +194,81 @@ def test_captured_step_retries_after_overflow(gb):
     E2, F2, V2 = m.step_fused(b2, torch.tensor(c, dtype=torch.float32, device=DEV))
     torch.cuda.synchronize()
     assert torch.equal(F, F2.cpu())
+
+
+# ---- torch.ops.deepmd.prod_env_mat_a: plans kept by the native operator part
+
+def _op_env(frame, avg, std, dtype=torch.float64):
+    c, t, b = frame
+    n = len(t)
+    T = lambda a, d=dtype: torch.tensor(np.asarray(a), dtype=d, device=DEV)
+    natoms = torch.tensor([n, n, int((t == 0).sum()), int((t == 1).sum())], dtype=torch.int32)
+    return torch.ops.deepmd.prod_env_mat_a(
+        T(c.reshape(1, -1)), T(t.reshape(1, -1), torch.int32), natoms, T(b.reshape(1, 9)),
+        torch.zeros(6, dtype=torch.int32), T(avg), T(std), 6.0, 6.0, 0.5, SEL, [0, 0])
+
+
+def _check_op(oracle, out, frame, avg, std):
+    c, t, b = frame
+    em, emd, rij, nl = oracle.prod_env_mat_a_pbc(c, t, b, avg, std, 6.0, 0.5, SEL, cell_list=True)
+    np.testing.assert_array_equal(out[3][0].cpu().numpy(), nl)
+    np.testing.assert_allclose(out[0][0].cpu().numpy(), em, atol=1e-12, rtol=1e-12)
+
+
+def test_operator_grows_and_keeps_the_capacity(oracle):
+    """About 900 candidates a centre against the default 512: the operator
+    doubles its plan's capacity and runs again; a second call with the same
+    box starts from the grown capacity; both give the reference's list."""
+    frame = _lattice(10, 1.0, seed=5)
+    avg, std = _stats()
+    for _ in range(2):
+        _check_op(oracle, _op_env(frame, avg, std), frame, avg, std)
+
+
+def test_operator_at_the_capacity_limit(gb):
+    """Some 4,190 candidates a centre, above the limit of 4,096: an error that
+    says so, not a truncated list; a later call is served as usual."""
+    avg, std = _stats()
+    for _ in range(2):
+        with pytest.raises(gb._lib.GbdpError, match="candidate overflow.* at max_cand 4096"):
+            _op_env(_lattice(21, 0.6, seed=6), avg, std)
+    out = _op_env(_lattice(8, 2.5, seed=7), avg, std)
+    assert bool((out[3] >= 0).any())
+
+
+def test_operator_over_many_boxes(oracle):
+    """More boxes than plans are kept, twice over: every list is its own."""
+    water = __import__("dpmd_public_gb300.water", fromlist=["x"])
+    avg, std = _stats()
+    frames = [water.water_frame(2, 6.2 + 0.11 * k, 60 + k) for k in range(20)]
+    for frame in frames + frames:
+        _check_op(oracle, _op_env(frame, avg, std), frame, avg, std)
+
+
+def test_operator_from_two_threads(oracle):
+    """Two threads on two streams over one box, so over one plan: each gets the
+    lists of its own coordinates."""
+    import threading
+
+    water = __import__("dpmd_public_gb300.water", fromlist=["x"])
+    avg, std = _stats()
+    frames = [water.water_frame(8, 24.84, 90 + k) for k in range(2)]
+    ref = [[x.clone() for x in _op_env(f, avg, std)] for f in frames]
+    torch.cuda.synchronize()
+    bad = []
+
+    def work(k):
+        with torch.cuda.stream(torch.cuda.Stream()):
+            for _ in range(25):
+                out = _op_env(frames[k], avg, std)
+                if not all(torch.equal(a, b) for a, b in zip(out, ref[k])):
+                    bad.append(k)
+
+    threads = [threading.Thread(target=work, args=(k,)) for k in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not bad
+    for k in range(2):
+        _check_op(oracle, ref[k], frames[k], avg, std)
