@@ -184,7 +184,8 @@ def autotune_report() -> list[str]:
     """One line per tuned shape key: kernel, dtype, sizes, the chosen warps
     per CTA (and for the backward the neighbours in flight per 16-lane group)
     and the measured milliseconds of every choice (forward: 1, 2, 4 warps;
-    backward: 1, 2, 4 warps at 1 neighbour, then at 2).""" 
+    backward: 1, 2, 4 warps at 1 neighbour, then at 2; none for a choice kept
+    by gbdp_autotune_set)."""
     lib = load()
     n = lib.gbdp_autotune_report(None, 0)
     buf = ctypes.create_string_buffer(n + 1)

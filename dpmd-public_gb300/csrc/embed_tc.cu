@@ -705,7 +705,9 @@ __global__ void k_emb_dx(float* __restrict__ dxs, const float* __restrict__ dD,
 
 // The same for 16 axis columns (same sums in the same order, the same bits:
 // dX is rounded to BF16 operands later), a warp per atom: the row of dD by
-// coalesced 16-byte loads, 26 atoms in flight per SM instead of a CTA each (6,141 atoms: 70 -> 26 us).
+// coalesced 16-byte loads, 24 atoms in flight per SM (six CTAs by shared
+// memory, 33.6 KB each at 100 columns) instead of a CTA each (6,141 atoms: 70
+// -> 26 us).
 constexpr int kDxWarps = 4;
 __host__ __device__ constexpr size_t dx16_warp_bytes(int N3) {
   return (size_t)N3 * 16 + ((size_t)N3 * 17 * 4 + 15) / 16 * 16;  // X^T, then dD (odd row stride)

@@ -27,9 +27,10 @@
 // epilogue applies the layer's activation (forward) or gradient chain
 // (backward) and writes the next GEMM's A operand already split, so the
 // whole per-type fitting net (deepmd/pt/model/task/fitting.py:734-899,
-// layer semantics deepmd/dpmodel/utils/network.py) is six layers, from 30 row
-// blocks on in three launches (k_fit_f1; k_fit_mid for F2, F3, B3 and B2;
-// k_fit_b1), below in six of k_fit_tc (narrow tiles):
+// layer semantics deepmd/dpmodel/utils/network.py) is six layers, above 30 row
+// blocks in three launches (k_fit_f1; k_fit_mid for F2, F3, B3 and B2;
+// k_fit_b1), up to there in five of k_fit_tc (narrow tiles) and B1 (k_fit_tc
+// up to 4 row blocks, k_fit_b1 above):
 //   F1  T1 = tanh(D W1 + b1)                    -> H1 = T1 (split)
 //   F2  T2 = tanh(H1 W2 + b2), H2 = T2 idt2 + T1 (split)
 //   F3  T3 = tanh(H2 W3 + b3), H3 = T3 idt3 + H2, e += H3 w_out,
@@ -54,7 +55,10 @@ namespace {
 constexpr int TBM = 128, TBK = 64;     // a k-block: 64 FP16 = one 128-byte swizzle row
 constexpr int A_TILE = TBM * TBK * 2;  // 16 KiB
 
-// Tile configurations of the per-tile kernel k_fit_tc:
+// Wide tile configurations of the per-tile kernel k_fit_tc.  On a GPU of 152
+// SMs they and k_fit_pers run only where
+// gbdp_fitting_tc_set_persistent_min_tiles was given a value other than its
+// default: one launch a layer at every size, to compare the fused form with.
 //   CfgLongK   F1 (K 1600): 128 x 128 tiles (two N tiles, the second
 //              holding columns 128-239 and 16 zero-filled ones that the
 //              epilogue skips), 3 stages, 3 main accumulators, one CTA per
@@ -71,8 +75,6 @@ constexpr int A_TILE = TBM * TBK * 2;  // 16 KiB
 //              per SM, a second CTA's epilogue overlapping the first's main
 //              loop measured faster than the persistent kernel (about 21 us
 //              against 25-27 us a layer).
-// Where F1, the K-240 layers and B1 have kernels of their own (k_fit_f1,
-// k_fit_mid, k_fit_b1) these two serve what those leave.
 template <int TBN_, int STAGES_, int NACC_>
 struct TcCfg {
   static constexpr int TBN = TBN_, STAGES = STAGES_, NACC = NACC_;
@@ -322,9 +324,6 @@ __device__ __forceinline__ void row_ld16(const float* chunk, int lane, float* v)
     v[q * 4 + 3] = u.w;
   }
 }
-
-// programmatic dependent launch: wait for the grid this one depends on (all
-// its writes visible); let the dependent grid be scheduled
 
 // Per-warp epilogue progress, carried across the tiles a CTA processes:
 // chunks done (input and output staging buffers alternate by chunk) and
@@ -634,11 +633,10 @@ __global__ void __launch_bounds__(128, 1)
                  : "memory");
 }
 
-// Persistent form of k_fit_tc for a layer with one main accumulator, used for
-// B1 (13 N tiles of 128 per row block: about 8 tiles per SM on the
-// 12,288-row step) and for the K-240 layers once they have many tiles per
-// SM (on the 12,288-row step they have about two and run faster as two
-// per-tile CTAs per SM): one CTA per SM walks the layer's tiles, the N tiles
+// Persistent form of k_fit_tc for a layer with one main accumulator: the K-240
+// layers, one launch each, from the number of tiles per SM that
+// gbdp_fitting_tc_set_persistent_min_tiles sets (not at its default, where
+// k_fit_mid or narrow tiles run them): one CTA per SM walks the layer's tiles, the N tiles
 // of a row block consecutively so that they run at the same time on
 // neighbouring SMs and share A through L2.  Warp 0 issues the TMA loads,
 // warp 1 the MMAs, warps 2-5 run the epilogue (warp w reads TMEM lanes
@@ -1311,7 +1309,7 @@ __global__ void __launch_bounds__(64 + MID_WARPS * 32, 1)
   unsigned char* ring = smem + 2 * MID_A;
   uint64_t* full = reinterpret_cast<uint64_t*>(ring + MID_RING * MID_PIECE);
   uint64_t* empty = full + MID_RING;
-  uint64_t* aready = empty + MID_RING;  // A written (8 epilogue warps)
+  uint64_t* aready = empty + MID_RING;  // A written (the epilogue warps)
   uint64_t* accfull = aready + 1;       // a layer's MMAs complete
   uint64_t* mdone = accfull + 1;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(mdone + 1);
@@ -1508,7 +1506,7 @@ __global__ void __launch_bounds__(64 + MID_WARPS * 32, 1)
       }
       if (!ok) break;
       p.epart[(size_t)(rb * TBM + r) * MID_PARTS + part] = esum;
-      // GZ1: this warp's rows of its two k-blocks, from the A buffer
+      // GZ1: this warp's rows of its k-block, from the A buffer
       fence_proxy_async_smem();
       __syncwarp();
       if (lane == 0) {

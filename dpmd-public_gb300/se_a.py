@@ -377,7 +377,8 @@ class SeAModel:
 
     def fitting_tc(self, b: "Batch"):
         """Both types' fitting nets on the tensor cores (six tcgen05 GEMM
-        launches with fused epilogues over the padded type blocks)."""
+        layers with fused epilogues over the padded type blocks, in three to
+        six launches by the number of rows)."""
         nt = self.cfg.ntypes
         nrows = (ctypes.c_int * nt)(*[c for _, c in b.type_rows])
         L.check(self._lib.gbdp_fitting_tc_f32(

@@ -569,13 +569,15 @@ GBDP_API int gbdp_fitting_tc_f32(float* e, float* dE_dD, const void* D_hi, const
 GBDP_API int gbdp_fitting_tc_status(const void* workspace, int rows, gbdp_stream stream);
 
 /* Launch-shape control of the tensor-core fitting (no counterpart in the
- * reference).  At the default, 32, the library chooses how the four K-240
- * layers (F2, F3, B3, B2) run: fused in one launch above 30 row blocks of 128,
- * one CTA per narrow tile below.  Any other value makes them one launch each,
- * one CTA per 128 x 80 tile (narrower for few rows), two per SM, while a layer
- * has fewer than `tiles_per_sm` tiles per SM, and on the persistent kernel
- * (one CTA per SM, double-buffered accumulators) from there on.
- * Process-wide. */
+ * reference).  32, the default, stands for the library's own choice of how the
+ * four K-240 layers (F2, F3, B3, B2) run: fused in one launch above 30 row
+ * blocks of 128, one CTA per narrow tile up to there.  Any other value makes
+ * them one launch each, one CTA per 128 x 80 tile (narrower for few rows), two
+ * per SM, while a layer has fewer than `tiles_per_sm` tiles per SM, and on the
+ * persistent kernel (one CTA per SM, double-buffered accumulators) from there
+ * on.  dE_dD has the same bits in every form; e sums its layer's partial sums
+ * in groups that depend on the form and the number of rows, and agrees to FP32
+ * rounding.  Process-wide. */
 GBDP_API void gbdp_fitting_tc_set_persistent_min_tiles(int tiles_per_sm);
 
 /* ---- launch-shape autotuning ----------------------------------------------
