@@ -50,10 +50,10 @@ int cuda_status(cudaError_t e, const char* where);
 // after the wait, never through the read-only path (no const __restrict__
 // parameter, __ldg or ld.global.nc, which promise the opposite and which no
 // fence holds back), in asm as volatile with a memory clobber.  What was
-// written before that kernel began is complete when this one begins.  A step on 192 atoms from host
-// to host, 18 kernels and 6 memsets: 204 us; so launched, clears in the chain
-// and the short kernels at its end merged: 183.  12,288 atoms captured in a
-// graph: 487 and 476.
+// written before that kernel began is complete when this one begins.
+// A step on 192 atoms from host to host, 18 kernels and 6 memsets: 204 us; so
+// launched, clears in the chain and the short kernels at its end merged: 183.
+// 12,288 atoms captured in a graph: 487 and 476.
 __device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_release() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
